@@ -8,12 +8,11 @@
 //                masks the interval's ends (the reference's cudaMemset + first-word patch, :496-500);
 //   2. sieve:    clears the odd multiples of the base primes 37 <= p <= isqrt(hi-1)
 //                (the reference's sieve_w30_seg_kernel, :120-143, one launch per prime):
-//                  small primes  p <  tile_bytes/coop_div : one warp per prime: below
-//                                                            tile_bytes/512 each residue progression
-//                                                            split over all lanes in blocks of 4
-//                                                            hits (no bank conflicts), above it 4
-//                                                            lanes per residue,
-//                  medium primes p <  mult_factor*tile_bytes: one thread per prime, 8 residues,
+//                  small primes  p <  tile_bytes/coop_div : one warp per prime, its hits as 32
+//                                                            progressions that never share a bank,
+//                  medium primes p <  walk bound          : one thread per prime, 8 residues,
+//                                p <  mult_factor*tile_bytes: one thread per prime of one class mod
+//                                                            30, its eight first hits and rounds,
 //                  large primes  otherwise                 : one thread per prime, walking its
 //                                                            multiples across the tile's span;
 //   3. restore:  sets the bits of base primes lying in the tile (the reference starts each prime
@@ -53,13 +52,9 @@ __constant__ uint8_t c_walk_start[240];
 // funnel shift takes its count mod 32, so byte << 3 is that rotation),
 // .y = gap_j | corr << 16.
 __constant__ uint2 c_walk_step[64];
-// The same steps packed into registers for the tile kernel's walk (no table load per visit:
-// shared-memory wavefronts are as scarce as issue slots there): nibble j of [bi] is corr_j,
-// nibble j of [8 + bi] the bit of p*m, nibble j of kGap2Packed gap_j / 2; the walk rotates the
-// three words by 4 bits per step, so the current step is always nibble 0.
-__constant__ uint32_t c_walk_pk[16];
-constexpr uint32_t kGap2Packed = 0x13212123u;
-
+// [bi*8 + j], for the primes that a tile takes by class: .x = D_j - D_{j-1} (D_j = floor(W30[bi] W30[j] / 30),
+// D_{-1} = 0), .y = the bit of W30[bi] * W30[j].
+__constant__ uint2 c_cls_step[64];
 static int ensure_tables();
 
 // Constant memory is per device: the tables are uploaded once for each device ordinal.
@@ -88,6 +83,26 @@ __device__ __forceinline__ uint32_t mod_by_magic_fma(uint64_t x, double xs, uint
   r += (int32_t)r < 0 ? p : 0u;
   r -= r >= p ? p : 0u;
   return r;
+}
+
+// x mod p for x < 2^58 and 8 <= p < 2^24, with xd = x as a double and inv = 1/p rounded to double.
+// Below 2^53 xd is exact and xd * inv is x/p within a relative 2^-53 (x/p < 2^50: 1/8), so the
+// integer q that adding 2^52 in the same rounding leaves in the low mantissa bits is within 0.63 of
+// x/p: the low 32 bits of x - q p are the remainder or the remainder less p.  Larger x go in two
+// steps of that kind: (x >> 28) mod p, then the rest below 2^24 * 2^28.
+__device__ __forceinline__ uint32_t mod_by_inv(uint64_t x, double xd, uint32_t p, double inv) {
+  constexpr double kTwo52 = 4503599627370496.0;
+  uint32_t r;
+  if (x < (1ull << 53)) {
+    r = (uint32_t)x - (uint32_t)__double2loint(__fma_rn(xd, inv, kTwo52)) * p;
+  } else {
+    const uint32_t h = (uint32_t)(x >> 28);
+    uint32_t rh = h - (uint32_t)__double2loint(__fma_rn((double)h, inv, kTwo52)) * p;
+    rh = min(rh, rh + p);
+    const uint64_t y = ((uint64_t)rh << 28) | (x & ((1ull << 28) - 1));
+    r = (uint32_t)y - (uint32_t)__double2loint(__fma_rn((double)y, inv, kTwo52)) * p;
+  }
+  return min(r, r + p);  // a negative remainder is a large unsigned
 }
 
 // x mod p from a double-precision estimate of the quotient, for p >= 2^11 and x < 2^62:
@@ -173,128 +188,150 @@ __device__ __forceinline__ uint32_t find_interval(const SieveArgs& a, uint32_t t
 #define VOSS_SM_GUARD(idx, limit)
 #endif
 
-__device__ __forceinline__ void clear_bit_word(uint32_t* bm, uint32_t word, uint32_t mask,
-                                               uint32_t limit, uint32_t* err) {
-  VOSS_SM_GUARD(word, limit)
-  atomicAnd(bm + word, mask);
+// The tile's bitmap in shared memory, words addressed by byte offset (a multiple of 4).  A clear
+// that may fall outside goes to the lane's own word behind the tile instead of around a branch:
+// shared-memory atomics are not predicated, and the divergence region of a branch costs five
+// instructions per clear (11.8 instructions against 6 for the hits of clear_class_primes).
+struct TileBits {
+  uint32_t* bm;
+  uint32_t spare;  // byte offset of the lane's word behind the tile (kSpareWords follow every tile)
+  uint32_t nw;     // words of this tile
+  uint32_t* err;
+
+  __device__ __forceinline__ void clear(uint32_t off, uint32_t mask) const {
+    VOSS_SM_GUARD(off >> 2, nw + kSpareWords)
+    atomicAnd(reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(bm) + off), mask);
+  }
+  // the word of byte x, or one behind the tile when x >= 4 nw (every such x, also wrapped below zero)
+  __device__ __forceinline__ void clear_or_spare(uint32_t x, uint32_t mask) const {
+    clear(min(x, spare) & ~3u, mask);
+  }
+};
+
+// The clear mask of bit `bit` of byte `byte`: ~1 rotated by 8 (byte mod 4) + bit (the funnel shift
+// takes its count mod 32).
+__device__ __forceinline__ uint32_t bit_mask(uint32_t byte, uint32_t bit) {
+  return __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, (byte << 3) + bit);
 }
 
-// Clears bit `bit` of every byte start, start + 4 ws, start + 8 ws, ... below Lt (one lane of a
-// warp-cooperative small prime; the stride is 4 ws bytes = ws words).  The stride is a multiple of
-// 4 bytes, so the byte lane inside the word, and with it the mask, never changes; four clears per
-// loop trip.
-__device__ __forceinline__ void clear_lane_progression(uint32_t* bm, uint32_t start, uint32_t ws,
-                                                       uint32_t bit, uint32_t Lt, uint32_t nw,
-                                                       uint32_t* err) {
-  const uint32_t mask = ~(1u << (((start & 3u) << 3) | bit));
-  const uint32_t wlim = (Lt + 3u - (start & 3u)) >> 2;  // start + 4k < Lt  <=>  (start >> 2) + k < wlim
-  uint32_t w = start >> 2;
-  if (wlim > 3u * ws) {
-    const uint32_t wlim4 = wlim - 3u * ws;
-#pragma unroll 2
-    for (; w < wlim4; w += 4u * ws) {
-      clear_bit_word(bm, w, mask, nw, err);
-      clear_bit_word(bm, w + ws, mask, nw, err);
-      clear_bit_word(bm, w + 2u * ws, mask, nw, err);
-      clear_bit_word(bm, w + 3u * ws, mask, nw, err);
-    }
+// Small primes, a warp per prime.  The prime's hits are 32 progressions of words, one per lane:
+// residue o = lane mod 8, first hit u = lane / 8 of four; a lane's bytes are s_o + u p + 4 p k, so
+// its byte lane, and with it the clear mask, is fixed and it advances by p words per step.  If lane
+// l starts in word c_l, step k clears words c_l + p k: the banks of a step are those of step 0
+// shifted, so lanes that collide once collide at every step.  As p is odd, p^-1 mod 32 turns banks
+// into places phi_l = c_l p^-1 (mod 32) on a circle that every lane walks one place per step.  The
+// lanes are sorted by phi (rank r_l) and lane l starts d_l = K + phi_l - r_l >= 0 steps late
+// (K = max(r - phi)): at every step the 32 lanes then stand on 32 different places, i.e. in 32
+// different banks, and each atomic instruction is a single wavefront.  The delays reach about 8
+// steps (the spread of 32 uniform points around their ranks) next to the Lt / (4 p) steps of the
+// prime.  Banks are the bound: an atomic of random banks takes 3.0 cycles of the SM's
+// shared-memory pipe, a conflict-free one 1.0 (measured).  Per tile of 6.02e6 integers the small
+// primes take 46k wavefronts; 4 lanes per residue at random banks from tile/512 on, with eight
+// set-ups per prime below, took 81k.
+__device__ __forceinline__ void clear_small_prime(const TileBits& T, uint32_t rec, const uint8_t* s_step,
+                                                  uint32_t lane, uint32_t Lt) {
+  constexpr unsigned kFull = 0xFFFFFFFFu;
+  const uint32_t r = rec & 0x1FFFu, p = (rec >> 13) & 0x1FFFu, bi = rec >> 26;
+  const uint32_t o = lane & 7u;
+  const uint32_t e = s_step[bi * 8u + o];
+  const uint32_t delta = (p / 30u) * w30(o) + (e & 31u);
+  const uint32_t byte = (delta >= r ? delta - r : delta + p - r) + (lane >> 3) * p;
+  const uint32_t mask = bit_mask(byte, e >> 5);
+  const uint32_t word = byte >> 2;
+  const uint32_t phi = (word * (p * (2u - p * p))) & 31u;  // p (2 - p^2) = p^-1 (mod 64) for odd p
+  uint32_t rank = 0;
+  unsigned eq = kFull;  // lanes whose phi agrees with mine in the bits looked at so far
+#pragma unroll
+  for (int b = 4; b >= 0; --b) {
+    const bool one = (phi >> b) & 1u;
+    const unsigned m = __ballot_sync(kFull, one);
+    rank += one ? (uint32_t)__popc(eq & ~m) : 0u;
+    eq &= one ? m : ~m;
   }
-  for (; w < wlim; w += ws) clear_bit_word(bm, w, mask, nw, err);
-}
-
-// One lane's share of a warp-cooperative residue progression bytes s, s + p, s + 2p, ... (p odd):
-// lane m clears the hits 4m + 128t + u (u = 0..3, t >= 0), i.e. bytes
-// byte + u p + 128 p t with byte = s + 4 p m, all below Lt.  For a fixed (t, u) the 32 lanes'
-// words are c + p m + 32 p t with c = (s + u p) >> 2 common to the warp: as p is odd they fall
-// in 32 distinct banks, so every shared-memory atomic of the warp is a single wavefront.  The
-// lane's four bytes of a block lie in four distinct byte lanes of their words and a block
-// advances by 128 p bytes = 32 p words, so the four masks and word offsets stay fixed.
-__device__ __forceinline__ void clear_block_progression(uint32_t* bm, uint32_t byte, uint32_t p, uint32_t bit,
-                                                        uint32_t Lt, uint32_t nw, uint32_t* err) {
-  if (byte + 3u * p < Lt) {
-    const uint32_t b1 = byte + p, b2 = b1 + p, b3 = b2 + p;
-    // ~(1 << bit) rotated to each byte's lane (the funnel shift takes its count mod 32)
-    const uint32_t nb = ~(1u << bit);
-    const uint32_t m0 = __funnelshift_l(nb, nb, byte << 3), m1 = __funnelshift_l(nb, nb, b1 << 3);
-    const uint32_t m2 = __funnelshift_l(nb, nb, b2 << 3), m3 = __funnelshift_l(nb, nb, b3 << 3);
-    uint32_t w0 = byte >> 2;
-    const uint32_t d1 = (b1 >> 2) - w0, d2 = (b2 >> 2) - w0, d3 = (b3 >> 2) - w0;
-    const uint32_t ws = 32u * p;
-    // b3 + 128 p k < Lt  <=>  (b3 >> 2) + 32 p k < lim
-    const uint32_t lim = ((Lt + 3u - (b3 & 3u)) >> 2) - d3;
-    uint32_t k = 0;
-#pragma unroll 4
-    for (; w0 < lim; w0 += ws, ++k) {
-      clear_bit_word(bm, w0, m0, nw, err);
-      clear_bit_word(bm, w0 + d1, m1, nw, err);
-      clear_bit_word(bm, w0 + d2, m2, nw, err);
-      clear_bit_word(bm, w0 + d3, m3, nw, err);
-    }
-    byte += 128u * p * k;
+  rank += (uint32_t)__popc(eq & ((1u << lane) - 1u));
+  const int K = __reduce_max_sync(kFull, (int)rank - (int)phi);
+  const uint32_t late = (uint32_t)(K + (int)phi - (int)rank);
+  // byte offsets of the words, negative before the lane's start (a large unsigned: the spare word);
+  // Lt is a multiple of 4, so byte + 4 p k < Lt  <=>  4 (word + p k) < Lt
+  uint32_t w = 4u * (word - p * late);
+  const uint32_t step = 4u * p;
+  const int left = (int)(Lt - w);
+  const int x_in = __reduce_max_sync(kFull, -(int)w);  // from here on every lane has started,
+  const int x_out = __reduce_min_sync(kFull, left);    // up to here none has finished
+  const int x_end = __reduce_max_sync(kFull, left);
+  int x = 0;
+  for (; x < x_in; x += (int)step, w += step) T.clear_or_spare(w, mask);
+#pragma unroll 1
+  for (; x + 3 * (int)step < x_out; x += 4 * (int)step) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j, w += step) T.clear(w, mask);
   }
-  // at most three hits remain (byte + 3p >= Lt); the next block belongs to the next lane
-  {
-    const uint32_t nb = ~(1u << bit);  // rotated by 8 * (byte & 3): the funnel shift takes byte << 3 mod 32
-    for (; byte < Lt; byte += p) clear_bit_word(bm, byte >> 2, __funnelshift_l(nb, nb, byte << 3), nw, err);
-  }
+  for (; x < x_end; x += (int)step, w += step) T.clear_or_spare(w, mask);
 }
 
 // Clears bit `bit` of bytes byte, byte + p, byte + 2p, ... below Lt (p odd).  Four consecutive
 // hits fall in the four distinct byte lanes of their words, and advancing all four by 4p bytes
-// moves each by exactly p words, so the unrolled loop keeps four fixed masks and word offsets.
-__device__ __forceinline__ void clear_progression(uint32_t* bm, uint32_t byte, uint32_t p, uint32_t bit,
-                                                  uint32_t Lt, uint32_t nw, uint32_t* err) {
-  if (byte + 3u * p < Lt) {
-    // the four hits' byte lanes are j0, j0 + p, j0 + 2p, j0 + 3p (mod 4): one lane up each time
-    // for p = 1 (mod 4), one lane down for p = 3, so each mask is the previous one rotated by a byte
-    const uint32_t j0 = byte & 3u;
-    const uint32_t nb = ~(1u << bit);
-    const uint32_t rot = (p & 2u) ? 24u : 8u;
-    const uint32_t m0 = __funnelshift_l(nb, nb, byte << 3), m1 = __funnelshift_l(m0, m0, rot),
-                   m2 = __funnelshift_l(m1, m1, rot), m3 = __funnelshift_l(m2, m2, rot);
-    uint32_t w0 = byte >> 2;
-    const uint32_t d1 = (j0 + p) >> 2, d2 = (j0 + 2u * p) >> 2, d3 = (j0 + 3u * p) >> 2;
-    // b3 + 4pk < Lt  <=>  w0 + k < lim  (w0 + d3 = b3 >> 2)
-    const uint32_t lim = ((Lt + 3u - ((j0 + 3u * p) & 3u)) >> 2) - d3;
-    for (; w0 < lim; w0 += p) {
-      clear_bit_word(bm, w0, m0, nw, err);
-      clear_bit_word(bm, w0 + d1, m1, nw, err);
-      clear_bit_word(bm, w0 + d2, m2, nw, err);
-      clear_bit_word(bm, w0 + d3, m3, nw, err);
-    }
-    byte = (w0 << 2) | j0;  // the loop advanced by 4p bytes (p words) per trip
+// moves each by exactly p words, so the unrolled loop keeps four fixed masks and word offsets; the
+// up to three hits that remain are predicated.
+__device__ __forceinline__ void clear_progression(const TileBits& T, uint32_t byte, uint32_t p, uint32_t bit,
+                                                  uint32_t Lt) {
+  // the four hits' byte lanes are j0, j0 + p, j0 + 2p, j0 + 3p (mod 4): one lane up each time
+  // for p = 1 (mod 4), one lane down for p = 3, so each mask is the previous one rotated by a byte
+  const uint32_t b1 = byte + p, b2 = b1 + p, b3 = b2 + p;
+  const uint32_t rot = (p & 2u) ? 24u : 8u;
+  const uint32_t m0 = bit_mask(byte, bit), m1 = __funnelshift_l(m0, m0, rot), m2 = __funnelshift_l(m1, m1, rot);
+  uint32_t w0 = byte & ~3u;
+  const uint32_t d1 = (b1 & ~3u) - w0, d2 = (b2 & ~3u) - w0, step = 4u * p;
+  if (b3 < Lt) {
+    const uint32_t m3 = __funnelshift_l(m2, m2, rot);
+    const uint32_t d3 = (b3 & ~3u) - w0;
+    const uint32_t lim = Lt - (b3 - w0);  // b3 + 4pk < Lt  <=>  w0 + 4pk < lim
+    do {
+      T.clear(w0, m0);
+      T.clear(w0 + d1, m1);
+      T.clear(w0 + d2, m2);
+      T.clear(w0 + d3, m3);
+      w0 += step;
+    } while (w0 < lim);
   }
-  {
-    const uint32_t nb = ~(1u << bit);  // rotated by 8 * (byte & 3): the funnel shift takes byte << 3 mod 32
-    for (; byte < Lt; byte += p) clear_bit_word(bm, byte >> 2, __funnelshift_l(nb, nb, byte << 3), nw, err);
-  }
+  T.clear_or_spare(w0, m0);
+  T.clear_or_spare(w0 + d1, m1);
+  T.clear_or_spare(w0 + d2, m2);
 }
 
-// Clears every multiple p*m (gcd(m, 30) = 1) of prime p = 30a + W30[bi] in the tile whose first
-// integer is vbase (a multiple of 30) and whose length is Lt bytes, visiting only those multiples
-// (about 8*Lt/p of them) instead of eight residue progressions.  rv = vbase mod p.
-__device__ __forceinline__ void clear_wheel_walk(uint32_t* bm, uint32_t p, uint32_t a, uint32_t bi, uint32_t rv,
-                                                 const uint8_t* s_wstart, const uint2* s_wpk,
-                                                 uint32_t Lt, uint32_t nw, uint32_t* err) {
-  uint32_t off = rv ? p - rv : 0u;         // first multiple of p at or above vbase, as an offset
-  const uint32_t t = off - 30u * (off / 30u);
-  const uint32_t st = s_wstart[bi * 30u + t];
-  off += (st & 7u) * p;                     // first multiple with m coprime to 30
-  const uint32_t sh = 4u * (st >> 3);
-  uint32_t byte = off / 30u;
-  const uint2 cb = s_wpk[bi];
-  const uint32_t c0 = cb.x, b0 = cb.y;
-  uint32_t G = __funnelshift_r(kGap2Packed, kGap2Packed, sh);
-  uint32_t C = __funnelshift_r(c0, c0, sh), B = __funnelshift_r(b0, b0, sh);
-  const uint32_t a2 = 2u * a;
-  while (byte < Lt) {
-    // ~(1 << bit) rotated by 8 * (byte & 3): the funnel shift takes its count mod 32, and
-    // bit < 8 leaves the byte-lane part of (byte << 3) + bit untouched
-    clear_bit_word(bm, byte >> 2, __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, ((byte << 3) & 24u) | (B & ~24u)), nw, err);
-    byte += a2 * (G & 3u) + (C & 7u);
-    G = __funnelshift_r(G, G, 4);
-    C = __funnelshift_r(C, C, 4);
-    B = __funnelshift_r(B, B, 4);
+// The multiples of 32 primes of one residue class mod 30 (p = 30a + W30[bi], a lane per prime, in
+// ascending order, pmin the first lane's) in the tile: the first hits s_j of the eight
+// progressions by additions from the remainder r of the tile's first byte (progression j holds
+// the bytes = a W30[j] + D_j (mod p), and a step from j to j + 1 adds a (W30[j+1] - W30[j]) + corr_j),
+// then rounds of eight predicated clears, each round one period p further.  For primes above the
+// tile length one round does it.  The class is the warp's, so corr_j and the bits are the same
+// for all lanes: nothing is looked up per hit, and nothing branches but the round loop.
+// Bound by issue slots: 401k warp instructions per tile near 10^12, against 451k of a walk from multiple
+// to multiple whose steps depend on the lane's own class.
+__device__ __forceinline__ void clear_class_primes(const TileBits& T, uint32_t p, uint32_t r, uint32_t pmin,
+                                                   uint32_t cls, uint32_t Lt) {
+  const uint32_t a = p / 30u;
+  uint32_t corr[8], bit[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint2 e = c_cls_step[8u * cls + j];
+    corr[j] = e.x;
+    bit[j] = e.y;
+  }
+  constexpr uint32_t gap[8] = {1, 6, 4, 2, 4, 2, 4, 6};  // W30[j] - W30[j - 1]
+  uint32_t s[8];
+  uint32_t t = 0u - r;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    t += a * gap[j] + corr[j];  // in (-p, p)
+    s[j] = min(t, t + p);       // t mod p: a negative t is a large unsigned
+  }
+  for (uint32_t x = 0; x < Lt; x += pmin) {  // s_j >= x in round x / pmin
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      T.clear_or_spare(s[j], bit_mask(s[j], bit[j]));
+      s[j] += p;
+    }
   }
 }
 
@@ -452,7 +489,8 @@ struct TileHdr {  // one tile's header (double-buffered: the next tile's is buil
   uint32_t pre_base[kPreGroups];
   uint32_t interval, tile;
   uint32_t r0, r1;       // base primes lying in the tile (restore)
-  uint32_t coop_ctr, b_ctr, c_ctr;  // work counters of the three prime categories
+  uint32_t coop_ctr, b_ctr, w_ctr, c_ctr;  // work counters of the prime categories
+  uint32_t w_items, w_lo[8], w_n[8];  // primes taken by class: items of 32, first and number per class
   unsigned long long gword;         // the tile's first word in the large-prime bitmap
   uint32_t first;
 };
@@ -582,12 +620,8 @@ __device__ __forceinline__ uint32_t acc_index(uint32_t i) {
   return (uint32_t)kAccCls143 + 8u * (c >= 143u ? c - 143u : c) + (i & 7u);
 }
 
-// Warp-cooperative primes p >= tile bytes / kSmallSplitDiv give each residue 4 lanes (their few
-// hits per residue keep a lane's loop long); smaller ones give each residue all 32 lanes in turn.
-#ifndef VOSS_SMALL_SPLIT_DIV
-#define VOSS_SMALL_SPLIT_DIV 512
-#endif
-constexpr uint32_t kSmallSplitDiv = VOSS_SMALL_SPLIT_DIV;
+// Small primes' records (prime, remainder, residue class) take 13 + 13 + 3 bits of a word.
+constexpr uint32_t kSmallPrimeEnd = 1u << 13;
 
 constexpr uint32_t kFlushEvery = 2048;  // tiles between counter flushes (u32 headroom)
 
@@ -620,7 +654,9 @@ __device__ __forceinline__ void tile_header(TileHdr& H, CtaState& St, const Siev
       uint32_t np = sq >= a.p_max ? a.n_primes : count_le_warp(a.primes, a.n_primes, sq, ln);
       if (a.gbm && np > a.scatter_first) np = a.scatter_first;  // the rest came from the pre-pass
       if (lt != St.c_lt) {
-        const uint32_t ia = count_lt_warp(a.primes, a.n_primes, (uint64_t)(lt / a.coop_div), ln);
+        // one record per thread of the block, and primes that fit a record (clear_small_prime)
+        const uint32_t ia0 = count_lt_warp(a.primes, a.n_primes, (uint64_t)min(lt / a.coop_div, kSmallPrimeEnd), ln);
+        const uint32_t ia = min(ia0, (uint32_t)blockDim.x);
         const uint32_t ib = count_lt_warp(a.primes, a.n_primes, (uint64_t)lt * a.mult_factor, ln);
         const uint32_t iw = count_lt_warp(a.primes, a.n_primes, ((uint64_t)lt * a.walk_sixteenths) >> 4, ln);
         __syncwarp();
@@ -635,8 +671,21 @@ __device__ __forceinline__ void tile_header(TileHdr& H, CtaState& St, const Siev
       const uint32_t ia = min(St.c_ia, np);
       const uint32_t ib0 = min(St.c_ib, np);
       const uint32_t ib = ib0 < ia ? ia : ib0;
-      const uint32_t iw0 = min(St.c_iw, np);
-      const uint32_t iw = iw0 < ia ? ia : (iw0 > ib ? ib : iw0);
+      // the by-class primes [iwb, ib): their lower end and the ascending list's upper end meet at a
+      // multiple of kClsBlock, where the numbers of primes per class are tabulated; the upper end is
+      // rounded up (a few primes beyond the tile's root or the pre-pass's first strike out
+      // composites again)
+      const uint32_t iwb = max(St.c_iw & ~(kClsBlock - 1u), (ia + kClsBlock - 1u) & ~(kClsBlock - 1u));
+      const uint32_t iw = min(iwb, ib);
+      uint32_t w_n = 0;
+      if (ib > iwb && ln < 8u) {
+        const uint32_t hb = min((ib + kClsBlock - 1u) / kClsBlock, a.n_cls_blocks);
+        const uint32_t lo = a.cls_index[8u * (iwb / kClsBlock) + ln];
+        w_n = a.cls_index[8u * hb + ln] - lo;
+        H.w_lo[ln] = a.cls_first[ln] + lo;
+        H.w_n[ln] = w_n;
+      }
+      const uint32_t w_items = 8u * ((__reduce_max_sync(0xFFFFFFFFu, w_n) + 31u) >> 5);
       uint32_t r0 = a.n_primes, r1 = a.n_primes;
       if (vbase <= a.p_max) {
         r0 = count_lt_warp(a.primes, a.n_primes, vbase, ln);
@@ -679,6 +728,8 @@ __device__ __forceinline__ void tile_header(TileHdr& H, CtaState& St, const Siev
         for (int g = 0; g < kPreGroups; ++g) H.pre_base[g] = (uint32_t)(wt % pre_mod(g));
         H.coop_ctr = 0;
         H.b_ctr = 0;
+        H.w_ctr = 0;
+        H.w_items = w_items;
         H.c_ctr = 0;
         H.first = kNone;
       }
@@ -691,7 +742,7 @@ __global__ void __launch_bounds__(BLOCK, (BLOCK == 512 ? 2 : 1))
 sieve_tiles_kernel(SieveArgs a) {
   extern __shared__ __align__(16) uint32_t smem[];
   uint32_t* bm = smem;
-  uint32_t* pre = smem + a.tile_words;
+  uint32_t* pre = smem + a.tile_words + kSpareWords;
   uint32_t* cnt = pre + kPreWords;
   __shared__ TileHdr HH[2];  // this tile's header and the next one's
   __shared__ CtaState St;
@@ -701,9 +752,8 @@ sieve_tiles_kernel(SieveArgs a) {
   __shared__ __align__(8) uint8_t s_step[64];
   __shared__ int8_t s_rb[32];
   __shared__ uint32_t s_pos[32];  // bit b of a word -> integer offset 30 * (b / 8) + W30[b % 8]
-  __shared__ uint8_t s_wstart[240];
-  __shared__ uint2 s_wpk[8];
-  __shared__ uint32_t s_rank[EMIT ? 1 : BLOCK];   // first tile rank of each thread's chunk
+  // extraction: first tile rank of each thread's chunk; sieve: the small primes' records
+  __shared__ uint32_t s_rank[BLOCK];
   __shared__ int32_t s_before[EMIT ? 1 : BLOCK];  // last prime before each chunk (-1: none)
   __shared__ uint16_t s_mid[EMIT ? 1 : BLOCK];    // primes in the first C / 2 words of each chunk
   uint32_t* err = a.error;
@@ -713,8 +763,6 @@ sieve_tiles_kernel(SieveArgs a) {
   if (tid < 64) s_step[tid] = c_wheel_step[tid];
   if (tid < 32) s_rb[tid] = c_res_bit[tid];
   if (tid < 32) s_pos[tid] = 30u * ((uint32_t)tid >> 3) + w30((uint32_t)tid & 7u);
-  if (tid < 240) s_wstart[tid] = c_walk_start[tid];
-  if (tid < 8) s_wpk[tid] = make_uint2(c_walk_pk[tid], c_walk_pk[8 + tid]);
   if (!EMIT)
     for (uint32_t i = tid; i < (uint32_t)kSmCounters; i += BLOCK) cnt[i] = 0;
   if (tid == 0) {
@@ -770,6 +818,17 @@ sieve_tiles_kernel(SieveArgs a) {
     VOSS_PHASE(1)
 
     const uint32_t nw = H.nw, Lt = H.lt;
+    // tiles below 2^53 reduce the prime offsets with one fma instead of the 64-bit Barrett product
+    const bool fma_mod = H.vbase < (1ull << 53);
+    const double ks = (double)H.ktile * 0x1p-64, vs = (double)H.vbase * 0x1p-64;
+
+    // the small primes' records, a thread per prime: remainder of the tile's first byte, p, class
+    if ((uint32_t)tid < H.ia) {
+      const uint32_t p = a.primes[tid];
+      const uint64_t m = a.magic[tid];
+      const uint32_t r = fma_mod ? mod_by_magic_fma(H.ktile, ks, p, m) : mod_barrett(H.ktile, p, m);
+      s_rank[tid] = r | p << 13 | (uint32_t)s_rb[p % 30u] << 26;
+    }
 
     // ---- 1. fill ----------------------------------------------------------------------
     {
@@ -819,40 +878,14 @@ sieve_tiles_kernel(SieveArgs a) {
     {
       const uint64_t ktile = H.ktile;
       const uint32_t ia = H.ia, ib = H.ib, iw = H.iw, np = H.np;
-      // tiles below 2^53 reduce the prime offsets with one fma instead of the 64-bit Barrett product
-      const bool fma_mod = H.vbase < (1ull << 53);
-      const double ks = (double)ktile * 0x1p-64, vs = (double)H.vbase * 0x1p-64;
+      const TileBits T{bm, Lt + 4u * (uint32_t)lane, nw, err};
       // small primes: a warp per prime
-      const uint32_t split = Lt / kSmallSplitDiv;
-      const uint32_t lane_ofs = 4u * (uint32_t)lane;
       for (;;) {
         uint32_t i = 0;
         if (lane == 0) i = atomicAdd(&H.coop_ctr, 1u);
         i = __shfl_sync(0xFFFFFFFFu, i, 0);
         if (i >= ia) break;
-        const uint32_t p = a.primes[i];
-        const uint64_t m = a.magic[i];
-        const uint32_t r = fma_mod ? mod_by_magic_fma(ktile, ks, p, m) : mod_barrett(ktile, p, m);
-        const uint32_t pa = p / 30u, bi = (uint32_t)s_rb[p - 30u * pa];
-        if (p >= split) {
-          // 4 lanes per residue progression (lane = 4 o + q: bytes s_o + q p + 4p k)
-          const uint32_t o = (uint32_t)lane >> 2;
-          const uint32_t e = s_step[bi * 8u + o];
-          const uint32_t delta = pa * w30(o) + (e & 31u);
-          const uint32_t s = delta >= r ? delta - r : delta + p - r;
-          clear_lane_progression(bm, s + ((uint32_t)lane & 3u) * p, p, e >> 5, Lt, nw, err);
-        } else {
-          // the eight residue progressions in turn, each split over all lanes in blocks of four
-          // consecutive hits (bank-conflict-free, clear_block_progression)
-          const uint32_t lp = lane_ofs * p;
-#pragma unroll 1
-          for (uint32_t o = 0; o < 8; ++o) {
-            const uint32_t e = s_step[bi * 8u + o];
-            const uint32_t delta = pa * w30(o) + (e & 31u);
-            const uint32_t s = delta >= r ? delta - r : delta + p - r;
-            clear_block_progression(bm, s + lp, p, e >> 5, Lt, nw, err);
-          }
-        }
+        clear_small_prime(T, s_rank[i], s_step, (uint32_t)lane, Lt);
       }
       VOSS_PHASE(3)
       // medium primes
@@ -862,16 +895,9 @@ sieve_tiles_kernel(SieveArgs a) {
           uint32_t base = 0;
           if (lane == 0) base = atomicAdd(&H.b_ctr, 32u);
           base = __shfl_sync(0xFFFFFFFFu, base, 0);
-          if (base >= ib - ia) break;
+          if (base >= iw - ia) break;
           const uint32_t i = ia + base + (uint32_t)lane;
-          if (i >= iw && i < ib) {
-            // few hits per tile: walk the prime's coprime multiples
-            const uint32_t p = a.primes[i];
-            const uint32_t pa = p / 30u, bi = (uint32_t)s_rb[p - 30u * pa];
-            const uint64_t m = a.magic[i];
-            clear_wheel_walk(bm, p, pa, bi, fma_mod ? mod_by_magic_fma(H.vbase, vs, p, m) : mod_barrett(H.vbase, p, m),
-                             s_wstart, s_wpk, Lt, nw, err);
-          } else if (i < ib) {
+          if (i < iw) {
             const uint32_t p = a.primes[i];
             const uint64_t m = a.magic[i];
             const uint32_t r = fma_mod ? mod_by_magic_fma(ktile, ks, p, m) : mod_barrett(ktile, p, m);
@@ -881,9 +907,27 @@ sieve_tiles_kernel(SieveArgs a) {
             for (uint32_t o = 0; o < 8; ++o) {
               const uint32_t e = ((o < 4u ? st8.x : st8.y) >> (8u * (o & 3u))) & 0xFFu;
               const uint32_t delta = pa * w30(o) + (e & 31u);
-              clear_progression(bm, delta >= r ? delta - r : delta + p - r, p, e >> 5, Lt, nw, err);
+              clear_progression(T, delta >= r ? delta - r : delta + p - r, p, e >> 5, Lt);
             }
           }
+        }
+        // few hits per tile: a thread per prime of a class, 32 primes of one class at a time (item
+        // i: class i mod 8, its (i / 8)-th group; the classes hold nearly equal numbers of primes)
+        const double kd = (double)ktile;
+        const uint32_t w_end = H.w_items;
+        for (;;) {
+          uint32_t it = 0;
+          if (lane == 0) it = atomicAdd(&H.w_ctr, 1u);
+          it = __shfl_sync(0xFFFFFFFFu, it, 0);
+          if (it >= w_end) break;
+          const uint32_t c = it & 7u, k = 32u * (it >> 3), n = H.w_n[c];
+          if (k >= n) continue;
+          const bool live = k + (uint32_t)lane < n;
+          const uint32_t i = H.w_lo[c] + (live ? k + (uint32_t)lane : n - 1u);  // idle lanes repeat the last prime
+          const uint32_t p = a.cls_primes[i];
+          const double inv = a.cls_inv[i];
+          const uint32_t r = mod_by_inv(ktile, kd, p, inv);
+          clear_class_primes(T, p, r, __shfl_sync(0xFFFFFFFFu, p, 0), c, Lt);
         }
       } else {
         // a lane per (prime, residue): a warp takes 4 consecutive primes, lane = 8*prime + residue
@@ -899,7 +943,7 @@ sieve_tiles_kernel(SieveArgs a) {
             const uint32_t pa = p / 30u, bi = (uint32_t)s_rb[p - 30u * pa];
             const uint32_t e = s_step[bi * 8u + o];
             const uint32_t delta = pa * wo + (e & 31u);
-            clear_progression(bm, delta >= r ? delta - r : delta + p - r, p, e >> 5, Lt, nw, err);
+            clear_progression(T, delta >= r ? delta - r : delta + p - r, p, e >> 5, Lt);
           }
         }
       }
@@ -921,7 +965,7 @@ sieve_tiles_kernel(SieveArgs a) {
           for (; d < span; d += p) {
             const uint32_t q = d / 30u;
             const int b = s_rb[d - 30u * q];
-            if (b >= 0) clear_bit_word(bm, q >> 2, ~(1u << (((q & 3u) << 3) | (uint32_t)b)), nw, err);
+            if (b >= 0) T.clear(q & ~3u, bit_mask(q, (uint32_t)b));
           }
         }
       }
@@ -1435,8 +1479,7 @@ static int ensure_tables() {
       step[bi * 8 + o] = (uint8_t)((bw / 30) | (rb[bw % 30] << 5));
     }
   uint8_t wstart[240];
-  uint2 wstep[64];
-  uint32_t wpk[16] = {0};
+  uint2 wstep[64], cls[64];
   for (int bi = 0; bi < 8; ++bi) {
     int pinv = 1;
     while ((kW30h[bi] * pinv) % 30 != 1) ++pinv;
@@ -1451,14 +1494,13 @@ static int ensure_tables() {
       const int d0 = (w * kW30h[j]) / 30;
       const int gap = (j < 7 ? kW30h[j + 1] : 31) - kW30h[j];
       const int corr = j < 7 ? (w * kW30h[j + 1]) / 30 - d0 : w + 0 - d0;  // j = 7: next m is 30(c+1) + 1
+      cls[bi * 8 + j] = make_uint2((uint32_t)(d0 - (j ? (w * kW30h[j - 1]) / 30 : 0)), (uint32_t)rb[(w * kW30h[j]) % 30]);
       wstep[bi * 8 + j] = make_uint2(~(1u << rb[(w * kW30h[j]) % 30]), (uint32_t)gap | ((uint32_t)corr << 16));
-      wpk[bi] |= (uint32_t)corr << (4 * j);
-      wpk[8 + bi] |= (uint32_t)rb[(w * kW30h[j]) % 30] << (4 * j);
     }
   }
   if (cudaMemcpyToSymbol(c_walk_start, wstart, sizeof(wstart)) != cudaSuccess) return -1;
   if (cudaMemcpyToSymbol(c_walk_step, wstep, sizeof(wstep)) != cudaSuccess) return -1;
-  if (cudaMemcpyToSymbol(c_walk_pk, wpk, sizeof(wpk)) != cudaSuccess) return -1;
+  if (cudaMemcpyToSymbol(c_cls_step, cls, sizeof(cls)) != cudaSuccess) return -1;
   if (cudaMemcpyToSymbol(c_wheel_step, step, sizeof(step)) != cudaSuccess) return -1;
   if (cudaMemcpyToSymbol(c_res_bit, rb, sizeof(rb)) != cudaSuccess) return -1;
   g_tables_ready.fetch_or(bit);
@@ -1485,7 +1527,7 @@ void build_presieve_tables(uint32_t* out) {
 }
 
 size_t sieve_smem_bytes(uint32_t tile_words) {
-  return (size_t)(tile_words + kPreWords + kSmCounters) * sizeof(uint32_t);
+  return (size_t)(tile_words + kSpareWords + kPreWords + kSmCounters) * sizeof(uint32_t);
 }
 
 template <int BLOCK, bool EMIT>

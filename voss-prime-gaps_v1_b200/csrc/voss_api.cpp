@@ -147,6 +147,40 @@ int apply_tuning(voss_ctx* c, const voss_tuning& t0) {
 }
 
 
+// The primes below kClsLimit grouped by residue class mod 30 (SieveArgs::cls_primes).
+int upload_class_primes(voss_ctx* c) {
+  int idx[30];
+  for (int i = 0; i < 30; ++i) idx[i] = -1;
+  for (int i = 0; i < 8; ++i) idx[kW30[i]] = i;
+  const size_t n = (size_t)(std::lower_bound(c->primes.begin(), c->primes.end(), kClsLimit) - c->primes.begin());
+  c->n_cls_blocks = (uint32_t)((n + kClsBlock - 1) / kClsBlock);
+  std::vector<uint32_t> by[8], index(8 * ((size_t)c->n_cls_blocks + 1));
+  for (auto& v : by) v.reserve(n / 8 + n / 64 + 16);
+  for (size_t i = 0; i < n; ++i) {
+    if (i % kClsBlock == 0)
+      for (int k = 0; k < 8; ++k) index[8 * (i / kClsBlock) + k] = (uint32_t)by[k].size();
+    by[idx[c->primes[i] % 30]].push_back(c->primes[i]);
+  }
+  std::vector<uint32_t> all;
+  all.reserve(n + 1);
+  for (int k = 0; k < 8; ++k) {
+    index[8 * (size_t)c->n_cls_blocks + k] = (uint32_t)by[k].size();
+    c->cls_first[k] = (uint32_t)all.size();
+    all.insert(all.end(), by[k].begin(), by[k].end());
+  }
+  if (all.empty()) all.push_back(0);
+  std::vector<double> inv(all.size(), 0.0);
+  for (size_t i = 0; i < n; ++i) inv[i] = 1.0 / all[i];
+  int rc;
+  if ((rc = c->d_cls_primes.ensure(all.size() * sizeof(uint32_t))) || (rc = c->d_cls_inv.ensure(inv.size() * sizeof(double))) ||
+      (rc = c->d_cls_index.ensure(index.size() * sizeof(uint32_t))))
+    return rc;
+  CUDA_TRY(cudaMemcpy(c->d_cls_primes.p, all.data(), all.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpy(c->d_cls_inv.p, inv.data(), inv.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpy(c->d_cls_index.p, index.data(), index.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+  return VOSS_OK;
+}
+
 // Cut intervals [lo_i, hi_i) into tiles; intervals without wheel integers get no tiles.
 int plan_intervals(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, uint32_t n,
                    uint64_t seg_k, RunPlan* P) {
@@ -203,6 +237,11 @@ int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPl
   a.magic = c->d_magic.as<uint64_t>();
   a.n_primes = (uint32_t)c->primes.size();
   a.p_max = c->primes.empty() ? 0u : c->primes.back();
+  a.cls_primes = c->d_cls_primes.as<uint32_t>();
+  a.cls_inv = c->d_cls_inv.as<double>();
+  a.cls_index = c->d_cls_index.as<uint32_t>();
+  std::memcpy(a.cls_first, c->cls_first, sizeof(a.cls_first));
+  a.n_cls_blocks = c->n_cls_blocks;
   a.pretab = c->d_pretab.as<uint32_t>();
   a.iv = W.iv.as<IntervalDev>();
   a.n_intervals = n_iv;
@@ -877,6 +916,7 @@ VOSS_API int voss_ctx_create(int device, uint64_t max_hi, voss_ctx** out) {
   }
   if (cudaMemcpy(c->d_pretab.p, pre.data(), kPreWords * 4, cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(fail(VOSS_ERR_CUDA, "presieve table upload failed"));
+  if ((rc = upload_class_primes(c))) return bail(rc);
   voss_tuning t{};
   if ((rc = apply_tuning(c, t))) return bail(rc);
   if (const char* lim = std::getenv("VOSS_STAGE_LIMIT")) {

@@ -115,6 +115,9 @@ struct voss_ctx {
   uint64_t max_hi = 0;
   std::vector<uint32_t> primes;  // >= 37
   voss_host::DevBuf d_primes, d_magic, d_pretab;
+  voss_host::DevBuf d_cls_primes, d_cls_inv, d_cls_index;  // the primes below kClsLimit by class (SieveArgs)
+  uint32_t cls_first[8] = {0};
+  uint32_t n_cls_blocks = 0;
   voss_tuning tune{};
   int ctas_per_sm = 1;
   voss_host::Workspace ws;

@@ -29,6 +29,10 @@ constexpr uint32_t kPreMod[kPreGroups] = {1001u /*7*11*13*/, 323u /*17*19*/, 667
                                           31u /*31*/};
 constexpr uint32_t kPreOff[kPreGroups] = {0u, 1001u, 1324u, 1991u};
 constexpr uint32_t kPreWords = 2022u;
+constexpr uint32_t kSpareWords = 32u;  // behind every tile in shared memory: one word per lane (TileBits)
+constexpr uint32_t kClsBlock = 256u;
+// mult_factor * tile bytes, the end of the primes that tiles take by class, is at most 64 * 252,252
+constexpr uint32_t kClsLimit = 1u << 24;
 constexpr uint32_t kFirstSievePrime = 37u;  // the base-prime table starts here
 
 // ---- accumulator layout (u64 words per interval) ----------------------------------------
@@ -129,6 +133,14 @@ struct SieveArgs {
   const uint64_t* magic;    // floor((2^64-1)/p) per prime
   uint32_t n_primes;
   uint32_t p_max;           // the last (largest) base prime, 0 when there is none
+  // The base primes below kClsLimit again, grouped by residue class mod 30 (W30 order), ascending
+  // within a class, with 1/p; cls_index[8 i + c] counts those of class c among the first
+  // kClsBlock * i primes of the ascending table (i = n_cls_blocks: all of them).
+  const uint32_t* cls_primes;
+  const double* cls_inv;
+  const uint32_t* cls_index;
+  uint32_t cls_first[8];    // each class's first entry
+  uint32_t n_cls_blocks;
   const uint32_t* pretab;   // kPreWords presieve masks
   const IntervalDev* iv;
   const uint32_t* tile_iv;  // interval of each tile (nullptr: found by binary search over iv)
