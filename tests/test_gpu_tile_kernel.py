@@ -1,0 +1,55 @@
+"""The tile kernel at the sizes where its parts can go wrong, against the CPU oracle (exact): the
+last words of a tile, tiles of a few words, tiles without a far gap (the longest gap is then
+searched again), primes taken as small, by progressions and by class in every proportion."""
+import pytest
+
+import oracle_lib as O
+from test_gpu_sieve import assert_range_equal
+
+pytestmark = pytest.mark.gpu
+
+WORD = 120  # integers per 32-bit bitmap word
+
+
+# words of the range: around one residue-class period (1001), a warp, the full tile (50176) and two
+@pytest.mark.parametrize("words", [1, 2, 31, 33, 1000, 1001, 1002, 50175, 50176, 50177, 100353])
+@pytest.mark.parametrize("lo", [120 * 10**4, 10**12 - 77])
+def test_tile_lengths(gpu_ctx, lo, words):
+    hi = lo + WORD * words - 13
+    assert_range_equal(gpu_ctx.sieve_range(lo, hi), O.sieve_range(lo, hi))
+
+
+@pytest.mark.parametrize("lo,ln", [(10**6, 40), (10**6, 400), (10**9 + 1, 1500), (10**12, 90), (10**12, 5000)])
+def test_short_tiles_find_their_longest_gap(gpu_ctx, lo, ln):
+    for k in range(12):
+        a = lo + 997 * k
+        assert_range_equal(gpu_ctx.sieve_range(a, a + ln), O.sieve_range(a, a + ln))
+
+
+@pytest.mark.parametrize("tuning", [
+    dict(coop_div=1),                             # more small primes than records
+    dict(coop_div=100000, walk_sixteenths=1),     # none, and the classes from a sixteenth of a tile on
+    dict(walk_sixteenths=128),                    # no prime by class
+    dict(mult_factor=1, walk_sixteenths=16),      # the classes end at the tile length
+    dict(mult_factor=64),
+    dict(medium_mode=1),
+    dict(block_threads=512, chunk_words=9),
+    dict(block_threads=1024, chunk_words=1),
+])
+def test_tunings(gpu_ctx, tuning):
+    lo, hi = 10**13 - 3 * 10**6, 10**13 + 5 * 10**6 + 1
+    o = O.sieve_range(lo, hi)
+    try:
+        gpu_ctx.set_tuning(**tuning)
+        assert_range_equal(gpu_ctx.sieve_range(lo, hi), o)
+    finally:
+        gpu_ctx.set_tuning()
+
+
+@pytest.mark.parametrize("min_gap", [3, 4, 6, 30, 100, 130])
+def test_gap_lists_down_to_the_smallest_gaps(gpu_ctx, min_gap):
+    lo, hi = 10**10, 10**10 + 2 * 10**6
+    p = O.primes_range(lo, hi)
+    want = [(int(b), int(b - a)) for a, b in zip(p[:-1], p[1:]) if b - a >= min_gap]
+    got = gpu_ctx.gaps_at_least(lo, hi, min_gap)
+    assert [(int(a), int(g)) for a, g in zip(got["position"], got["gap"])] == want

@@ -202,9 +202,15 @@ struct TileBits {
     VOSS_SM_GUARD(off >> 2, nw + kSpareWords)
     atomicAnd(reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(bm) + off), mask);
   }
-  // the word of byte x, or one behind the tile when x >= 4 nw (every such x, also wrapped below zero)
-  __device__ __forceinline__ void clear_or_spare(uint32_t x, uint32_t mask) const {
-    clear(min(x, spare) & ~3u, mask);
+  // the same, or a word behind the tile when off >= 4 nw (an offset below zero is a large unsigned)
+  __device__ __forceinline__ void clear_word_or_spare(uint32_t off, uint32_t mask) const {
+    clear(min(off, spare), mask);
+  }
+  // bit x of the tile, or some bit of a spare word when x >= 32 nw
+  __device__ __forceinline__ void clear_bit_or_spare(uint32_t x) const {
+    const uint32_t word = min(x, 8u * spare) >> 5;
+    VOSS_SM_GUARD(word, nw + kSpareWords)
+    atomicAnd(bm + word, __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, x));
   }
 };
 
@@ -254,19 +260,19 @@ __device__ __forceinline__ void clear_small_prime(const TileBits& T, uint32_t re
   // byte offsets of the words, negative before the lane's start (a large unsigned: the spare word);
   // Lt is a multiple of 4, so byte + 4 p k < Lt  <=>  4 (word + p k) < Lt
   uint32_t w = 4u * (word - p * late);
-  const uint32_t step = 4u * p;
+  const int step = 4 * (int)p;
   const int left = (int)(Lt - w);
   const int x_in = __reduce_max_sync(kFull, -(int)w);  // from here on every lane has started,
-  const int x_out = __reduce_min_sync(kFull, left);    // up to here none has finished
-  const int x_end = __reduce_max_sync(kFull, left);
+  const int x_out = __reduce_min_sync(kFull, left);    // up to here none has finished,
+  const int x_end = __reduce_max_sync(kFull, left);    // and here all have
   int x = 0;
-  for (; x < x_in; x += (int)step, w += step) T.clear_or_spare(w, mask);
+  for (; x < x_in; x += step, w += (uint32_t)step) T.clear_word_or_spare(w, mask);
 #pragma unroll 1
-  for (; x + 3 * (int)step < x_out; x += 4 * (int)step) {
+  for (const int x_8 = x_out - 7 * step; x < x_8; x += 8 * step) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j, w += step) T.clear(w, mask);
+    for (int j = 0; j < 8; ++j, w += (uint32_t)step) T.clear(w, mask);
   }
-  for (; x < x_end; x += (int)step, w += step) T.clear_or_spare(w, mask);
+  for (; x < x_end; x += step, w += (uint32_t)step) T.clear_word_or_spare(w, mask);
 }
 
 // Clears bit `bit` of bytes byte, byte + p, byte + 2p, ... below Lt (p odd).  Four consecutive
@@ -294,10 +300,14 @@ __device__ __forceinline__ void clear_progression(const TileBits& T, uint32_t by
       w0 += step;
     } while (w0 < lim);
   }
-  T.clear_or_spare(w0, m0);
-  T.clear_or_spare(w0 + d1, m1);
-  T.clear_or_spare(w0 + d2, m2);
+  T.clear_word_or_spare(w0, m0);
+  T.clear_word_or_spare(w0 + d1, m1);
+  T.clear_word_or_spare(w0 + d2, m2);
 }
+
+struct ClassStep {  // c_cls_step of one class
+  uint32_t corr[8], bit[8];
+};
 
 // The multiples of 32 primes of one residue class mod 30 (p = 30a + W30[bi], a lane per prime, in
 // ascending order, pmin the first lane's) in the tile: the first hits s_j of the eight
@@ -306,33 +316,41 @@ __device__ __forceinline__ void clear_progression(const TileBits& T, uint32_t by
 // then rounds of eight predicated clears, each round one period p further.  For primes above the
 // tile length one round does it.  The class is the warp's, so corr_j and the bits are the same
 // for all lanes: nothing is looked up per hit, and nothing branches but the round loop.
-// Bound by issue slots: 401k warp instructions per tile near 10^12, against 451k of a walk from multiple
-// to multiple whose steps depend on the lane's own class.
+// Bound by issue slots: 52 instructions per round of eight clears and about 100 around them (loads,
+// remainder, first hits), against 451k per tile near 10^12 of a walk from multiple to multiple
+// whose steps depend on the lane's own class; shared-memory wavefronts are next (3.2 per clear).
 __device__ __forceinline__ void clear_class_primes(const TileBits& T, uint32_t p, uint32_t r, uint32_t pmin,
-                                                   uint32_t cls, uint32_t Lt) {
-  const uint32_t a = p / 30u;
-  uint32_t corr[8], bit[8];
+                                                   const ClassStep& C, uint32_t Lt) {
+  const uint32_t a = p / 30u, a2 = 2u * a, a4 = 2u * a2, a6 = a4 + a2;
+  uint32_t x[8];        // the hits as bit indices: 8 times the byte plus the bit
+  uint32_t t = 0u - r;  // in (-p, p)
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const uint2 e = c_cls_step[8u * cls + j];
-    corr[j] = e.x;
-    bit[j] = e.y;
+    constexpr uint32_t gap[8] = {1, 6, 4, 2, 4, 2, 4, 6};  // W30[j] - W30[j - 1]
+    t += (gap[j] == 1 ? a : gap[j] == 2 ? a2 : gap[j] == 4 ? a4 : a6) + C.corr[j];
+    x[j] = 8u * min(t, t + p) + C.bit[j];  // t mod p: a negative t is a large unsigned
   }
-  constexpr uint32_t gap[8] = {1, 6, 4, 2, 4, 2, 4, 6};  // W30[j] - W30[j - 1]
-  uint32_t s[8];
-  uint32_t t = 0u - r;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    t += a * gap[j] + corr[j];  // in (-p, p)
-    s[j] = min(t, t + p);       // t mod p: a negative t is a large unsigned
-  }
-  for (uint32_t x = 0; x < Lt; x += pmin) {  // s_j >= x in round x / pmin
+  const uint32_t period = 8u * p;
+  for (uint32_t start = 0; start < Lt; start += pmin) {  // no hit of round start / pmin lies below byte start
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      T.clear_or_spare(s[j], bit_mask(s[j], bit[j]));
-      s[j] += p;
+      T.clear_bit_or_spare(x[j]);
+      x[j] += period;
     }
   }
+}
+
+// x = *p (shared memory) if `yes`, as a predicated load.
+__device__ __forceinline__ void load_if(uint32_t& x, const uint32_t* p, bool yes) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred yes;\n\t"
+      "setp.ne.u32 yes, %2, 0;\n\t"
+      "@yes ld.shared.u32 %0, [%1];\n\t"
+      "}"
+      : "+r"(x)
+      : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"((uint32_t)yes)
+      : "memory");
 }
 
 __device__ __forceinline__ void sm_add(uint32_t* cnt, uint32_t idx, uint32_t* err) {
@@ -490,7 +508,7 @@ struct TileHdr {  // one tile's header (double-buffered: the next tile's is buil
   uint32_t interval, tile;
   uint32_t r0, r1;       // base primes lying in the tile (restore)
   uint32_t coop_ctr, b_ctr, w_ctr, c_ctr;  // work counters of the prime categories
-  uint32_t w_items, w_lo[8], w_n[8];  // primes taken by class: items of 32, first and number per class
+  uint32_t w_items, w_item, w_lo[8], w_n[8];  // primes taken by class: items, primes per item, first and number per class
   unsigned long long gword;         // the tile's first word in the large-prime bitmap
   uint32_t first;
 };
@@ -508,6 +526,7 @@ struct BlockScratch {
   int32_t block_max;
   uint32_t warp_sum[BLOCK / 32];
   unsigned long long warp_key[BLOCK / 32];
+  bool redo;
 };
 
 // Exclusive max-scan of `v` over thread order; returns the exclusive prefix and, through
@@ -572,46 +591,40 @@ __device__ __forceinline__ uint32_t block_excl_sum(uint32_t v, BlockScratch<BLOC
   return ex;
 }
 
+// The largest key of the block, to thread 0.
 template <int BLOCK>
-__device__ __forceinline__ void block_reduce_tile(uint32_t cnt, unsigned long long key,
-                                                  BlockScratch<BLOCK>& S, uint32_t* cnt_total,
-                                                  unsigned long long* key_max) {
+__device__ __forceinline__ void block_max_key(unsigned long long key, BlockScratch<BLOCK>& S,
+                                              unsigned long long* key_max) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
-    cnt += __shfl_down_sync(0xFFFFFFFFu, cnt, d);
     unsigned long long k2 = __shfl_down_sync(0xFFFFFFFFu, key, d);
     key = k2 > key ? k2 : key;
   }
-  if (lane == 0) {
-    S.warp_sum[warp] = cnt;
-    S.warp_key[warp] = key;
-  }
+  if (lane == 0) S.warp_key[warp] = key;
   __syncthreads();
   if (warp == 0) {
-    uint32_t c = lane < BLOCK / 32 ? S.warp_sum[lane] : 0;
     unsigned long long k = lane < BLOCK / 32 ? S.warp_key[lane] : 0ull;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
-      c += __shfl_down_sync(0xFFFFFFFFu, c, d);
       unsigned long long k2 = __shfl_down_sync(0xFFFFFFFFu, k, d);
       k = k2 > k ? k2 : k;
     }
-    if (lane == 0) {
-      *cnt_total = c;
-      *key_max = k;
-    }
+    if (lane == 0) *key_max = k;
   }
 }
 
-// Accumulator word of shared counter i.  The class counters fold: shared class c of the
-// (k mod 28) block is class c mod 28, of the (k mod 143) block class c mod 143.
+// Accumulator word of shared counter i, kNone for one that does not count (kSmSpare, distance 0).
+// The class counters fold: shared class c of the (k mod 28) block is class c mod 28, of the
+// (k mod 143) block class c mod 143.
 __device__ __forceinline__ uint32_t acc_index(uint32_t i) {
-  if (i < (uint32_t)kSmModq) return (uint32_t)kAccHist + i;
-  if (i < (uint32_t)kSmCls28) {
-    const uint32_t j = i - (uint32_t)kSmModq;  // 8 * bin + residue
-    return (uint32_t)kAccModq + (j & 7u) * (uint32_t)kModqBins + (j >> 3);
+  if (i < (uint32_t)kSmSpare) {
+    const uint32_t d = i >> 3, o = i & 7u;
+    if (d == 0) return kNone;
+    const uint32_t g = 30u * ((o + d) >> 3) + w30((o + d) & 7u) - w30(o);
+    return g < 2u * kModqBins ? (uint32_t)kAccModq + o * (uint32_t)kModqBins + (g >> 1) : (uint32_t)kAccHist + (g >> 1);
   }
+  if (i < (uint32_t)kSmCls28) return kNone;
   if (i < (uint32_t)kSmCls143) {
     const uint32_t c = (i - (uint32_t)kSmCls28) >> 3;
     return (uint32_t)kAccCls28 + 8u * (c >= 28u ? c - 28u : c) + (i & 7u);
@@ -685,7 +698,12 @@ __device__ __forceinline__ void tile_header(TileHdr& H, CtaState& St, const Siev
         H.w_lo[ln] = a.cls_first[ln] + lo;
         H.w_n[ln] = w_n;
       }
-      const uint32_t w_items = 8u * ((__reduce_max_sync(0xFFFFFFFFu, w_n) + 31u) >> 5);
+      // primes that a warp claims at a time: an item costs a claim and its class's constants (256
+      // against 128 and 64: 18.40, 18.70 and 19.35 ms for the 10^11 integers below 10^12), but few
+      // primes have to keep all warps busy
+      const uint32_t w_max = __reduce_max_sync(0xFFFFFFFFu, w_n);
+      const uint32_t w_item = w_max >= 4096u ? 256u : (w_max >= 1024u ? 128u : 32u);
+      const uint32_t w_items = 8u * ((w_max + w_item - 1u) / w_item);
       uint32_t r0 = a.n_primes, r1 = a.n_primes;
       if (vbase <= a.p_max) {
         r0 = count_lt_warp(a.primes, a.n_primes, vbase, ln);
@@ -730,6 +748,7 @@ __device__ __forceinline__ void tile_header(TileHdr& H, CtaState& St, const Siev
         H.b_ctr = 0;
         H.w_ctr = 0;
         H.w_items = w_items;
+        H.w_item = w_item;
         H.c_ctr = 0;
         H.first = kNone;
       }
@@ -800,7 +819,8 @@ sieve_tiles_kernel(SieveArgs a) {
       for (uint32_t i = tid; i < (uint32_t)kSmCounters; i += BLOCK) {
         uint32_t v = cnt[i];
         if (v) {
-          atomicAdd(acc + acc_index(i), (unsigned long long)v);
+          const uint32_t k = acc_index(i);
+          if (k != kNone) atomicAdd(acc + k, (unsigned long long)v);
           cnt[i] = 0;
         }
       }
@@ -831,13 +851,11 @@ sieve_tiles_kernel(SieveArgs a) {
     }
 
     // ---- 1. fill ----------------------------------------------------------------------
-    {
-      uint32_t ix[kPreGroups], st[kPreGroups];
-#pragma unroll
-      for (int g = 0; g < kPreGroups; ++g) {
-        ix[g] = (H.pre_base[g] + (uint32_t)tid) % pre_mod(g);
-        st[g] = (uint32_t)BLOCK % pre_mod(g);
-      }
+    // Thread c < 1001 writes the words w = c (mod 1001): the mask of 7 * 11 * 13 is then the
+    // thread's own constant, and the other tables' indices advance by fixed steps (three loads and
+    // one store per word; 26k warp instructions less per tile than words tid + BLOCK k from four
+    // tables with an edge test each).
+    if (tid < 1001 || BLOCK < 1001) {
       const uint64_t vbase = H.vbase, vlo = H.vlo, vhi = H.vhi;
       const uint32_t* gbm = a.gbm ? a.gbm + H.gword : nullptr;
       // words [w_in, w_out) lie wholly inside [vlo, vhi) (v0 + 1 >= vlo and v0 + 120 <= vhi):
@@ -845,20 +863,34 @@ sieve_tiles_kernel(SieveArgs a) {
       const uint64_t lo_words = vlo <= vbase + 1 ? 0ull : (vlo - vbase + 118ull) / 120ull;
       const uint64_t hi_words = vhi < vbase + 120 ? 0ull : (vhi - vbase) / 120ull;
       const uint32_t w_in = (uint32_t)(lo_words < a.tile_words ? lo_words : a.tile_words);
-      const uint32_t w_out = (uint32_t)(hi_words < a.tile_words ? hi_words : a.tile_words);
-#pragma unroll 4
-      for (uint32_t w = tid; w < a.tile_words; w += BLOCK) {
-        uint32_t m = 0;
-        if (w < nw) {
-          m = pre[ix[0]] & pre[1001u + ix[1]] & pre[1324u + ix[2]] & pre[1991u + ix[3]];
-          if (gbm) m &= gbm[w];
-          if (w < w_in || w >= w_out) m &= edge_mask(vbase + 120ull * w, vlo, vhi);
-        }
-        bm[w] = m;
+      const uint32_t w_out = (uint32_t)(hi_words < nw ? hi_words : nw);
+      for (uint32_t c = tid; c < 1001u; c += BLOCK) {
+        uint32_t i0 = H.pre_base[0] + c, ix[kPreGroups];
+        i0 -= i0 >= pre_mod(0) ? pre_mod(0) : 0u;
+        const uint32_t m0 = pre[i0];
 #pragma unroll
-        for (int g = 0; g < kPreGroups; ++g) {
-          ix[g] += st[g];
-          if (ix[g] >= pre_mod(g)) ix[g] -= pre_mod(g);
+        for (int g = 1; g < kPreGroups; ++g) ix[g] = (H.pre_base[g] + c) % pre_mod(g);
+        auto mask = [&] {
+          const uint32_t m = m0 & pre[pre_off(1) + ix[1]] & pre[pre_off(2) + ix[2]] & pre[pre_off(3) + ix[3]];
+#pragma unroll
+          for (int g = 1; g < kPreGroups; ++g) {
+            ix[g] += 1001u % pre_mod(g);
+            ix[g] = min(ix[g], ix[g] - pre_mod(g));
+          }
+          return m;
+        };
+        uint32_t w = c;
+        if (gbm || w < w_in) {
+          for (; w < nw; w += 1001u) {
+            uint32_t m = mask();
+            if (gbm) m &= gbm[w];
+            if (w < w_in || w >= w_out) m &= edge_mask(vbase + 120ull * w, vlo, vhi);
+            bm[w] = m;
+          }
+        } else {
+#pragma unroll 4
+          for (; w < w_out; w += 1001u) bm[w] = mask();
+          for (; w < nw; w += 1001u) bm[w] = mask() & edge_mask(vbase + 120ull * w, vlo, vhi);
         }
       }
     }
@@ -912,22 +944,44 @@ sieve_tiles_kernel(SieveArgs a) {
           }
         }
         // few hits per tile: a thread per prime of a class, 32 primes of one class at a time (item
-        // i: class i mod 8, its (i / 8)-th group; the classes hold nearly equal numbers of primes)
+        // i: class i mod 8, its (i / 8)-th item; the classes hold nearly equal numbers of primes)
         const double kd = (double)ktile;
-        const uint32_t w_end = H.w_items;
+        const uint32_t w_end = H.w_items, w_item = H.w_item;
         for (;;) {
           uint32_t it = 0;
           if (lane == 0) it = atomicAdd(&H.w_ctr, 1u);
           it = __shfl_sync(0xFFFFFFFFu, it, 0);
           if (it >= w_end) break;
-          const uint32_t c = it & 7u, k = 32u * (it >> 3), n = H.w_n[c];
+          const uint32_t c = it & 7u, n = H.w_n[c];
+          uint32_t k = w_item * (it >> 3);
           if (k >= n) continue;
-          const bool live = k + (uint32_t)lane < n;
-          const uint32_t i = H.w_lo[c] + (live ? k + (uint32_t)lane : n - 1u);  // idle lanes repeat the last prime
-          const uint32_t p = a.cls_primes[i];
-          const double inv = a.cls_inv[i];
-          const uint32_t r = mod_by_inv(ktile, kd, p, inv);
-          clear_class_primes(T, p, r, __shfl_sync(0xFFFFFFFFu, p, 0), c, Lt);
+          ClassStep C;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint2 e = c_cls_step[8u * c + j];
+            C.corr[j] = e.x;
+            C.bit[j] = e.y;
+          }
+          const uint32_t k_end = min(n, k + w_item);
+          const uint32_t* pp = a.cls_primes + H.w_lo[c];
+          const double* pi = a.cls_inv + H.w_lo[c];
+          // idle lanes repeat the last prime; the next 32 primes are loaded ahead
+          uint32_t i = min(k + (uint32_t)lane, n - 1u);
+          uint32_t p = pp[i];
+          double inv = pi[i];
+          for (;;) {
+            const uint32_t p_now = p;
+            const double inv_now = inv;
+            k += 32u;
+            if (k < k_end) {
+              i = min(k + (uint32_t)lane, n - 1u);
+              p = pp[i];
+              inv = pi[i];
+            }
+            const uint32_t r = mod_by_inv(ktile, kd, p_now, inv_now);
+            clear_class_primes(T, p_now, r, __shfl_sync(0xFFFFFFFFu, p_now, 0), C, Lt);
+            if (k >= k_end) break;
+          }
         }
       } else {
         // a lane per (prime, residue): a warp takes 4 consecutive primes, lane = 8*prime + residue
@@ -1032,7 +1086,7 @@ sieve_tiles_kernel(SieveArgs a) {
       for (uint32_t w = cend; pc && w > c0;) {  // the chunk's last prime: its last non-zero word
         const uint32_t x = bm[--w];
         if (x) {
-          my_last = (int32_t)(120u * w + s_pos[31u - (uint32_t)__clz(x)]);
+          my_last = (int32_t)(32u * w + 31u - (uint32_t)__clz(x));
           break;
         }
       }
@@ -1076,108 +1130,161 @@ sieve_tiles_kernel(SieveArgs a) {
         }
         if (k) {  // the primes of that word before mine: the last of them is my predecessor
           for (; k > 1u; --k) x &= x - 1u;
-          prev = (int32_t)(120u * w + s_pos[(uint32_t)__ffs(x) - 1u]);
+          prev = (int32_t)(32u * w + (uint32_t)__ffs(x) - 1u);
           x &= x - 1u;
         } else {  // mine is the word's first prime: the predecessor is in an earlier word
           prev = s_before[lo];
           for (uint32_t ww = w; ww > lo * C;) {
             const uint32_t y = bm[--ww];
             if (y) {
-              prev = (int32_t)(120u * ww + s_pos[31u - (uint32_t)__clz(y)]);
+              prev = (int32_t)(32u * ww + 31u - (uint32_t)__clz(y));
               break;
             }
           }
         }
       }
-      const uint32_t vb = H.vb;
+      // The walk works in bitmap bits (bit 8k + o of the tile = integer 30k + W30[o]): one counter
+      // per (distance d, residue of the lower prime), no conversion to integers.  Only gaps of at
+      // least t_far bits are looked at closer (far_gap): t_far is such that every large-gap
+      // candidate is one (a gap of g holds at least 8g/30 - 0.87 bits), and about sixteen others of
+      // the tile, so that the longest gap is found among them.  If it is not clear that it was (a
+      // gap below t_far bits is below 3.75 t_far), the tile's gaps are gone through again.
+      // Bound by issue slots: 205k warp instructions per tile of 218,000 primes (near 10^12), against
+      // 294k with positions as integers, a branch per reload and the longest gap tracked per prime.
       const uint32_t cthr = H.cthr;
+      uint32_t t_far;
+      {
+        const float bits = 32.0f * (float)nw / (float)(tile_cnt | 1u);
+        const float t = bits * __logf((float)(tile_cnt | 1u) * (1.0f / 16.0f));
+        t_far = t < 1.0f ? 1u : (t > (float)kGapBits ? kGapBits : (uint32_t)t);
+        if (cthr < 2u * kGapBits * 15u / 8u) t_far = min(t_far, max(1u, 8u * cthr / 30u));
+      }
       uint32_t mg = 0, mlo = 0;
-      uint32_t o_prev = 0;  // wheel residue of the previous prime (modq counters: 8 * (g / 2) + o)
-      if (prev >= 0) {
-        const uint32_t kp = (uint32_t)prev / 30u;
-        o_prev = (uint32_t)s_rb[(uint32_t)prev - 30u * kp];
-      }
-      uint32_t wpos = 120u * w;
-      uint32_t it0 = 0;
-      if (prev < 0 && n_mine) {
-        // the tile's first prime: no predecessor in the tile (exactly one thread)
-        while (x == 0u) {
-          x = bm[++w];
-          wpos += 120u;
-        }
-        const uint32_t b = (uint32_t)__ffs(x) - 1u;
-        x &= x - 1u;
-        const uint32_t pos = wpos + s_pos[b];
-        H.first = pos;
-        prev = (int32_t)pos;
-        o_prev = b & 7u;
-        it0 = 1;
-      }
-      uint32_t pv = (uint32_t)prev;
-      // Instantiated twice: in a tile without a segment boundary (vb = kNone, nearly all of
-      // them) the crossing test drops out of the loop.
-      auto walk = [&](auto cross_tag) {
-        constexpr bool kCross = decltype(cross_tag)::value;
-        // unrolled by 4: one trip-count test per four primes (the count is known at entry)
-#pragma unroll 4
-        for (uint32_t it = it0; it < n_mine; ++it) {
-          while (x == 0u) {  // the tile holds rb >= ra + it + 1 primes: w stays inside it
-            x = bm[++w];
-            wpos += 120u;
-          }
-          const uint32_t b = (uint32_t)__ffs(x) - 1u;
-          x &= x - 1u;
-          const uint32_t pos = wpos + s_pos[b];
-          const uint32_t g = pos - pv;
-          const bool crossing = kCross && (pv < vb) && (pos >= vb);
-          const bool small = g < 100u && !crossing;
-          if (small || g < 2u * kHistBins) {
-            sm_add(cnt, small ? (uint32_t)kSmModq + 4u * g + o_prev : (uint32_t)kSmHist + (g >> 1), err);
+      auto value = [&](uint32_t bit) { return 120u * (bit >> 5) + s_pos[bit & 31u]; };
+      auto far_gap = [&](uint32_t lo_bit, uint32_t hi_bit, bool crossing) {
+        const uint32_t pv = value(lo_bit), pos = value(hi_bit), g = pos - pv;
+        if (crossing || hi_bit - lo_bit >= kGapBits) {  // not counted in shared memory
+          unsigned long long* acc = a.acc + (size_t)H.interval * kAccStride;
+          if (g < 2u * kHistBins) {
+            atomicAdd(acc + kAccHist + (g >> 1), 1ull);
           } else {
-            atomicAdd(a.acc + (size_t)H.interval * kAccStride + kAccHistOver, 1ull);
+            atomicAdd(acc + kAccHistOver, 1ull);
             const uint32_t slot = atomicAdd(a.over_count, 1u);
             if (slot < a.over_cap) a.over[slot] = OverflowGap{H.interval, g};
             else atomicOr(err, kErrOverflowList);
           }
-          mlo = g > mg ? pv : mlo;
-          mg = g > mg ? g : mg;
-          if (g >= cthr && !crossing) {
-            const uint64_t v0 = H.vbase + pv;
-            const double merit_d = (double)g / log((double)v0);
-            if (a.large_min_gap || g >= 500u || merit_d >= 10.0) {
-              const uint32_t slot = atomicAdd(a.large_count, 1u);
-              if (slot < a.large_cap) {
-                a.large[slot] = LargeGapDev{H.vbase + pos, (int32_t)g, (float)merit_d};
-                a.large_iv[slot] = H.interval;
-              }
+        }
+        mlo = g > mg ? pv : mlo;
+        mg = g > mg ? g : mg;
+        if (g >= cthr && !crossing) {
+          const uint64_t v0 = H.vbase + pv;
+          const double merit_d = (double)g / log((double)v0);
+          if (a.large_min_gap || g >= 500u || merit_d >= 10.0) {
+            const uint32_t slot = atomicAdd(a.large_count, 1u);
+            if (slot < a.large_cap) {
+              a.large[slot] = LargeGapDev{H.vbase + pos, (int32_t)g, (float)merit_d};
+              a.large_iv[slot] = H.interval;
             }
           }
-          pv = pos;
-          o_prev = b & 7u;
+        }
+      };
+      uint32_t it0 = 0;
+      if (prev < 0 && n_mine) {
+        // the tile's first prime: no predecessor in the tile (exactly one thread)
+        while (x == 0u) x = bm[++w];
+        const uint32_t b = (uint32_t)__ffs(x) - 1u;
+        x &= x - 1u;
+        prev = (int32_t)(32u * w + b);
+        H.first = value((uint32_t)prev);
+        it0 = 1;
+      }
+      if (n_mine > it0)
+        while (x == 0u) x = bm[++w];  // the tile holds primes of this thread: w stays inside it
+      uint32_t pv = (uint32_t)prev;
+      const uint32_t vb = H.vb == kNone ? kNone : 8u * (H.vb / 30u);  // the boundary's first bit
+      // Instantiated twice: in a tile without a segment boundary (nearly all of them) the crossing
+      // test drops out of the loop.
+      auto walk = [&](auto cross_tag) {
+        constexpr bool kCross = decltype(cross_tag)::value;
+        uint32_t left = n_mine - it0;
+        // All but the last prime, the warp's lanes side by side: the next word is a predicated load,
+        // and one vote covers what is rare, a far gap or a word without primes (a branch of its own
+        // for the reload diverges at nearly every prime).
+        const uint32_t common = __reduce_min_sync(0xFFFFFFFFu, left);
+#pragma unroll 4
+        for (uint32_t it = 1; it < common; ++it) {
+          const uint32_t bit = 32u * w + (uint32_t)__ffs(x) - 1u;
+          x &= x - 1u;
+          const bool spent = x == 0u;
+          w += spent ? 1u : 0u;
+          load_if(x, bm + w, spent);
+          const uint32_t d = bit - pv;
+          const bool crossing = kCross && (pv < vb) && (bit >= vb);
+          const uint32_t slot = min(8u * d + (pv & 7u), (uint32_t)kSmSpare);
+          sm_add(cnt, crossing ? (uint32_t)kSmSpare : slot, err);
+          const bool far = d >= t_far || crossing;
+          if (__any_sync(0xFFFFFFFFu, far || x == 0u)) {
+            if (far) far_gap(pv, bit, crossing);
+            while (x == 0u) x = bm[++w];  // this lane has primes left: w stays inside the tile
+          }
+          pv = bit;
+        }
+        left -= common ? common - 1u : 0u;
+        for (; left; --left) {
+          while (x == 0u) x = bm[++w];
+          const uint32_t bit = 32u * w + (uint32_t)__ffs(x) - 1u;
+          x &= x - 1u;
+          const uint32_t d = bit - pv;
+          const bool crossing = kCross && (pv < vb) && (bit >= vb);
+          const uint32_t slot = min(8u * d + (pv & 7u), (uint32_t)kSmSpare);
+          sm_add(cnt, crossing ? (uint32_t)kSmSpare : slot, err);
+          if (d >= t_far || crossing) far_gap(pv, bit, crossing);
+          pv = bit;
         }
       };
       if (vb == kNone) walk(std::false_type{});
       else walk(std::true_type{});
-      const unsigned long long key =
-          mg ? (((unsigned long long)mg << 32) | (unsigned long long)(0xFFFFFFFFu - mlo)) : 0ull;
-      uint32_t tile_cnt2;
-      unsigned long long tile_key;
-      __syncthreads();  // H.first visible, scratch reuse
-      VOSS_PHASE(8)
-      block_reduce_tile<BLOCK>(n_mine, key, S, &tile_cnt2, &tile_key);
-      (void)tile_cnt2;  // = tile_cnt
-      if (tid == 0) {
+      auto gap_key = [&] {
+        return mg ? (((unsigned long long)mg << 32) | (unsigned long long)(0xFFFFFFFFu - mlo)) : 0ull;
+      };
+      auto store_partial = [&](unsigned long long key) {
         TilePartial P;
         P.first = tile_cnt ? H.first : kNone;
-        P.last = tile_cnt ? (uint32_t)tile_last : kNone;
+        P.last = tile_cnt ? value((uint32_t)tile_last) : kNone;
         P.count = tile_cnt;
-        P.max_gap = (uint32_t)(tile_key >> 32);
-        P.max_lo = tile_key ? 0xFFFFFFFFu - (uint32_t)(tile_key & 0xFFFFFFFFull) : 0u;
+        P.max_gap = (uint32_t)(key >> 32);
+        P.max_lo = key ? 0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFull) : 0u;
         P.bgap = 0;
         P.bgap_lo = 0;
         a.partials[H.tile] = P;
+      };
+      unsigned long long tile_key;
+      __syncthreads();  // H.first visible, scratch reuse
+      VOSS_PHASE(8)
+      block_max_key<BLOCK>(gap_key(), S, &tile_key);
+      if (tid == 0) {
+        store_partial(tile_key);
+        S.redo = tile_cnt >= 2u && 4u * (uint32_t)(tile_key >> 32) < 15u * t_far;
         St.count_total += tile_cnt;
         St.since_flush++;
+      }
+      __syncthreads();
+      if (S.redo) {  // the longest gap may be a short one: every chunk's gaps in order
+        mg = mlo = 0;
+        int32_t pb = s_before[tid];
+        for (uint32_t ww = c0; ww < cend; ++ww) {
+          for (uint32_t y = bm[ww]; y; y &= y - 1u) {
+            const uint32_t bit = 32u * ww + (uint32_t)__ffs(y) - 1u;
+            if (pb >= 0) {
+              const uint32_t lo_v = value((uint32_t)pb), g = value(bit) - lo_v;
+              mlo = g > mg ? lo_v : mlo;
+              mg = g > mg ? g : mg;
+            }
+            pb = (int32_t)bit;
+          }
+        }
+        block_max_key<BLOCK>(gap_key(), S, &tile_key);
+        if (tid == 0) store_partial(tile_key);
       }
     }
     cur ^= 1u;

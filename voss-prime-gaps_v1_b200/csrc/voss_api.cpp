@@ -121,7 +121,7 @@ int apply_tuning(voss_ctx* c, const voss_tuning& t0) {
   if (!t.chunk_words) t.chunk_words = t.block_threads == 1024 ? 49 : 45;
   if (!t.coop_div) t.coop_div = 80;
   if (!t.mult_factor) t.mult_factor = 8;
-  if (!t.walk_sixteenths) t.walk_sixteenths = 4;
+  if (!t.walk_sixteenths) t.walk_sixteenths = 2;
   if (!t.mr_route) t.mr_route = 50;
   if (t.block_threads != 512 && t.block_threads != 1024)
     return fail(VOSS_ERR_ARG, "block_threads must be 512 or 1024");

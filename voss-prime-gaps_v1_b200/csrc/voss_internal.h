@@ -49,16 +49,20 @@ constexpr int kAccCls143 = kAccCls28 + kCls28;              // 1650
 constexpr int kAccUsed = kAccCls143 + kCls143;              // 2794
 constexpr int kAccStride = 2800;
 
-// Shared-memory counter block (u32), same order as the accumulator from kAccHist on, except
-// that the class blocks are not wrapped: byte j of a word whose first byte has class c counts
-// in class c + j (up to 30 and 145), and the flush adds classes 28..30 / 143..145 to 0..2.
+// Shared-memory counter block (u32).  Gaps are counted by their distance in bitmap bits: counter
+// 8 d + o is a gap of d < kGapBits bits above a prime of wheel residue o (the flush turns it into
+// the accumulators' (residue, g < 100) or g bins; longer gaps go to the accumulators directly, and
+// kSmSpare takes what must not be counted here).  The class blocks are not wrapped: byte j of a word
+// whose first byte has class c counts in class c + j (up to 30 and 145), and the flush adds
+// classes 28..30 / 143..145 to 0..2.
+constexpr uint32_t kGapBits = 64;
 constexpr int kSmCls28Rows = 28 + 3;
 constexpr int kSmCls143Rows = 143 + 3;
-constexpr int kSmHist = 0;
-constexpr int kSmModq = kSmHist + kHistBins;                // 1024
-constexpr int kSmCls28 = kSmModq + 8 * kModqBins;           // 1424
-constexpr int kSmCls143 = kSmCls28 + 8 * kSmCls28Rows;      // 1672
-constexpr int kSmCounters = kSmCls143 + 8 * kSmCls143Rows;  // 2840
+constexpr int kSmGap = 0;
+constexpr int kSmSpare = kSmGap + 8 * (int)kGapBits;        // 512
+constexpr int kSmCls28 = kSmSpare + 8;                      // 520
+constexpr int kSmCls143 = kSmCls28 + 8 * kSmCls28Rows;      // 768
+constexpr int kSmCounters = kSmCls143 + 8 * kSmCls143Rows;  // 1936
 
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
