@@ -194,14 +194,11 @@ VOSS_API int voss_mr_verify_device(voss_ctx* ctx, const uint64_t* d_n, uint64_t 
  * during the call: processes whose device memory is already reserved by another allocator (a
  * framework's caching allocator or a memory pool), and service request paths where
  * cudaMalloc/cudaFree would synchronize the device.  No counterpart in the reference.
- * It takes no context and allocates nothing: its scratch is a fixed array inside libvoss.so
- * (16 MiB, held on every device that loads the library until exit), so
+ * It takes no context and allocates nothing; it needs no scratch memory either, so
  *   - count may not exceed 4194304 (1 << 22) per call; larger counts return VOSS_ERR_ARG;
- *   - every call shares that array: calls that overlap on the GPU (different streams, or
- *     different host threads on one device) race; order them on one stream;
- *   - the first call on a device sets up (looks up the array's device address and uploads the
- *     Miller-Rabin constant tables) on the calling thread's current device; make that first
- *     call before any stream capture.
+ *   - calls may overlap on the GPU (different streams or host threads);
+ *   - the first call on a device uploads the trial-division constant tables on the calling
+ *     thread's current device; make that first call before any stream capture.
  * d_n and d_is_prime are device pointers on the current device; `stream` is a cudaStream_t or
  * NULL for the legacy default stream.  The call is asynchronous on `stream`. */
 VOSS_API int voss_mr_verify_noalloc(const uint64_t* d_n, uint64_t count, uint8_t* d_is_prime,

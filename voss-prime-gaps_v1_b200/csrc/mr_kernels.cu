@@ -6,14 +6,21 @@
 //   verify_gap (:59-93): both ends prime, then every interior integer must be marked by the
 //   interval sieve (evens, then odd multiples of the odd base primes q <= isqrt(p_after)).
 //
-// Arithmetic: 64-bit Montgomery multiplication with R = 2^64 (mul.lo/mul.hi on the integer
-// pipe, no 128-bit division); the reference's u128 '%' (verify_cpp.cpp:24) is not used.
-// Base 2 is special-cased: its square-and-multiply multiplies by 2 with a modular addition.
-// Work is split in two kernels so that warps stay full: mr_sieve_kernel resolves every
-// candidate that trial division or base 2 decides (nearly all composites) and appends the rest
-// to a work list; mr_finish_kernel runs the remaining bases on that list, as many as the size
-// of n requires for an exact verdict (bases_needed: 6, 7, 9 or all 12), so its results equal
-// the reference's twelve-base test for every 64-bit n.
+// The verdicts are exact for every 64-bit n, so they equal the reference's twelve strong
+// probable-prime tests, which are exact below 2^64 too.  They come from trial division by 2..37, a
+// strong probable-prime test to base 2 and, for its survivors, an extra strong Lucas test (Baillie
+// and Wagstaff 1980; Grantham 2001: the smallest P >= 3 with (P^2 - 4 | n) = -1, Q = 1): no
+// composite below 2^64 passes both (checked over Feitsma's list of all base-2 pseudoprimes below
+// 2^64; PARI's and FLINT's primality tests of 64-bit integers rest on the same fact).  The Lucas
+// test costs two products per bit, the five to eleven further bases it replaces 1.5 each.
+//
+// Arithmetic, by the size of n:
+//   n < 2^49: products mod n in double precision from exact fma halves (DMod): six operations of the
+//             fp64 pipe, 9.8 products per cycle and SM measured;
+//   others:   64-bit Montgomery multiplication with R = 2^64 (mul.lo/mul.hi on the integer pipe, no
+//             128-bit division), 2.36 per cycle and SM.
+// One kernel does all of it: candidates that trial division leaves open wait in per-warp queues by
+// test and size, and each time a queue holds 32 they are tested together, a lane each.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -35,24 +42,21 @@ static std::atomic<uint64_t> g_mr_ready{0};
 static const uint64_t kBases[12] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37};
 
 struct Mont {
-  uint64_t n, ninv, one, mone;
+  uint64_t n, inv, ninv, one, mone;  // inv = n^-1, ninv = -n^-1 (mod 2^64); one = 2^64 mod n, mone = n - one
 };
 
+// a b / 2^64 mod n for a, b < n: with m = (a b) n^-1 mod 2^64 the low halves of a b and m n agree, so
+// the quotient is the difference of the high halves, without a carry; one conditional addition.
 __device__ __forceinline__ uint64_t mont_mul(uint64_t a, uint64_t b, const Mont& M) {
   const uint64_t lo = a * b;
   const uint64_t hi = __umul64hi(a, b);
-  const uint64_t m = lo * M.ninv;
-  const uint64_t mh = __umul64hi(m, M.n);
-  // (a*b + m*n) / 2^64 = hi + mh + carry, carry = (lo != 0) because lo + (m*n mod 2^64) = 0 mod 2^64
-  const uint64_t t = hi + mh;
-  const bool c1 = t < hi;
-  const uint64_t t2 = t + (lo != 0 ? 1ull : 0ull);
-  const bool c2 = t2 < t;
-  return (c1 || c2 || t2 >= M.n) ? t2 - M.n : t2;
+  const uint64_t mh = __umul64hi(lo * M.inv, M.n);
+  const uint64_t t = hi - mh;
+  return hi < mh ? t + M.n : t;
 }
 
-// mont_mul for n < 2^63: hi + mh < 2n < 2^64 and the low-half carry keeps it <= 2n, so no
-// 64-bit overflow checks are needed.
+// The same for n < 2^63 as a sum: with m = -(a b) n^-1 the low halves add up to 2^64 (or 0), and
+// hi + mh + carry < 2n < 2^64 (2.36 products per cycle and SM against 2.22).
 __device__ __forceinline__ uint64_t mont_mul_small(uint64_t a, uint64_t b, const Mont& M) {
   const uint64_t lo = a * b;
   const uint64_t hi = __umul64hi(a, b);
@@ -87,6 +91,7 @@ __device__ __forceinline__ Mont mont_setup(uint64_t n) {
   uint64_t x = n;  // inverse of n mod 2^3
 #pragma unroll
   for (int i = 0; i < 5; ++i) x *= 2ull - n * x;
+  M.inv = x;
   M.ninv = 0ull - x;
   M.one = two64_mod(n);  // R mod n
   M.mone = n - M.one;
@@ -95,7 +100,7 @@ __device__ __forceinline__ Mont mont_setup(uint64_t n) {
 
 // Trial phase of is_prime_u64: 1 = prime, 0 = composite, -1 = undecided.
 __device__ __forceinline__ int trial_phase(uint64_t n) {
-  if (n < 2) return 0;
+  if (n < 2) return 0;  // (41^2 = 1681 is the smallest composite that stays undecided)
   if (n == 2) return 1;
   if ((n & 1ull) == 0) return 0;
 #pragma unroll
@@ -105,268 +110,332 @@ __device__ __forceinline__ int trial_phase(uint64_t n) {
     if (n == B) return 1;
     if (n * c_base_inv[i] <= c_base_lim[i]) return 0;
   }
+  if (n < 1681) return 1;
   return -1;
 }
 
-// How many of the bases 2, 3, 5, ..., 37 (in this order) decide primality exactly for n.  The
-// smallest strong pseudoprimes to the first k prime bases are 3,474,749,660,383 (k = 6),
-// 341,550,071,728,321 (k = 7, 8) and 3,825,123,056,546,413,051 (k = 9..11) (Jaeschke 1993; OEIS
-// A014233); below them the first 6, 7 or 9 bases already give the same verdict as all twelve,
-// which remain exact for every n < 2^64.
-__device__ __forceinline__ int bases_needed(uint64_t n) {
-  return n < 3474749660383ull ? 6 : (n < 341550071728321ull ? 7 : (n < 3825123056546413051ull ? 9 : 12));
-}
-constexpr uint64_t kSmallMr = 3474749660383ull;  // survivors below go to the front work list
+// ---- products mod n in double precision -------------------------------------------------------
+// For odd n in [1681, 2^49) and integers |a|, |b| < n (a doubled factor below 2n is allowed too): an
+// integer r = a b (mod n) with |r| < n, all values exact in doubles.  h = a b rounded and l = a b - h
+// (fma, exact); q = h / n rounded to an integer by adding 1.5 * 2^52 in the same rounding; h - q n is
+// an integer below 2^53, so the fma that computes it is exact.  |q - h/n| <= 1/2 + |h/n| 2^-53 (the
+// rounding of 1/n) and |l| <= |h| 2^-53 <= (|a b| / n) n 2^-53, so with |a b| <= 2 B^2 n^2 and n < 2^49
+// |r| <= (1/2 + B^2 / 4) n: B = 0.59 reproduces itself.
+constexpr uint64_t kDModEnd = 1ull << 49;
+struct DMod {
+  double n, inv;
+};
 
-// Strong probable-prime test of odd n > 37 to the base whose Montgomery form is am.
-__device__ __forceinline__ bool sprp(const Mont& M, uint64_t am, uint64_t d, int r) {
-  uint64_t x = M.one;
-  const int top = 63 - __clzll(d);
-  for (int b = top; b >= 0; --b) {
-    x = mont_mul(x, x, M);
-    if ((d >> b) & 1ull) x = mont_mul(x, am, M);
-  }
-  if (x == M.one || x == M.mone) return true;
-  for (int j = 0; j < r - 1; ++j) {
-    x = mont_mul(x, x, M);
-    if (x == M.mone) return true;
-  }
-  return false;
+__device__ __forceinline__ DMod dmod_setup(uint64_t n) {
+  DMod M;
+  M.n = (double)n;
+  M.inv = __drcp_rn(M.n);
+  return M;
 }
 
-__device__ __forceinline__ bool sprp2(const Mont& M, uint64_t d, int r) {
-  uint64_t x = M.one;
-  const int top = 63 - __clzll(d);
-  for (int b = top; b >= 0; --b) {
-    x = mont_mul(x, x, M);
-    if ((d >> b) & 1ull) x = mod_add(x, x, M.n);
-  }
-  if (x == M.one || x == M.mone) return true;
-  for (int j = 0; j < r - 1; ++j) {
-    x = mont_mul(x, x, M);
-    if (x == M.mone) return true;
-  }
-  return false;
+__device__ __forceinline__ double dmod_mul(double a, double b, const DMod& M) {
+  constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
+  const double h = a * b;
+  const double l = __fma_rn(a, b, -h);
+  const double q = __fma_rn(h, M.inv, kRound) - kRound;
+  return __fma_rn(-q, M.n, h) + l;
 }
 
-// Bases 3..37 (Montgomery forms built from R by modular additions).
-__device__ __forceinline__ bool sprp_rest(const Mont& M, uint64_t d, int r) {
-  const uint64_t n = M.n;
-  const uint64_t r1 = M.one, r2 = mod_add(r1, r1, n), r4 = mod_add(r2, r2, n), r6 = mod_add(r4, r2, n);
-  uint64_t a = mod_add(r2, r1, n);  // 3R
-  // gaps between consecutive bases 3,5,7,11,13,17,19,23,29,31,37
-  const int steps[10] = {2, 2, 4, 2, 4, 2, 4, 6, 2, 6};
-  if (!sprp(M, a, d, r)) return false;
-#pragma unroll
-  for (int i = 0; i < 10; ++i) {
-    const int s = steps[i];
-    a = mod_add(a, s == 2 ? r2 : (s == 4 ? r4 : r6), n);
-    if (!sprp(M, a, d, r)) return false;
+// ---- strong probable-prime test to base 2 -----------------------------------------------------
+// Warp-uniform: every lane runs the same number of squarings (the warp's longest exponent and
+// largest r) and keeps its verdict in a flag.  Early exits inside these loops let the lanes of a
+// warp drift apart and never reconverge (measured: 2.8 active lanes per instruction).
+struct OddPart {
+  uint64_t d;  // m = d 2^r
+  int r, top_w, r_w;  // top_w, r_w: the warp's longest d (index of the top bit) and largest r
+};
+
+__device__ __forceinline__ OddPart odd_part(uint64_t m) {
+  OddPart E;
+  E.r = __ffsll((long long)m) - 1;
+  E.d = m >> E.r;
+  E.top_w = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)(63 - __clzll(E.d)));
+  E.r_w = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)E.r);
+  return E;
+}
+
+__device__ __forceinline__ bool sprp2(const DMod& M, const OddPart& E) {
+  // the top five bits of the exponent at once: 2^e <= 2^31 reduced by one product
+  int b = E.top_w > 4 ? E.top_w - 4 : 0;
+  double x = dmod_mul((double)(1u << (uint32_t)(E.d >> b)), 1.0, M);
+  for (--b; b >= 0; --b) {
+    const double y = x + x;
+    x = dmod_mul(x, ((E.d >> b) & 1ull) ? y : x, M);
   }
-  return true;
+  bool ok = (x == 1.0) | (x == -1.0);
+  for (int j = 0; j < E.r_w - 1; ++j) {
+    x = dmod_mul(x, x, M);
+    ok |= (j < E.r - 1) & (x == -1.0);
+  }
+  return ok;
 }
 
-__device__ bool is_prime_u64_dev(uint64_t n) {
-  const int t = trial_phase(n);
-  if (t >= 0) return t == 1;
-  const Mont M = mont_setup(n);
-  uint64_t d = n - 1;
-  const int r = __ffsll((long long)d) - 1;
-  d >>= r;
-  if (!sprp2(M, d, r)) return false;
-  return sprp_rest(M, d, r);
-}
-
-// Warp-uniform strong probable-prime test: every lane runs the same number of squarings and
-// multiplications (the warp's longest exponent and largest r) and keeps its verdict in a flag.
-// Early exits inside these loops let the lanes of a warp drift apart and never reconverge
-// (measured: 2.8 active lanes per instruction); uniform loops keep all 32 lanes in step.
 // kSmallN: every lane's n < 2^63 (mont_mul_small).
-template <bool kSmallN = false>
-__device__ __forceinline__ bool sprp_uniform(const Mont& M, uint64_t am, uint64_t d, int r, int top_w, int r_w,
-                                             bool base2) {
+template <bool kSmallN>
+__device__ __forceinline__ uint64_t mont_product(uint64_t a, uint64_t b, const Mont& M) {
+  return kSmallN ? mont_mul_small(a, b, M) : mont_mul(a, b, M);
+}
+
+template <bool kSmallN>
+__device__ __forceinline__ bool sprp2(const Mont& M, const OddPart& E) {
   uint64_t x = M.one;
-  for (int b = top_w; b >= 0; --b) {
-    x = kSmallN ? mont_mul_small(x, x, M) : mont_mul(x, x, M);
-    const uint64_t y = base2 ? mod_add(x, x, M.n) : (kSmallN ? mont_mul_small(x, am, M) : mont_mul(x, am, M));
-    x = ((d >> b) & 1ull) ? y : x;
+  for (int b = E.top_w; b >= 0; --b) {
+    x = mont_product<kSmallN>(x, x, M);
+    const uint64_t y = mod_add(x, x, M.n);
+    x = ((E.d >> b) & 1ull) ? y : x;
   }
   bool ok = (x == M.one) | (x == M.mone);
-  for (int j = 0; j < r_w - 1; ++j) {
-    x = kSmallN ? mont_mul_small(x, x, M) : mont_mul(x, x, M);
-    ok |= (j < r - 1) & (x == M.mone);
+  for (int j = 0; j < E.r_w - 1; ++j) {
+    x = mont_product<kSmallN>(x, x, M);
+    ok |= (j < E.r - 1) & (x == M.mone);
   }
   return ok;
 }
 
-// sprp_uniform for a base whose products are real multiplications, with 2-bit exponent digits:
-// x <- x^4 * a^digit for each digit of d from the top, a^0 = R, a, a^2, a^3 precomputed and
-// picked by selects (no memory).  A base then costs about 1.5 products per bit of d instead of
-// the 2 of the bitwise loop, which must multiply at every bit because some lane's bit is set.
+// ---- extra strong Lucas test --------------------------------------------------------------------
+// Jacobi symbol (a | n) for odd n and 0 < a < 2^32.
+__device__ inline int jacobi(uint32_t a, uint64_t n) {
+  int j = 1;
+  int z = __ffs((int)a) - 1;
+  a >>= z;
+  if ((z & 1) && ((n & 7) == 3 || (n & 7) == 5)) j = -j;
+  if ((a & 3) == 3 && (n & 3) == 3) j = -j;
+  uint32_t b = (uint32_t)(n % a);  // (a | n) = +-(n mod a | a)
+  while (b) {
+    z = __ffs((int)b) - 1;
+    b >>= z;
+    if ((z & 1) && ((a & 7) == 3 || (a & 7) == 5)) j = -j;
+    if ((a & 3) == 3 && (b & 3) == 3) j = -j;
+    const uint32_t t = a % b;
+    a = b;
+    b = t;
+  }
+  return a == 1 ? j : 0;
+}
+
+// The smallest P >= 3 with (P^2 - 4 | n) = -1 for odd n without prime factors up to 37; 0 when n is
+// found composite on the way (a perfect square, for which there is none, or a common factor).
+// P^2 - 4 = 5, 12, 21, 32, 45, 60, 77, 96, 117, ...: while the symbols of the primes up to 13 are
+// all +1, only 5, 3, 7, 2, 11, 13, 17, 19 bring a new one, at P = 3, 4, 5, 6, 9, 11, 15, 17.
+__device__ __forceinline__ uint32_t lucas_p(uint64_t n) {
+  const uint32_t m = (uint32_t)(n % 4849845ull);  // 3 * 5 * 7 * 11 * 13 * 17 * 19
+  const uint32_t n3 = (uint32_t)(n >> 1) & 1u;    // n = 3 (mod 4): (q | n) = -(n | q) for q = 3 (mod 4)
+  const uint32_t n8 = (uint32_t)n & 7u;
+  // bit n mod q of the masks: non-residues of q
+  const uint32_t b5 = (0xCu >> (m % 5u)) & 1u, b3 = ((0x4u >> (m % 3u)) & 1u) ^ n3;
+  const uint32_t b7 = ((0x68u >> (m % 7u)) & 1u) ^ n3, b2 = (n8 == 3u || n8 == 5u) ? 1u : 0u;
+  const uint32_t b11 = ((0x5C4u >> (m % 11u)) & 1u) ^ n3, b13 = (0x9E4u >> (m % 13u)) & 1u;
+  const uint32_t b17 = (0x5CE8u >> (m % 17u)) & 1u, b19 = ((0x4F50Cu >> (m % 19u)) & 1u) ^ n3;
+  const uint32_t minus = b5 | b3 << 1 | b7 << 2 | b2 << 3 | b11 << 4 | b13 << 5 | b17 << 6 | b19 << 7;
+  if (minus) return (uint32_t)(0x110F0B0906050403ull >> (8 * (__ffs((int)minus) - 1))) & 0xFFu;
+  const uint64_t s = (uint64_t)sqrt((double)n);
+  for (uint64_t t = s > 0 ? s - 1 : 0; t <= s + 1 && t <= 0xFFFFFFFFull; ++t)
+    if (t * t == n) return 0;
+  for (uint32_t P = 20;; ++P) {  // n is no square: half of all symbols are -1
+    const int j = jacobi(P * P - 4u, n);
+    if (j == -1) return P;
+    if (j == 0) return 0;
+  }
+}
+
+// n + 1 = d 2^s: passes if U_d = 0 and V_d = +-2, or V_{d 2^r} = 0 for some 0 <= r < s - 1 (mod n).
+// The ladder holds (V_k, V_{k+1}): V_{2k} = V_k^2 - 2, V_{2k+1} = V_k V_{k+1} - P, two products per
+// bit.  U_d = 0 <=> 2 V_{d+1} = P V_d, i.e. V_{d+1} = P or -P beside V_d = 2 or -2.  All lanes start from
+// (V_0, V_1) = (2, P), which leading zero bits leave alone, so they share one trip count.
+__device__ __forceinline__ bool lucas(const DMod& M, const OddPart& E, uint32_t P) {
+  const double p = (double)P;
+  double v = 2.0, w = p;
+  for (int b = E.top_w; b >= 0; --b) {
+    const bool one = (E.d >> b) & 1ull;
+    const double t = dmod_mul(v, w, M) - p;
+    const double x = one ? w : v;
+    const double y = dmod_mul(x, x, M) - 2.0;
+    v = one ? t : y;
+    w = one ? y : t;
+  }
+  bool ok = (v == 2.0 && w == p) | (v == -2.0 && w == -p);
+  ok |= (E.r > 1) & (v == 0.0);
+  for (int j = 1; j < E.r_w - 1; ++j) {
+    v = dmod_mul(v, v, M) - 2.0;
+    ok |= (j < E.r - 1) & (v == 0.0);
+  }
+  return ok;
+}
+
+__device__ __forceinline__ uint64_t mod_sub(uint64_t a, uint64_t b, uint64_t n) {
+  return a >= b ? a - b : a - b + n;
+}
+
 template <bool kSmallN>
-__device__ __forceinline__ bool sprp_uniform_w2(const Mont& M, uint64_t am, uint64_t d, int r, int top_w, int r_w) {
-  const uint64_t a2 = kSmallN ? mont_mul_small(am, am, M) : mont_mul(am, am, M);
-  const uint64_t a3 = kSmallN ? mont_mul_small(a2, am, M) : mont_mul(a2, am, M);
-  // an odd number of bits (top_w even) starts with the single top bit, then bit pairs (b, b - 1)
-  uint64_t x;
-  int b;
-  if ((top_w & 1) == 0) {
-    x = ((d >> top_w) & 1ull) ? am : M.one;
-    b = top_w - 1;
+__device__ __forceinline__ bool lucas(const Mont& M, const OddPart& E, uint32_t P) {
+  const uint64_t n = M.n, two = mod_add(M.one, M.one, n);
+  uint64_t p = 0;  // P R mod n by doubling
+  for (int b = 31 - __clz((int)P); b >= 0; --b) {
+    p = mod_add(p, p, n);
+    if ((P >> b) & 1u) p = mod_add(p, M.one, n);
+  }
+  uint64_t v = two, w = p;
+  for (int b = E.top_w; b >= 0; --b) {
+    const bool one = (E.d >> b) & 1ull;
+    const uint64_t t = mod_sub(mont_product<kSmallN>(v, w, M), p, n);
+    const uint64_t x = one ? w : v;
+    const uint64_t y = mod_sub(mont_product<kSmallN>(x, x, M), two, n);
+    v = one ? t : y;
+    w = one ? y : t;
+  }
+  bool ok = (v == two && w == p) | (v == n - two && w == n - p);
+  ok |= (E.r > 1) & (v == 0);
+  for (int j = 1; j < E.r_w - 1; ++j) {
+    v = mod_sub(mont_product<kSmallN>(v, v, M), two, n);
+    ok |= (j < E.r - 1) & (v == 0);
+  }
+  return ok;
+}
+
+// The two tests of a warp's 32 candidates, all of one size class (kDouble: n < kDModEnd).
+template <bool kDouble>
+__device__ __forceinline__ bool test_base2(uint64_t n) {
+  const OddPart E = odd_part(n - 1);
+  if (kDouble) return sprp2(dmod_setup(n), E);
+  const Mont M = mont_setup(n);
+  return __all_sync(0xFFFFFFFFu, n < (1ull << 63)) ? sprp2<true>(M, E) : sprp2<false>(M, E);
+}
+
+template <bool kDouble>
+__device__ __forceinline__ bool test_lucas(uint64_t n) {
+  const uint32_t P = lucas_p(n);
+  __syncwarp();
+  const OddPart E = odd_part(n + 1);  // n + 1 < 2^64: 2^64 - 1 has small factors
+  bool ok;
+  if (kDouble) {
+    ok = lucas(dmod_setup(n), E, P);
   } else {
-    const uint32_t g = (uint32_t)(d >> (top_w - 1)) & 3u;
-    x = g == 0u ? M.one : (g == 1u ? am : (g == 2u ? a2 : a3));
-    b = top_w - 2;
+    const Mont M = mont_setup(n);
+    ok = __all_sync(0xFFFFFFFFu, n < (1ull << 63)) ? lucas<true>(M, E, P) : lucas<false>(M, E, P);
   }
-  for (; b >= 1; b -= 2) {
-    x = kSmallN ? mont_mul_small(x, x, M) : mont_mul(x, x, M);
-    x = kSmallN ? mont_mul_small(x, x, M) : mont_mul(x, x, M);
-    const uint32_t g = (uint32_t)(d >> (b - 1)) & 3u;
-    const uint64_t t = g == 0u ? M.one : (g == 1u ? am : (g == 2u ? a2 : a3));
-    x = kSmallN ? mont_mul_small(x, t, M) : mont_mul(x, t, M);
-  }
-  bool ok = (x == M.one) | (x == M.mone);
-  for (int j = 0; j < r_w - 1; ++j) {
-    x = kSmallN ? mont_mul_small(x, x, M) : mont_mul(x, x, M);
-    ok |= (j < r - 1) & (x == M.mone);
-  }
-  return ok;
+  return ok && P != 0;
 }
 
-// Bases 3, 5, 7, ... of mr_finish_kernel for one warp: each lane stops after bases_needed(n)
-// bases or its first failure; the warp stops when no lane wants another base.
-template <bool kSmallN>
-__device__ __forceinline__ bool sprp_bases_3_on(const Mont& M, uint64_t d, int r, int top_w, int r_w, int need) {
-  const uint64_t n_ = M.n;
-  const uint64_t r1 = M.one, r2 = mod_add(r1, r1, n_), r4 = mod_add(r2, r2, n_), r6 = mod_add(r4, r2, n_);
-  uint64_t a = mod_add(r2, r1, n_);  // 3R: bases 3,5,7,11,13,17,19,23,29,31,37 by their gaps
-  bool prime = sprp_uniform_w2<kSmallN>(M, a, d, r, top_w, r_w);
-#pragma unroll 1
-  for (int s = 0; s < 10; ++s) {
-    // base index s + 2 (5, 7, 11, ...): still wanted by a lane that is prime so far and needs it
-    const bool want = prime && (s + 2 < need);
-    if (!__any_sync(0xFFFFFFFFu, want)) break;
-    const int step = (0x6264242422ull >> (4 * s)) & 0xF;  // 2,2,4,2,4,2,4,6,2,6
-    a = mod_add(a, step == 2 ? r2 : (step == 4 ? r4 : r6), n_);
-    const bool pass = sprp_uniform_w2<kSmallN>(M, a, d, r, top_w, r_w);
-    prime = want ? pass : prime;
-  }
-  return prime;
-}
+// Trial division for every candidate (a lane per candidate); the undecided wait in the warp's
+// shared-memory queues, one per size class for the base-2 test and one for the Lucas test of its
+// survivors, and each time a queue holds 32 they are tested together.  Lanes whose candidate is
+// decided early, and short exponents beside long ones, would otherwise leave most of the warp idle
+// (13 of 32 lanes active per instruction when each lane ran its own test).
+// Bound by the pipe of the products: 5e6 primes below 10^12 take 0.50 ms (two tests in double
+// precision; 3.6 ms with six Montgomery tests each), 4,000,001 random odd 64-bit numbers 0.34 ms
+// (0.77 ms with up to twelve bases and the survivors in a work list for a second kernel), 1000 of
+// them 24 us (123 us).  Eight blocks per SM, two waves, against 4 and 16: 0.34, 0.37 and
+// 0.35 ms (a second wave evens out what the warps of the first happen to find).
+constexpr int kMrBlock = 256;
+constexpr int kMrBlocksPerSm = 8;
+constexpr int kMrQueue = 64;  // at most 31 waiting + 32 arriving
 
-// Trial division for every candidate (a lane per candidate), then base 2 for the undecided ones:
-// those wait in the warp's shared-memory queues, one for n below 3,474,749,660,383 (exponents of
-// at most 42 bits, six bases needed) and one for the rest, and each time a queue holds 32 they are
-// tested together with warp-uniform loops (sprp_uniform), a lane each.  Lanes whose candidate
-// trial division decides, and short exponents beside long ones, would otherwise leave most of the
-// warp idle (13 of 32 lanes active per instruction when each lane ran its own test).  Base-2
-// survivors go to the work list: the small ones from the front, the others from the back, so that
-// the warps of mr_finish_kernel mostly share one base count.
-constexpr int kSieveBlock = 256;
-constexpr int kMrQueue = 64;  // per warp and size class: at most 31 waiting + 32 arriving
-
-__device__ __forceinline__ void mr_base2_drain(const uint64_t* __restrict__ cand, uint8_t* __restrict__ out,
-                                               uint32_t* __restrict__ work, uint32_t* __restrict__ nwork,
-                                               uint64_t count, uint32_t* q, uint32_t& nq, bool small_class,
-                                               uint32_t lane) {
+// Take up to 32 entries from the queue's front; lanes beyond `take` repeat lane 0's.
+__device__ __forceinline__ uint32_t queue_take(uint32_t* q, uint32_t& nq, uint32_t lane, bool& live) {
   __syncwarp();
   const uint32_t take = nq < 32u ? nq : 32u;
-  const bool live = lane < take;
-  uint32_t i = live ? q[lane] : 0u;
+  live = lane < take;
+  const uint32_t i = q[live ? lane : 0u];
   __syncwarp();
   if (lane + 32u < nq) q[lane] = q[lane + 32u];
   nq -= take;
   __syncwarp();
-  const uint32_t i0 = __shfl_sync(0xFFFFFFFFu, i, 0);  // idle lanes shadow lane 0
-  if (!live) i = i0;
-  const uint64_t n = cand[i];
-  const Mont M = mont_setup(n);
-  uint64_t d = n - 1;
-  const int r = __ffsll((long long)d) - 1;
-  d >>= r;
-  const int top_w = __reduce_max_sync(0xFFFFFFFFu, (unsigned)(63 - __clzll(d)));
-  const int r_w = __reduce_max_sync(0xFFFFFFFFu, (unsigned)r);
-  const bool ok = __all_sync(0xFFFFFFFFu, n < (1ull << 63)) ? sprp_uniform<true>(M, 0, d, r, top_w, r_w, true)
-                                                           : sprp_uniform<false>(M, 0, d, r, top_w, r_w, true);
-  if (live && !ok) out[i] = 0;
-  const bool keep = live && ok;
-  const unsigned mk = __ballot_sync(0xFFFFFFFFu, keep);
-  if (mk) {
-    uint32_t at = 0;
-    if (lane == 0) at = atomicAdd(nwork + (small_class ? 0 : 1), (uint32_t)__popc(mk));
-    at = __shfl_sync(0xFFFFFFFFu, at, 0) + (uint32_t)__popc(mk & ((1u << lane) - 1u));
-    if (keep) {
-      if (small_class) work[at] = i;
-      else work[count - 1 - at] = i;
-    }
-  }
+  return i;
 }
 
-__global__ void __launch_bounds__(kSieveBlock) mr_sieve_kernel(const uint64_t* __restrict__ cand, uint64_t count,
-                                                              uint8_t* __restrict__ out, uint32_t* __restrict__ work,
-                                                              uint32_t* __restrict__ nwork) {
-  __shared__ uint32_t s_q[kSieveBlock / 32][2][kMrQueue];
+__device__ __forceinline__ void queue_add(uint32_t* q, uint32_t& nq, uint32_t lane, uint32_t i, bool add) {
+  const unsigned m = __ballot_sync(0xFFFFFFFFu, add);
+  if (add) q[nq + __popc(m & ((1u << lane) - 1u))] = i;
+  nq += __popc(m);
+}
+
+struct MrQueues {  // of one size class
+  uint32_t *base2, *lucas;
+  uint32_t n_base2, n_lucas;
+};
+
+template <bool kDouble>
+__device__ __forceinline__ void drain_lucas(const uint64_t* __restrict__ cand, uint8_t* __restrict__ out, MrQueues& Q,
+                                            uint32_t lane) {
+  bool live;
+  const uint32_t i = queue_take(Q.lucas, Q.n_lucas, lane, live);
+  const bool ok = test_lucas<kDouble>(cand[i]);
+  if (live) out[i] = ok ? 1 : 0;
+}
+
+template <bool kDouble>
+__device__ __forceinline__ void drain_base2(const uint64_t* __restrict__ cand, uint8_t* __restrict__ out, MrQueues& Q,
+                                            uint32_t lane) {
+  bool live;
+  const uint32_t i = queue_take(Q.base2, Q.n_base2, lane, live);
+  const bool ok = test_base2<kDouble>(cand[i]);
+  if (live && !ok) out[i] = 0;
+  queue_add(Q.lucas, Q.n_lucas, lane, i, live && ok);
+  if (Q.n_lucas >= 32u) drain_lucas<kDouble>(cand, out, Q, lane);
+}
+
+__global__ void __launch_bounds__(kMrBlock) mr_kernel(const uint64_t* __restrict__ cand, uint64_t count,
+                                                      uint8_t* __restrict__ out) {
+  __shared__ uint32_t s_q[kMrBlock / 32][4][kMrQueue];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t* qs = s_q[warp][0];
-  uint32_t* ql = s_q[warp][1];
-  uint32_t ns = 0, nl = 0;  // warp-uniform queue lengths
-  const unsigned below = (1u << lane) - 1u;
+  MrQueues qd = {s_q[warp][0], s_q[warp][1], 0, 0}, qm = {s_q[warp][2], s_q[warp][3], 0, 0};
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + 32u * warp; base < count; base += stride) {
     const uint64_t i = base + lane;
-    bool und = false, small = false;
+    bool open = false, dbl = false;
     if (i < count) {
       const uint64_t n = cand[i];
       const int t = trial_phase(n);
       if (t >= 0) out[i] = (uint8_t)t;
       else {
-        und = true;
-        small = n < kSmallMr;
+        open = true;
+        dbl = n < kDModEnd;
       }
     }
-    const unsigned ms = __ballot_sync(0xFFFFFFFFu, und && small);
-    const unsigned ml = __ballot_sync(0xFFFFFFFFu, und && !small);
-    if (und && small) qs[ns + __popc(ms & below)] = (uint32_t)i;
-    if (und && !small) ql[nl + __popc(ml & below)] = (uint32_t)i;
-    ns += __popc(ms);
-    nl += __popc(ml);
-    if (ns >= 32u) mr_base2_drain(cand, out, work, nwork, count, qs, ns, true, lane);
-    if (nl >= 32u) mr_base2_drain(cand, out, work, nwork, count, ql, nl, false, lane);
+    queue_add(qd.base2, qd.n_base2, lane, (uint32_t)i, open && dbl);
+    queue_add(qm.base2, qm.n_base2, lane, (uint32_t)i, open && !dbl);
+    if (qd.n_base2 >= 32u) drain_base2<true>(cand, out, qd, lane);
+    if (qm.n_base2 >= 32u) drain_base2<false>(cand, out, qm, lane);
   }
-  if (ns) mr_base2_drain(cand, out, work, nwork, count, qs, ns, true, lane);
-  if (nl) mr_base2_drain(cand, out, work, nwork, count, ql, nl, false, lane);
-}
-
-// `work` holds candidate indices (< 2^32: the entry points take fewer than 2^32 candidates per call):
-// nwork[0] of them at the front, nwork[1] at the back (work[count - 1], work[count - 2], ...).
-__global__ void mr_finish_kernel(const uint64_t* __restrict__ cand, uint8_t* __restrict__ out,
-                                 const uint32_t* __restrict__ work, const uint32_t* __restrict__ nwork,
-                                 uint32_t count) {
-  const uint32_t na = nwork[0];
-  const uint32_t nw = na + nwork[1];
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t base = warp0 * 32u; base < nw; base += nwarps * 32u) {  // warp-uniform loop
-    const uint32_t k = base + lane;
-    const bool live = k < nw;
-    const uint32_t i = live ? work[k < na ? k : count - 1 - (k - na)] : 0u;
-    uint64_t n = live ? cand[i] : 0ull;
-    const uint64_t n0 = __shfl_sync(0xFFFFFFFFu, n, 0);  // idle lanes shadow lane 0
-    if (!live) n = n0;
-    const Mont M = mont_setup(n);
-    uint64_t d = n - 1;
-    const int r = __ffsll((long long)d) - 1;
-    d >>= r;
-    const int top = 63 - __clzll(d);
-    const int top_w = __reduce_max_sync(0xFFFFFFFFu, (unsigned)top);
-    const int r_w = __reduce_max_sync(0xFFFFFFFFu, (unsigned)r);
-    const int need = bases_needed(n);  // >= 6: bases 2 (done) and 3 always run
-    const bool prime = __all_sync(0xFFFFFFFFu, n < (1ull << 63))
-                           ? sprp_bases_3_on<true>(M, d, r, top_w, r_w, need)
-                           : sprp_bases_3_on<false>(M, d, r, top_w, r_w, need);
-    if (live) out[i] = prime ? 1 : 0;
-  }
+  // What is left in the queues (up to 31 each) is put together over the block, so that the last
+  // tests run on full warps: at 4,000,001 candidates a warp sees 422 and leaves half a warp of
+  // candidates for each test.
+  __shared__ uint32_t s_rest[4][kMrBlock / 32 * 32];
+  __shared__ uint32_t s_n[4];
+  if (threadIdx.x < 4) s_n[threadIdx.x] = 0;
+  __syncthreads();
+  auto put = [&](int k, const uint32_t* q, uint32_t nq) {
+    uint32_t at = 0;
+    if (lane == 0 && nq) at = atomicAdd(&s_n[k], nq);
+    at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    if (lane < nq) s_rest[k][at + lane] = q[lane];
+  };
+  put(0, qd.base2, qd.n_base2);
+  put(1, qm.base2, qm.n_base2);
+  qd.n_base2 = qm.n_base2 = 0;
+  __syncthreads();
+  // base 2: the block's warps take 32 at a time; survivors go to the warp's Lucas queue (31 + 32 fit)
+  auto take = [&](int k, uint32_t c, uint32_t* q, uint32_t& nq) {
+    const uint32_t n = s_n[k], first = 32u * c;
+    if (first >= n) return false;
+    nq = min(32u, n - first);
+    if (lane < nq) q[lane] = s_rest[k][first + lane];
+    return true;
+  };
+  constexpr uint32_t kWarps = kMrBlock / 32;
+  for (uint32_t c = warp; take(0, c, qd.base2, qd.n_base2); c += kWarps) drain_base2<true>(cand, out, qd, lane);
+  for (uint32_t c = warp; take(1, c, qm.base2, qm.n_base2); c += kWarps) drain_base2<false>(cand, out, qm, lane);
+  put(2, qd.lucas, qd.n_lucas);
+  put(3, qm.lucas, qm.n_lucas);
+  __syncthreads();
+  for (uint32_t c = warp; take(2, c, qd.lucas, qd.n_lucas); c += kWarps) drain_lucas<true>(cand, out, qd, lane);
+  for (uint32_t c = kWarps - 1 - warp; take(3, c, qm.lucas, qm.n_lucas); c += kWarps)
+    drain_lucas<false>(cand, out, qm, lane);
 }
 
 // Gap proofs: one warp per gap.  Interior integers are split over the lanes; an interior odd
@@ -398,7 +467,7 @@ constexpr uint32_t kProveChunk = 256;  // interior odd integers examined per rou
 // kProveChunk odd interior integers: trial division by the bases 3..37 on all lanes, the
 // undecided integers above isqrt(p_after) are appended to a per-warp list in shared memory, and
 // the list is tested 32 at a time by a warp-uniform base-2 strong probable-prime test; only
-// integers passing it (primes, or base-2 strong pseudoprimes) take the remaining bases.
+// integers passing it (primes, or base-2 strong pseudoprimes) take the Lucas test.
 __global__ void __launch_bounds__(kProveBlock) prove_interior_kernel(const uint64_t* __restrict__ p_after,
                                                                      const int32_t* __restrict__ gap, uint64_t count,
                                                                      const uint8_t* __restrict__ end_ok,
@@ -441,19 +510,10 @@ __global__ void __launch_bounds__(kProveBlock) prove_interior_kernel(const uint6
           for (uint32_t b0 = 0; b0 < n_list && !bad; b0 += 32) {
             const bool live = b0 + lane < n_list;
             const uint64_t v = list[live ? b0 + lane : b0];  // idle lanes shadow the first entry
-            const Mont M = mont_setup(v);
-            uint64_t d = v - 1;
-            const int r = __ffsll((long long)d) - 1;
-            d >>= r;
-            const int top = 63 - __clzll(d);
-            const int top_w = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)top);
-            const int r_w = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)r);
-            const bool small = __all_sync(0xFFFFFFFFu, v < (1ull << 63));
-            const bool prp = small ? sprp_uniform<true>(M, 0, d, r, top_w, r_w, true)
-                                   : sprp_uniform<false>(M, 0, d, r, top_w, r_w, true);
-            const bool pass = live && prp;
-            if (__any_sync(0xFFFFFFFFu, pass)) {
-              const bool prime = pass && sprp_rest(M, d, r);
+            const bool dbl = __all_sync(0xFFFFFFFFu, v < kDModEnd);
+            const bool prp = dbl ? test_base2<true>(v) : test_base2<false>(v);
+            if (__any_sync(0xFFFFFFFFu, prp)) {  // idle lanes have a live lane's verdict
+              const bool prime = (dbl ? test_lucas<true>(v) : test_lucas<false>(v)) && prp;
               bad = __any_sync(0xFFFFFFFFu, prime);
             }
           }
@@ -489,33 +549,29 @@ static int ensure_mr_tables() {
   return 0;
 }
 
-int launch_mr(const uint64_t* d_n, uint64_t count, uint8_t* d_out, uint32_t* d_work,
-              uint32_t* d_nwork, void* stream, int sm_count) {
+int launch_mr(const uint64_t* d_n, uint64_t count, uint8_t* d_out, void* stream, int sm_count) {
   if (ensure_mr_tables()) return -1;
   if (count == 0) return 0;
   if (count > 0xFFFFFFFFull) return -1;
   cudaStream_t s = (cudaStream_t)stream;
-  if (cudaMemsetAsync(d_nwork, 0, 2 * sizeof(uint32_t), s) != cudaSuccess) return -1;
-  const int blk = 256;
-  uint64_t want = (count + blk - 1) / blk;
-  int grid = (int)(want < (uint64_t)sm_count * 16 ? want : (uint64_t)sm_count * 16);
-  mr_sieve_kernel<<<grid, kSieveBlock, 0, s>>>(d_n, count, d_out, d_work, d_nwork);
-  mr_finish_kernel<<<sm_count * 8, blk, 0, s>>>(d_n, d_out, d_work, d_nwork, (uint32_t)count);
+  const uint64_t want = (count + kMrBlock - 1) / kMrBlock;
+  const uint64_t most = (uint64_t)sm_count * kMrBlocksPerSm;
+  const int grid = (int)(want < most ? want : most);
+  mr_kernel<<<grid, kMrBlock, 0, s>>>(d_n, count, d_out);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 int launch_prove_gaps(const uint64_t* d_p_after, const int32_t* d_gap, uint64_t count, uint8_t* d_ok,
-                      uint64_t* d_ends, uint8_t* d_ends_ok, uint32_t* d_work, uint32_t* d_nwork, void* stream,
-                      int sm_count) {
+                      uint64_t* d_ends, uint8_t* d_ends_ok, void* stream, int sm_count) {
   if (ensure_mr_tables()) return -1;
   if (count == 0) return 0;
   if (count > 0x7FFFFFFFull) return -1;
   cudaStream_t s = (cudaStream_t)stream;
-  // 1. both endpoints of every gap through the batched Miller-Rabin kernels
+  // 1. both endpoints of every gap through the Miller-Rabin kernel
   const uint64_t eg = (count + 255) / 256;
   gap_ends_kernel<<<(int)(eg < (uint64_t)sm_count * 8 ? eg : (uint64_t)sm_count * 8), 256, 0, s>>>(d_p_after, d_gap,
                                                                                                    count, d_ends);
-  if (launch_mr(d_ends, 2 * count, d_ends_ok, d_work, d_nwork, stream, sm_count)) return -1;
+  if (launch_mr(d_ends, 2 * count, d_ends_ok, stream, sm_count)) return -1;
   // 2. interiors
   const uint64_t want = (count + (kProveBlock / 32) - 1) / (kProveBlock / 32);
   const int grid = (int)(want < (uint64_t)sm_count * 8 ? want : (uint64_t)sm_count * 8);
@@ -599,21 +655,15 @@ int probe_mulmod(int sm_count, void* stream, double* full_per_s, double* small_p
 // already reserved by another allocator (a framework's caching allocator or a memory pool),
 // where cudaMalloc would fail or fragment that pool, and request paths of long-running
 // services, where cudaMalloc/cudaFree would synchronize the device and stall other streams.
-// The regular entry points allocate (the context at creation, per-call buffers on growth);
-// this one needs no context and allocates nothing: its scratch (the survivor work list and
-// its counter) is the fixed array below, which every device that loads libvoss.so holds
-// until the process exits.
+// The regular entry points allocate (the context at creation, per-call buffers on growth); this
+// one needs no context and no device memory of its own.
 // =====================================================================================
 namespace voss {
 
-constexpr uint64_t kNoAllocMaxCount = 1ull << 22;  // candidates per call (16 MiB of scratch)
-constexpr uint32_t kNoAllocListOffset = 64;         // counters at [0], [1]; list starts 256 B in
-
-static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocMaxCount + kNoAllocListOffset];
+constexpr uint64_t kNoAllocMaxCount = 1ull << 22;  // candidates per call
 
 static std::mutex g_noalloc_mu;
-static uint32_t* g_noalloc_ptr[64];  // device address of g_noalloc_scratch, per device ordinal
-static int g_noalloc_sms[64];
+static int g_noalloc_sms[64];  // SM count per device ordinal
 
 }  // namespace voss
 
@@ -635,31 +685,18 @@ extern "C" VOSS_API int voss_mr_verify_noalloc(const uint64_t* d_n, uint64_t cou
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
     return voss_detail::set_error(VOSS_ERR_NODEV, "no current CUDA device");
-  uint32_t* scratch = nullptr;
   int sms = 0;
   {
-    // set-up, once per device, on the calling thread's current device: the host-side name of
-    // the array is not a device address, so the kernel gets the address the runtime reports
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
-    if (!g_noalloc_ptr[dev]) {
-      void* p = nullptr;
-      const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-      if (e != cudaSuccess || !p) {
-        snprintf(msg, sizeof(msg), "cudaGetSymbolAddress(no-allocation scratch) failed: %s", cudaGetErrorString(e));
-        return voss_detail::set_error(VOSS_ERR_CUDA, msg);
-      }
+    if (!g_noalloc_sms[dev]) {
       int n = 0;
       if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
         return voss_detail::set_error(VOSS_ERR_CUDA, "cannot read the SM count");
-      g_noalloc_ptr[dev] = static_cast<uint32_t*>(p);
       g_noalloc_sms[dev] = n;
     }
-    scratch = g_noalloc_ptr[dev];
     sms = g_noalloc_sms[dev];
   }
-  // launch_mr clears the two list counters (cudaMemsetAsync on `scratch`) before its kernels;
-  // the list needs no clearing since entries are written before they are read.
-  if (launch_mr(d_n, count, d_is_prime, scratch + kNoAllocListOffset, scratch, stream, sms) != 0) {
+  if (launch_mr(d_n, count, d_is_prime, stream, sms) != 0) {
     snprintf(msg, sizeof(msg), "Miller-Rabin launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     return voss_detail::set_error(VOSS_ERR_CUDA, msg);
   }

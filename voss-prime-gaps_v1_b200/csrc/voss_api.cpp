@@ -526,12 +526,22 @@ void route_intervals(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, 
     bool mr = false;
     if (route != 0xFFFFFFFFull && a < hi[i]) {
       const uint64_t sq = isqrt_u64(hi[i] - 1);
-      const size_t np = (size_t)(std::upper_bound(c->primes.begin(), c->primes.end(),
-                                                  (uint32_t)std::min<uint64_t>(sq, 0xFFFFFFFFull)) -
-                                 c->primes.begin());
-      const uint64_t pairs = np;
       const uint64_t len = hi[i] - a;
-      mr = len < (1ull << 31) && pairs / route > len && R->n_cand + len <= cand_cap;
+      if (len < (1ull << 31) && R->n_cand + len <= cand_cap) {
+        // x / ln x < pi(x) < 1.2551 x / ln x (x >= 17; Rosser and Schoenfeld 1962) nearly always decide;
+        // a search of the table (50 million primes at 10^18) misses the host's caches a dozen times
+        const double x = (double)std::min<uint64_t>(sq, c->primes.empty() ? 0 : c->primes.back());
+        const double pi_lo = x >= 17.0 ? x / std::log(x) : 0.0;
+        if (x < 1e6 || (pi_lo - 12.0 < (double)route * (double)(len + 1) &&
+                        1.2551 * pi_lo >= (double)route * (double)len)) {
+          const uint64_t np = (uint64_t)(std::upper_bound(c->primes.begin(), c->primes.end(),
+                                                          (uint32_t)std::min<uint64_t>(sq, 0xFFFFFFFFull)) -
+                                         c->primes.begin());
+          mr = np / route > len;
+        } else {
+          mr = pi_lo - 12.0 >= (double)route * (double)(len + 1);
+        }
+      }
     }
     if (mr) {
       ShortInterval I;
@@ -540,8 +550,9 @@ void route_intervals(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, 
       I.j0 = (uint32_t)kCoprime30Below[a % 30];
       I.n_cand = (uint32_t)(wheel_count_below(hi[i]) - wheel_count_below(a));
       I.out_index = i;
-      I.pad = 0;
+      I.seg_begin = R->n_seg;
       R->n_cand += I.n_cand;
+      R->n_seg += short_segments(I.n_cand);
       R->sv.push_back(I);
     } else {
       R->lo.push_back(lo[i]);
@@ -580,15 +591,14 @@ int launch_routed(voss_ctx* c, Workspace& W, const LaunchEvents& E, const Interv
     NvtxRange r("short intervals by Miller-Rabin");
     const uint64_t nc = R.n_cand;
     if ((rc = W.sh_iv.ensure(sizeof(ShortInterval) * R.sv.size())) || (rc = W.mr_in.ensure(8 * std::max<uint64_t>(nc, 1))) ||
-        (rc = W.mr_out.ensure(std::max<uint64_t>(nc, 1))) || (rc = W.mr_work.ensure(sizeof(uint32_t) * (nc + 8))))
+        (rc = W.mr_out.ensure(std::max<uint64_t>(nc, 1))) || (rc = W.sh_seg.ensure(sizeof(ShortSegment) * R.n_seg)))
       return rc;
     CUDA_TRY(cudaMemcpyAsync(W.sh_iv.p, R.sv.data(), sizeof(ShortInterval) * R.sv.size(), cudaMemcpyHostToDevice, s));
-    uint32_t* work = W.mr_work.as<uint32_t>();
-    if (launch_short_intervals(W.sh_iv.as<ShortInterval>(), (uint32_t)R.sv.size(), nc, W.mr_in.as<uint64_t>(),
-                               W.mr_out.as<uint8_t>(), work + 8, work, W.istats.as<voss_interval_stats>(), c->sm_count,
-                               s))
+    if (launch_short_intervals(W.sh_iv.as<ShortInterval>(), (uint32_t)R.sv.size(), R.n_seg, nc,
+                               W.mr_in.as<uint64_t>(), W.mr_out.as<uint8_t>(), W.sh_seg.as<ShortSegment>(),
+                               W.istats.as<voss_interval_stats>(), c->sm_count, s))
       return fail(VOSS_ERR_CUDA, "short-interval launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-    k += nc ? 4 : 1;
+    k += nc ? 4 : 3;
   }
   if (E.ev2) CUDA_TRY(cudaEventRecord(E.ev2, s));  // finalize and the Miller-Rabin path count in the launch's time
   if (kernels) *kernels = k;
@@ -1167,10 +1177,7 @@ VOSS_API int voss_mr_verify_device(voss_ctx* c, const uint64_t* d_n, uint64_t co
   if (count > 0xFFFFFFFFull) return fail(VOSS_ERR_ARG, "count must be < 2^32 per call");
   cudaSetDevice(c->device);
   cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
-  int rc;
-  if ((rc = c->ws.mr_work.ensure(sizeof(uint32_t) * (std::max<uint64_t>(count, 1) + 8)))) return rc;
-  uint32_t* work = c->ws.mr_work.as<uint32_t>();
-  if (launch_mr(d_n, count, d_out, work + 8, work, s, c->sm_count))
+  if (launch_mr(d_n, count, d_out, s, c->sm_count))
     return fail(VOSS_ERR_CUDA, "Miller-Rabin launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   return VOSS_OK;
 }
@@ -1193,13 +1200,9 @@ VOSS_API int voss_mr_verify(voss_ctx* c, const uint64_t* n, uint64_t count, uint
   const bool staged = count >= (1ull << 20);
   if (staged && (rc = ensure_stage(c, std::min<uint64_t>(count, 1ull << 24)))) return rc;
   const uint64_t kChunk = staged ? c->h_stage_cap : (1ull << 24);  // candidates per launch
-  const uint64_t per = std::min(count, kChunk);
-  if ((rc = W.mr_in.ensure(count * 8)) || (rc = W.mr_out.ensure(count)) ||
-      (rc = W.mr_work.ensure(sizeof(uint32_t) * (per + 8))))
-    return rc;
+  if ((rc = W.mr_in.ensure(count * 8)) || (rc = W.mr_out.ensure(count))) return rc;
   uint64_t* d_in = W.mr_in.as<uint64_t>();
   uint8_t* d_out = W.mr_out.as<uint8_t>();
-  uint32_t* work = W.mr_work.as<uint32_t>();
   uint64_t i = 0;
   for (uint64_t off = 0; off < count; off += kChunk, ++i) {
     const uint64_t k = std::min(kChunk, count - off);
@@ -1214,7 +1217,7 @@ VOSS_API int voss_mr_verify(voss_ctx* c, const uint64_t* n, uint64_t count, uint
     }
     CUDA_TRY(cudaEventRecord(c->ev_copy, c->copy_stream));
     CUDA_TRY(cudaStreamWaitEvent(s, c->ev_copy, 0));
-    if (launch_mr(d_in + off, k, d_out + off, work + 8, work, s, c->sm_count))
+    if (launch_mr(d_in + off, k, d_out + off, s, c->sm_count))
       return fail(VOSS_ERR_CUDA, "Miller-Rabin launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   }
   if (!staged) {
@@ -1241,8 +1244,7 @@ VOSS_API int voss_prove_gaps(voss_ctx* c, const uint64_t* p_after, const int32_t
   Workspace& W = c->ws;  // context-owned, grow-only buffers: repeated calls do not allocate
   int rc;
   if ((rc = W.pg_pa.ensure(count * 8)) || (rc = W.pg_gap.ensure(count * 4)) || (rc = W.pg_ok.ensure(count)) ||
-      (rc = W.mr_in.ensure(2 * count * 8)) || (rc = W.mr_out.ensure(2 * count)) ||
-      (rc = W.mr_work.ensure(sizeof(uint32_t) * (2 * count + 8))))
+      (rc = W.mr_in.ensure(2 * count * 8)) || (rc = W.mr_out.ensure(2 * count)))
     return rc;
   // large batches cross through the pinned staging buffers (filled and emptied by host threads)
   const bool staged = count >= (1ull << 20);
@@ -1254,9 +1256,8 @@ VOSS_API int voss_prove_gaps(voss_ctx* c, const uint64_t* p_after, const int32_t
     CUDA_TRY(cudaMemcpyAsync(W.pg_pa.p, p_after, count * 8, cudaMemcpyHostToDevice, s));
     CUDA_TRY(cudaMemcpyAsync(W.pg_gap.p, gap, count * 4, cudaMemcpyHostToDevice, s));
   }
-  uint32_t* work = W.mr_work.as<uint32_t>();
   if (launch_prove_gaps(W.pg_pa.as<uint64_t>(), W.pg_gap.as<int32_t>(), count, W.pg_ok.as<uint8_t>(),
-                        W.mr_in.as<uint64_t>(), W.mr_out.as<uint8_t>(), work + 8, work, s, c->sm_count))
+                        W.mr_in.as<uint64_t>(), W.mr_out.as<uint8_t>(), s, c->sm_count))
     return fail(VOSS_ERR_CUDA, "gap proof launch failed");
   if (staged) {
     if ((rc = stage_out(c, ok, W.pg_ok.p, count, s))) return rc;

@@ -63,13 +63,13 @@ struct DevBuf {
 
 // Device memory of one launch of the tile kernel (and of Miller-Rabin batches).
 struct Workspace {
-  DevBuf iv, partials, acc, out, large, large_iv, over, counters, istats, offsets, emit, mr_work, mr_in, mr_out;
+  DevBuf iv, partials, acc, out, large, large_iv, over, counters, istats, offsets, emit, mr_in, mr_out;
   DevBuf gbm, scat;  // large-prime pre-pass: bitmap of the launch and its interval descriptors
   DevBuf tile_iv;    // interval of each tile, for launches of more than one interval
-  DevBuf pg_pa, pg_gap, pg_ok;  // gap proofs: inputs and verdicts (endpoints use mr_in / mr_out / mr_work)
+  DevBuf pg_pa, pg_gap, pg_ok;  // gap proofs: inputs and verdicts (endpoints use mr_in / mr_out)
   DevBuf sha_data, sha_off, sha_out;  // certificate hashing: messages, offsets, digests
   DevBuf ls_keys, ls_idx, ls_temp, ls_sorted;  // large-gap list sorted by position (large_sort.cu)
-  DevBuf sh_iv, sh_map;  // short intervals by Miller-Rabin (short_iv.cu); sieved intervals' result slots
+  DevBuf sh_iv, sh_map, sh_seg;  // short intervals by Miller-Rabin (short_iv.cu); sieved intervals' result slots
   // Largest large-prime bitmap this workspace may use; with gbm_fixed the buffers are never
   // grown (server slots size them at creation), and launches that need more skip the pre-pass.
   size_t gbm_budget = 8ull << 30;
@@ -89,7 +89,7 @@ struct RunPlan {
   uint64_t n_words = 0;
 };
 
-enum { kCtrTile = 0, kCtrLarge = 1, kCtrOver = 2, kCtrError = 3, kCtrMrWork = 4, kCtrWords = 8 };
+enum { kCtrTile = 0, kCtrLarge = 1, kCtrOver = 2, kCtrError = 3, kCtrWords = 8 };
 
 constexpr uint64_t kMaxHi = 1ull << 62;
 constexpr uint32_t kOverCap = 1u << 16;
@@ -161,6 +161,7 @@ struct IntervalRoute {
   std::vector<uint32_t> map;
   std::vector<voss::ShortInterval> sv;
   uint64_t n_cand = 0;
+  uint32_t n_seg = 0;  // segments of the Miller-Rabin intervals
 };
 // Split [lo_i, hi_i) by the context's mr_route, with at most cand_cap Miller-Rabin candidates.
 void route_intervals(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, uint32_t n, uint64_t cand_cap,

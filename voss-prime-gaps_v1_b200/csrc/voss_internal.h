@@ -104,7 +104,20 @@ struct ShortInterval {
   uint32_t j0;         // wheel integers of [base, a)
   uint32_t n_cand;     // wheel integers of [a, hi)
   uint32_t out_index;  // position in the caller's result array
-  uint32_t pad;
+  uint32_t seg_begin;  // its first segment among the launch's
+};
+
+// Candidates per segment of a short interval, and the segments of one with n candidates.
+constexpr uint32_t kShortSeg = 4096;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr uint32_t short_segments(uint32_t n_cand) { return n_cand ? (n_cand - 1) / kShortSeg + 1 : 1; }
+
+struct ShortSegment {
+  uint64_t first, last;  // ~0 / 0 when it holds no prime
+  uint64_t max_gap_lo;
+  uint32_t max_gap, count, over, pad;
 };
 
 struct TilePartial {
@@ -195,9 +208,9 @@ namespace voss {
 int launch_interval_finalize(const SieveArgs& a, const IntervalOut* io, voss_interval_stats* out,
                              const uint32_t* out_index, void* stream);
 // Short intervals by Miller-Rabin (short_iv.cu): candidates into d_cand (n_cand), verdicts into
-// d_ok, the work list and its counters in d_work / d_nwork, results at d_out[out_index].
-int launch_short_intervals(const ShortInterval* d_iv, uint32_t n_iv, uint64_t n_cand, uint64_t* d_cand,
-                           uint8_t* d_ok, uint32_t* d_work, uint32_t* d_nwork, voss_interval_stats* d_out,
+// d_ok, results at d_out[out_index].
+int launch_short_intervals(const ShortInterval* d_iv, uint32_t n_iv, uint32_t n_seg, uint64_t n_cand,
+                           uint64_t* d_cand, uint8_t* d_ok, ShortSegment* d_seg, voss_interval_stats* d_out,
                            int sm_count, void* stream);
 int launch_scatter_large(const uint32_t* primes, const uint64_t* magic, uint32_t j0, uint32_t j1,
                          const IntervalScatter* iv, uint32_t n_iv, uint32_t* gbm, int sm_count, void* stream);
@@ -209,14 +222,12 @@ int launch_large_sort(const LargeGapDev* in, uint32_t n, int end_bit, unsigned l
 void build_presieve_tables(uint32_t* out /* kPreWords */);
 int probe_smem_rmw(int sm_count, void* stream, float* ms, double* bytes);
 
-// Miller-Rabin (mr_kernels.cu).  d_work holds count entries, d_nwork two counters (cleared here).
-int launch_mr(const uint64_t* d_n, uint64_t count, uint8_t* d_out, uint32_t* d_work,
-              uint32_t* d_nwork, void* stream, int sm_count);
+// Exact primality of d_n[0..count) (mr_kernels.cu), count < 2^32.
+int launch_mr(const uint64_t* d_n, uint64_t count, uint8_t* d_out, void* stream, int sm_count);
 // Gap proofs: endpoints (into d_ends / d_ends_ok, 2 * count each) through the Miller-Rabin
-// kernels (work list d_work, counter d_nwork), then the interiors; count < 2^31.
+// kernel, then the interiors; count < 2^31.
 int launch_prove_gaps(const uint64_t* d_p_after, const int32_t* d_gap, uint64_t count, uint8_t* d_ok,
-                      uint64_t* d_ends, uint8_t* d_ends_ok, uint32_t* d_work, uint32_t* d_nwork, void* stream,
-                      int sm_count);
+                      uint64_t* d_ends, uint8_t* d_ends_ok, void* stream, int sm_count);
 // Montgomery products per second of independent squaring chains (moduli above / below 2^63).
 int probe_mulmod(int sm_count, void* stream, double* full_per_s, double* small_per_s);
 

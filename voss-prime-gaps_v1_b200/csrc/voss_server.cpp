@@ -161,12 +161,10 @@ int launch_batch(voss_server* S, Slot& sl) {
   parallel_gather(sl.h_mr_in, segs.data(), segs.size(), kCopyPart);
   if (sl.n_mr) {
     CUDA_TRY(cudaMemcpyAsync(sl.ws.mr_in.p, sl.h_mr_in, sl.n_mr * 8, cudaMemcpyHostToDevice, s));
-    uint32_t* work = sl.ws.mr_work.as<uint32_t>();
-    if (voss::launch_mr(sl.ws.mr_in.as<uint64_t>(), sl.n_mr, sl.ws.mr_out.as<uint8_t>(), work + 8, work, s,
-                        c->sm_count))
+    if (voss::launch_mr(sl.ws.mr_in.as<uint64_t>(), sl.n_mr, sl.ws.mr_out.as<uint8_t>(), s, c->sm_count))
       return fail(VOSS_ERR_CUDA, "Miller-Rabin launch failed");
     CUDA_TRY(cudaMemcpyAsync(sl.h_mr_out, sl.ws.mr_out.p, sl.n_mr, cudaMemcpyDeviceToHost, s));
-    S->launches += 2;
+    S->launches += 1;
   }
   CUDA_TRY(cudaEventRecord(sl.done, s));
   return VOSS_OK;
@@ -309,15 +307,15 @@ Slot* make_slot(voss_server* S, int* rc) {
       (e = W.out.ensure(sizeof(IntervalOut) * nreq)) || (e = W.counters.ensure(sizeof(uint32_t) * kCtrWords)) ||
       (e = W.over.ensure(sizeof(voss::OverflowGap) * kOverCap)) || (e = W.large.ensure(sizeof(voss::LargeGapDev))) ||
       (e = W.large_iv.ensure(sizeof(uint32_t))) || (e = W.istats.ensure(sizeof(voss_interval_stats) * nreq)) ||
-      (e = W.mr_in.ensure(8 * (C.max_batch_candidates + 1))) || (e = W.mr_out.ensure(C.max_batch_candidates + 1)) ||
-      (e = W.mr_work.ensure(4 * (C.max_batch_candidates + 8))))
+      (e = W.mr_in.ensure(8 * (C.max_batch_candidates + 1))) || (e = W.mr_out.ensure(C.max_batch_candidates + 1)))
     return bad(e);
   // the large-prime pre-pass bitmap: fixed size, never grown while serving
   W.gbm_budget = C.max_batch_bitmap_bytes;
   W.gbm_fixed = true;
   if (W.gbm_budget && ((e = W.gbm.ensure(W.gbm_budget)) || (e = W.scat.ensure(sizeof(voss::IntervalScatter) * nreq))))
     return bad(e);
-  if ((e = W.sh_iv.ensure(sizeof(voss::ShortInterval) * nreq)) || (e = W.sh_map.ensure(sizeof(uint32_t) * nreq)))
+  if ((e = W.sh_iv.ensure(sizeof(voss::ShortInterval) * nreq)) || (e = W.sh_map.ensure(sizeof(uint32_t) * nreq)) ||
+      (e = W.sh_seg.ensure(sizeof(voss::ShortSegment) * (C.max_batch_candidates / voss::kShortSeg + nreq + 1))))
     return bad(e);
   if (cudaMallocHost(&sl->h_istats, sizeof(voss_interval_stats) * nreq) != cudaSuccess ||
       cudaMallocHost(&sl->h_mr_in, 8 * (C.max_batch_candidates + 1)) != cudaSuccess ||
