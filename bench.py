@@ -207,7 +207,7 @@ def primes_upto(s: int):
     return p[p >= 7].astype(np.float64)
 
 
-def interval_work(lo, hi, p_large: int, mr_route: int = 50) -> dict:
+def interval_work(lo, hi, p_large: int, mr_route: int = 25) -> dict:
     """Algorithmic work terms of a batch of intervals [lo_i, hi_i).
 
     offsets: one first-hit computation per (interval, base prime 7 <= p <= isqrt(hi_i - 1)).

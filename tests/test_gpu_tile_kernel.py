@@ -53,3 +53,13 @@ def test_gap_lists_down_to_the_smallest_gaps(gpu_ctx, min_gap):
     want = [(int(b), int(b - a)) for a, b in zip(p[:-1], p[1:]) if b - a >= min_gap]
     got = gpu_ctx.gaps_at_least(lo, hi, min_gap)
     assert [(int(a), int(g)) for a, g in zip(got["position"], got["gap"])] == want
+
+
+def test_a_range_longer_than_a_prepass_window_equals_its_parts():
+    """The large-prime bitmap of a long range is pre-sieved in pieces; ranges of one piece do not."""
+    import voss
+    lo, cuts = 10**14 + 11, (0, 1_300_000_017, 2_500_000_000, 3_300_000_001)  # 1.5e9 integers per window
+    with voss.Context(10**14 + 10**10) as ctx:
+        whole = ctx.sieve_range(lo, lo + cuts[-1])
+        parts = [ctx.sieve_range(lo + a, lo + b) for a, b in zip(cuts[:-1], cuts[1:])]
+        assert_range_equal(voss.merge_stats(parts), whole)

@@ -312,7 +312,7 @@ Slot* make_slot(voss_server* S, int* rc) {
   // the large-prime pre-pass bitmap: fixed size, never grown while serving
   W.gbm_budget = C.max_batch_bitmap_bytes;
   W.gbm_fixed = true;
-  if (W.gbm_budget && ((e = W.gbm.ensure(W.gbm_budget)) || (e = W.scat.ensure(sizeof(voss::IntervalScatter) * nreq))))
+  if (W.gbm_budget && ((e = W.gbm.ensure(W.gbm_budget)) || (e = W.scat.ensure(sizeof(voss::IntervalScatter) * (nreq + W.gbm_budget / kScatterWindowBytes + 1)))))
     return bad(e);
   if ((e = W.sh_iv.ensure(sizeof(voss::ShortInterval) * nreq)) || (e = W.sh_map.ensure(sizeof(uint32_t) * nreq)) ||
       (e = W.sh_seg.ensure(sizeof(voss::ShortSegment) * (C.max_batch_candidates / voss::kShortSeg + nreq + 1))))
