@@ -111,13 +111,15 @@ typedef struct voss_interval_stats {
   uint64_t gap_hist[VOSS_IHIST];      /* bin g/2 = #gaps of length g; bin 0 = #gaps of length 1 */
 } voss_interval_stats;
 
-/* Sieve tuning; zero fields take the library's defaults. */
+/* Sieve tuning; zero fields take the library's defaults.  While block_threads, chunk_words, coop_div
+ * and mult_factor are all zero, launches too small for the default tile choose a smaller one. */
 typedef struct voss_tuning {
   uint32_t block_threads;   /* 512 or 1024 */
   uint32_t chunk_words;     /* odd; a tile is block_threads * chunk_words 32-bit words */
   uint32_t ctas_per_sm;     /* resident tiles per SM */
   uint32_t coop_div;        /* primes p < tile_bytes/coop_div are cleared warp-cooperatively */
-  uint32_t mult_factor;     /* primes p >= mult_factor*tile_bytes use the multiples walk */
+  uint32_t mult_factor;     /* primes p >= mult_factor*tile_bytes belong to the large-prime pre-pass (without
+                               one: to a walk of their multiples in the tiles) */
   uint32_t medium_mode;     /* other primes: 0 = a thread per prime, 1 = a lane per (prime, residue) */
   uint32_t walk_sixteenths; /* mode 0: primes p >= walk_sixteenths*tile_bytes/16 are taken by residue class
                                mod 30 instead of 8 residue progressions each (>= 16*mult_factor: never;

@@ -1,6 +1,7 @@
 """The tile kernel at the sizes where its parts can go wrong, against the CPU oracle (exact): the
 last words of a tile, tiles of a few words, tiles without a far gap (the longest gap is then
 searched again), primes taken as small, by progressions and by class in every proportion."""
+import numpy as np
 import pytest
 
 import oracle_lib as O
@@ -63,3 +64,30 @@ def test_a_range_longer_than_a_prepass_window_equals_its_parts():
         whole = ctx.sieve_range(lo, lo + cuts[-1])
         parts = [ctx.sieve_range(lo + a, lo + b) for a, b in zip(cuts[:-1], cuts[1:])]
         assert_range_equal(voss.merge_stats(parts), whole)
+
+
+@pytest.mark.parametrize("words", [1, 1024, 1025, 50175, 50176, 50177, 100353])
+def test_tile_lengths_in_the_large_tile(gpu_ctx, words):
+    """Small launches choose small tiles; the same lengths in the tile that long runs use."""
+    lo = 10**12 - 77
+    hi = lo + WORD * words - 13
+    try:
+        gpu_ctx.set_tuning(chunk_words=49)
+        assert_range_equal(gpu_ctx.sieve_range(lo, hi), O.sieve_range(lo, hi))
+    finally:
+        gpu_ctx.set_tuning()
+
+
+@pytest.mark.parametrize("n,ln", [(1, 10**5), (3, 10**6), (147, 3 * 10**5), (149, 3 * 10**5), (600, 10**5), (900, 10**4)])
+def test_chosen_tile_shapes_equal_the_fixed_one(gpu_ctx, n, ln):
+    rng = np.random.default_rng(n)
+    lo = (10 ** rng.uniform(6, 13, n)).astype(np.uint64)
+    hi = lo + rng.integers(0, 2 * ln, n).astype(np.uint64)
+    chosen = gpu_ctx.sieve_intervals(lo, hi)
+    try:
+        gpu_ctx.set_tuning(chunk_words=49)
+        fixed = gpu_ctx.sieve_intervals(lo, hi)
+    finally:
+        gpu_ctx.set_tuning()
+    for f in chosen.dtype.names:
+        np.testing.assert_array_equal(chosen[f], fixed[f], err_msg=f)

@@ -11,7 +11,7 @@
 //                  small primes  p <  tile_bytes/coop_div : one warp per prime, its hits as 32
 //                                                            progressions that never share a bank,
 //                  medium primes p <  walk bound          : one thread per prime, 8 residues,
-//                                p <  mult_factor*tile_bytes: one thread per prime of one class mod
+//                                p <  p_large           : one thread per prime of one class mod
 //                                                            30, its eight first hits and rounds,
 //                  large primes  otherwise                 : one thread per prime, walking its
 //                                                            multiples across the tile's span;
@@ -670,7 +670,7 @@ __device__ __forceinline__ void tile_header(TileHdr& H, CtaState& St, const Siev
         // one record per thread of the block, and primes that fit a record (clear_small_prime)
         const uint32_t ia0 = count_lt_warp(a.primes, a.n_primes, (uint64_t)min(lt / a.coop_div, kSmallPrimeEnd), ln);
         const uint32_t ia = min(ia0, (uint32_t)blockDim.x);
-        const uint32_t ib = count_lt_warp(a.primes, a.n_primes, (uint64_t)lt * a.mult_factor, ln);
+        const uint32_t ib = count_lt_warp(a.primes, a.n_primes, a.p_large, ln);
         const uint32_t iw = count_lt_warp(a.primes, a.n_primes, ((uint64_t)lt * a.walk_sixteenths) >> 4, ln);
         __syncwarp();
         if (ln == 0) {

@@ -117,6 +117,7 @@ namespace voss_host {
 
 int apply_tuning(voss_ctx* c, const voss_tuning& t0) {
   voss_tuning t = t0;
+  const bool auto_shape = !t.block_threads && !t.chunk_words && !t.coop_div && !t.mult_factor;
   if (!t.block_threads) t.block_threads = 1024;
   if (!t.chunk_words) t.chunk_words = t.block_threads == 1024 ? 49 : 45;
   if (!t.coop_div) t.coop_div = 80;
@@ -144,6 +145,7 @@ int apply_tuning(voss_ctx* c, const voss_tuning& t0) {
     return fail(VOSS_ERR_ARG, "tile of %u words does not fit in shared memory (%zu bytes)", tw, smem);
   if (!t.ctas_per_sm || (int)t.ctas_per_sm > maxc) t.ctas_per_sm = (uint32_t)maxc;
   c->tune = t;
+  c->auto_shape = auto_shape;
   c->ctas_per_sm = (int)t.ctas_per_sm;
   return VOSS_OK;
 }
@@ -183,10 +185,70 @@ int upload_class_primes(voss_ctx* c) {
   return VOSS_OK;
 }
 
+TileShape default_shape(const voss_ctx* c) {
+  const voss_tuning& t = c->tune;
+  return TileShape{t.chunk_words, t.coop_div, (uint32_t)std::min<uint64_t>(
+                       4ull * t.block_threads * t.chunk_words * t.mult_factor, kClsLimit)};
+}
+
+// Tiles of the default shape keep 148 SMs busy from about 10^10 integers on; a smaller launch runs a
+// nearly empty last wave, or leaves most SMs without a tile.  Such a launch takes the chunk length
+// that fills 1..6 waves, by the estimate waves * (chunk + 40): a tile's set-ups cost about what 40
+// words per thread do (1.1 to 1.4 us per word against 40 to 110 us per tile).  With it go
+//  - the pre-pass, which spreads over all SMs: at 40 sqrt(integers) the tiles' share of the
+//    remaining primes costs about what the pre-pass's bitmap atomics do (best of a sweep over
+//    2^11..2^19: 8192, 32768, 131072, 524288 for 10^5..10^8 integers);
+//  - in a single wave, small primes up to tile/20: a warp each instead of a lane each, whose few
+//    dozen clears in a row were the longest chain of such a launch.
+// Device time before and after: 10^6 integers at 10^12 115 -> 62 us, 10^7 203 -> 73, 10^8 201 -> 121,
+// 10^9 365 -> 317; [1, 10^8] 306 -> 92, [1, 10^9] 307 -> 266.
+TileShape choose_shape(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, uint32_t n, uint64_t max_tiles) {
+  constexpr uint64_t kMaxWaves = 6;
+  constexpr double kTileSetup = 40.0;
+  const TileShape dflt = default_shape(c);
+  const uint64_t slots = (uint64_t)c->sm_count * c->ctas_per_sm, block = c->tune.block_threads;
+  if (!c->auto_shape || n > kMaxWaves * slots) return dflt;
+  std::vector<uint64_t> words;
+  words.reserve(n);
+  uint64_t total = 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    const uint64_t a = std::max<uint64_t>(lo[i], 7);
+    if (a >= hi[i]) continue;
+    words.push_back(((hi[i] - 1) / 30 - ((a / 30) & ~3ull)) / 4 + 1);
+    total += words.back();
+  }
+  if (total == 0 || total > kMaxWaves * slots * block * dflt.chunk_words) return dflt;
+  auto waves_of = [&](uint64_t chunk) -> uint64_t {
+    uint64_t tiles = 0;
+    for (uint64_t w : words) tiles += (w + block * chunk - 1) / (block * chunk);
+    return max_tiles && tiles > max_tiles ? 0 : (tiles + slots - 1) / slots;
+  };
+  uint64_t best = dflt.chunk_words, best_waves = waves_of(best);
+  double cost = 0.95 * (double)best_waves * ((double)best + kTileSetup);  // at least 5 % better
+  for (uint64_t k = 1; k <= kMaxWaves; ++k) {
+    const uint64_t chunk = ((total + block * k * slots - 1) / (block * k * slots)) | 1;
+    if (chunk >= dflt.chunk_words) continue;
+    const uint64_t waves = waves_of(chunk);
+    if (waves && (double)waves * ((double)chunk + kTileSetup) < cost) {
+      best = chunk;
+      best_waves = waves;
+      cost = (double)waves * ((double)chunk + kTileSetup);
+    }
+  }
+  if (best == dflt.chunk_words) return dflt;
+  TileShape s = dflt;
+  s.chunk_words = (uint32_t)best;
+  const double reach = 40.0 * std::sqrt(120.0 * (double)total);
+  s.p_large = (uint32_t)std::min<double>(dflt.p_large, std::max(8192.0, reach));
+  if (best_waves == 1) s.coop_div = std::max(1u, dflt.coop_div / 4);
+  return s;
+}
+
 // Cut intervals [lo_i, hi_i) into tiles; intervals without wheel integers get no tiles.
 int plan_intervals(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, uint32_t n,
-                   uint64_t seg_k, RunPlan* P) {
-  const uint64_t tw = (uint64_t)c->tune.block_threads * c->tune.chunk_words;
+                   uint64_t seg_k, const TileShape& shape, RunPlan* P) {
+  const uint64_t tw = (uint64_t)c->tune.block_threads * shape.chunk_words;
+  P->shape = shape;
   P->iv.resize(n);
   uint64_t tiles = 0, words = 0;
   for (uint32_t i = 0; i < n; ++i) {
@@ -248,10 +310,10 @@ int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPl
   a.iv = W.iv.as<IntervalDev>();
   a.n_intervals = n_iv;
   a.n_tiles = P.n_tiles;
-  a.tile_words = c->tune.block_threads * c->tune.chunk_words;
-  a.chunk_words = c->tune.chunk_words;
-  a.coop_div = c->tune.coop_div;
-  a.mult_factor = c->tune.mult_factor;
+  a.tile_words = c->tune.block_threads * P.shape.chunk_words;
+  a.chunk_words = P.shape.chunk_words;
+  a.coop_div = P.shape.coop_div;
+  a.p_large = P.shape.p_large;
   a.walk_sixteenths = c->tune.walk_sixteenths;
   a.want_large = want_large ? 1u : 0u;
   a.large_min_gap = min_gap;
@@ -277,9 +339,9 @@ int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPl
   const size_t smem = sieve_smem_bytes(tw);
   const int slots = c->sm_count * c->ctas_per_sm;
   const int grid = (int)std::max<uint32_t>(1, std::min<uint32_t>(P.n_tiles, (uint32_t)slots));
-  // Large-prime pre-pass: primes p >= mult_factor * tile bytes are applied once per launch
-  // (prime-major) instead of once per tile, when the launch's bitmap fits the budget.
-  const uint64_t p_large = (uint64_t)c->tune.mult_factor * 4ull * tw;
+  // Large-prime pre-pass: primes p >= p_large are applied once per launch (prime-major) instead of
+  // once per tile, when the launch's bitmap fits the budget.
+  const uint64_t p_large = P.shape.p_large;
   uint64_t max_sq = 0;
   for (const IntervalDev& d : P.iv)
     if (d.n_tiles) max_sq = std::max<uint64_t>(max_sq, isqrt_u64(d.hi - 1));
@@ -288,7 +350,7 @@ int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPl
                                                   (uint32_t)std::min<uint64_t>(max_sq, 0xFFFFFFFFull)) -
                                  c->primes.begin());
   const size_t gbm_bytes = (size_t)P.n_words * 4;
-  bool scatter = P.n_tiles && j1 > j0 && p_large <= 0xFFFFFFFFull && gbm_bytes <= W.gbm_budget &&
+  bool scatter = P.n_tiles && j1 > j0 && gbm_bytes <= W.gbm_budget &&
                  (!W.gbm_fixed || gbm_bytes <= W.gbm.bytes);
   std::vector<IntervalScatter> sc;
   // Windows of consecutive intervals whose bitmap words total at most kScatterWindowBytes: the
@@ -574,7 +636,9 @@ int launch_routed(voss_ctx* c, Workspace& W, const LaunchEvents& E, const Interv
   uint32_t k = 0;
   if (!R.lo.empty()) {
     RunPlan P;
-    if ((rc = plan_intervals(c, R.lo.data(), R.hi.data(), (uint32_t)R.lo.size(), 0, &P))) return rc;
+    const TileShape shape = choose_shape(c, R.lo.data(), R.hi.data(), (uint32_t)R.lo.size(),
+                                         W.gbm_fixed ? W.partials.bytes / sizeof(TilePartial) : 0);
+    if ((rc = plan_intervals(c, R.lo.data(), R.hi.data(), (uint32_t)R.lo.size(), 0, shape, &P))) return rc;
     SieveArgs a;
     if ((rc = launch_plan_ws(c, W, E, P, false, 0, false, s, 0, &a))) return rc;
     k = (uint32_t)(&W == &c->ws ? c->last_kernels : 3) + 1;
@@ -788,7 +852,7 @@ int run_range_device(voss_ctx* c, uint64_t lo, uint64_t hi, uint32_t flags, uint
   int rc;
   {
     NvtxRange r("plan");
-    rc = plan_intervals(c, &lo, &hi, 1, seg_k, &P);
+    rc = plan_intervals(c, &lo, &hi, 1, seg_k, choose_shape(c, &lo, &hi, 1, 0), &P);
   }
   if (rc) return rc;
   {
@@ -1107,7 +1171,7 @@ VOSS_API int voss_gaps_at_least(voss_ctx* c, uint64_t lo, uint64_t hi, uint32_t 
   if (hi > c->max_hi) return fail(VOSS_ERR_RANGE, "hi exceeds the context limit");
   cudaSetDevice(c->device);
   RunPlan P;
-  int rc = plan_intervals(c, &lo, &hi, 1, 0, &P);
+  int rc = plan_intervals(c, &lo, &hi, 1, 0, choose_shape(c, &lo, &hi, 1, 0), &P);
   if (rc) return rc;
   const uint64_t devcap = std::min<uint64_t>(std::max<uint64_t>(cap, 1), kMaxLargeCap);
   rc = launch_plan(c, P, true, devcap, false, c->stream, min_gap);
@@ -1136,7 +1200,7 @@ VOSS_API int voss_primes_range(voss_ctx* c, uint64_t lo, uint64_t hi, uint64_t* 
   cudaSetDevice(c->device);
   cudaStream_t s = c->stream;
   RunPlan P;
-  int rc = plan_intervals(c, &lo, &hi, 1, 0, &P);
+  int rc = plan_intervals(c, &lo, &hi, 1, 0, choose_shape(c, &lo, &hi, 1, 0), &P);
   if (rc) return rc;
   // pass 1: per-tile counts
   rc = launch_plan(c, P, false, 0, false, s);

@@ -31,7 +31,7 @@ int count_tiles(voss_ctx* c, uint64_t lo, uint64_t hi, RunPlan* P, std::vector<u
   P->iv.clear();
   P->n_tiles = 0;
   if (a >= hi) return VOSS_OK;
-  int rc = plan_intervals(c, &a, &hi, 1, 0, P);
+  int rc = plan_intervals(c, &a, &hi, 1, 0, choose_shape(c, &a, &hi, 1, 0), P);
   if (rc) return rc;
   LaunchEvents E{c->ev0, c->ev1, c->ev2, c->evp};
   rc = launch_plan_ws(c, c->ws, E, *P, false, 0, false, s, 0, nullptr);
@@ -60,13 +60,13 @@ int emit_window(voss_ctx* c, const RunPlan& P, const std::vector<uint64_t>& pref
   uint32_t t0 = 0, t1 = P.n_tiles - 1;
   while (prefix[t0 + 1] <= r0) ++t0;
   while (t1 > t0 && prefix[t1] >= r1) --t1;
-  const uint64_t tw = (uint64_t)c->tune.block_threads * c->tune.chunk_words;
+  const uint64_t tw = (uint64_t)c->tune.block_threads * P.shape.chunk_words;
   const voss::IntervalDev& d = P.iv[0];
   const uint64_t sub_lo = t0 == 0 ? d.lo : 30ull * (d.k0 + 4ull * tw * t0);
   const uint64_t sub_hi = std::min<uint64_t>(hi, 30ull * (d.k0 + 4ull * tw * (t1 + 1)));
   RunPlan Q;
   int rc;
-  if ((rc = plan_intervals(c, &sub_lo, &sub_hi, 1, 0, &Q))) return rc;
+  if ((rc = plan_intervals(c, &sub_lo, &sub_hi, 1, 0, P.shape, &Q))) return rc;
   std::vector<unsigned long long> offs(std::max<uint32_t>(1, Q.n_tiles));
   for (uint32_t t = 0; t < Q.n_tiles; ++t) offs[t] = prefix[t0 + t] - r0;  // wraps below r0: not written
   const uint64_t n = r1 - r0;

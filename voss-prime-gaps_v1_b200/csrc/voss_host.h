@@ -83,8 +83,16 @@ struct LaunchEvents {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, evp = nullptr;
 };
 
+// How a launch cuts its intervals into tiles and its base primes into categories.
+struct TileShape {
+  uint32_t chunk_words = 0;  // 32-bit words per thread of a tile
+  uint32_t coop_div = 0;     // as voss_tuning
+  uint32_t p_large = 0;      // primes from here on belong to the pre-pass
+};
+
 struct RunPlan {
   std::vector<voss::IntervalDev> iv;
+  TileShape shape;
   uint32_t n_tiles = 0;
   uint64_t n_words = 0;
 };
@@ -121,6 +129,7 @@ struct voss_ctx {
   uint32_t cls_first[8] = {0};
   uint32_t n_cls_blocks = 0;
   voss_tuning tune{};
+  bool auto_shape = true;  // the tile shape was left to the library: small launches choose their own
   int ctas_per_sm = 1;
   voss_host::Workspace ws;
   // last range run
@@ -149,9 +158,14 @@ struct voss_ctx {
 
 namespace voss_host {
 
+// The context's tile shape.
+TileShape default_shape(const voss_ctx* c);
+// The shape for a launch of these intervals (at most max_tiles tiles, 0: no limit): the context's,
+// or a smaller one when the launch would leave SMs idle.
+TileShape choose_shape(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, uint32_t n, uint64_t max_tiles);
 // Cut intervals [lo_i, hi_i) into tiles; intervals without wheel integers get no tiles.
 int plan_intervals(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, uint32_t n, uint64_t seg_k,
-                   RunPlan* P);
+                   const TileShape& shape, RunPlan* P);
 // Queue the tile kernel (+ stitch and reduce unless emit) for plan P on stream s, using the
 // workspace W and events E.
 int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPlan& P, bool want_large,

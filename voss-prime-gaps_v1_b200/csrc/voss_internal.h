@@ -166,7 +166,7 @@ struct SieveArgs {
   uint32_t tile_words;
   uint32_t chunk_words;     // odd; tile_words = blockDim.x * chunk_words
   uint32_t coop_div;
-  uint32_t mult_factor;
+  uint32_t p_large;         // base primes from here on: applied by the pre-pass, or multiple by multiple
   uint32_t walk_sixteenths;
   uint32_t want_large;      // record large gaps
   uint32_t large_min_gap;   // 0: the reference's rule (gap >= 500 or merit >= 10); else every gap >= it
