@@ -327,8 +327,8 @@ VOSS_API int voss_probe_mulmod(voss_ctx* ctx, double* full_per_s, double* small_
  * the tile kernel, total_ms to the end of its last kernel. */
 VOSS_API int voss_last_kernel_ms(const voss_ctx* ctx, double* sieve_ms, double* total_ms);
 /* The same launch in three consecutive phases: prepass_ms = descriptor copies, memsets and the
- * large-prime pre-pass kernels; tile_ms = the tile kernel alone; tail_ms = the stitch, reduce and
- * (intervals) finalize kernels; kernels = how many kernels the launch ran. */
+ * large-prime pre-pass kernels; tile_ms = the tile kernel alone; tail_ms = the kernels behind it
+ * (seams, interval results, the sort of a short gap list); kernels = how many the launch ran. */
 VOSS_API int voss_last_phase_ms(const voss_ctx* ctx, double* prepass_ms, double* tile_ms, double* tail_ms,
                                 uint32_t* kernels);
 

@@ -91,3 +91,15 @@ def test_chosen_tile_shapes_equal_the_fixed_one(gpu_ctx, n, ln):
         gpu_ctx.set_tuning()
     for f in chosen.dtype.names:
         np.testing.assert_array_equal(chosen[f], fixed[f], err_msg=f)
+
+
+@pytest.mark.parametrize("ln", [10**5, 3 * 10**6, 11 * 10**6, 4 * 10**7, 5 * 10**7, 2 * 10**8])
+def test_gap_lists_of_every_sort_in_order(gpu_ctx, ln):
+    """Lists around 4096 records (copied with the state), 16384 (ranked) and beyond (radix sorted)."""
+    lo = 10**12
+    got = gpu_ctx.gaps_at_least(lo, lo + ln, 150)
+    p = O.primes_range(lo, lo + ln)
+    d = np.diff(p)
+    np.testing.assert_array_equal(got["position"], p[1:][d >= 150])
+    np.testing.assert_array_equal(got["gap"], d[d >= 150])
+    assert gpu_ctx.gaps_at_least(lo, lo + ln, 150, cap=max(1, got.size)).size == got.size

@@ -23,10 +23,11 @@
 //                block-wide max-scan of the chunks' last primes, and updates shared-memory
 //                counters: the gap histogram (:278-280), the per-residue gap histogram (:282-287),
 //                the large-gap list (:289-299) and the tile's maximal gap.  Primes never reach HBM.
-// The gaps across tile seams are added by stitch_kernel; reduce_kernel gives each interval its
-// first/last prime and maximal gap.
+// The gaps across tile seams and each interval's first/last prime and maximal gap come from
+// tail_kernel.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdint>
@@ -1297,14 +1298,12 @@ sieve_tiles_kernel(SieveArgs a) {
 #endif
 }
 
-// Gap between the last prime of the previous non-empty tile and this tile's first prime.
-__global__ void stitch_kernel(SieveArgs a) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= a.n_tiles) return;
-  const TilePartial P = a.partials[t];
-  if (P.count == 0) return;
-  const uint32_t ivx = find_interval(a, t);
-  const IntervalDev iv = a.iv[ivx];
+// The gap between the last prime of the previous non-empty tile and tile t's first prime (P, not
+// empty): counted, and kept in *gap / *gap_lo (0: none).
+__device__ __forceinline__ void tile_seam(const SieveArgs& a, const IntervalDev& iv, uint32_t ivx, uint32_t t,
+                                          const TilePartial& P, uint32_t* gap, uint64_t* gap_lo) {
+  *gap = 0;
+  *gap_lo = 0;
   uint32_t tp = t;
   bool found = false;
   while (tp > iv.tile_begin) {
@@ -1333,8 +1332,8 @@ __global__ void stitch_kernel(SieveArgs a) {
     if (slot < a.over_cap) a.over[slot] = OverflowGap{ivx, (uint32_t)(g > 0xFFFFFFFFull ? 0xFFFFFFFFull : g)};
     else atomicOr(a.error, kErrOverflowList);
   }
-  a.partials[t].bgap = (uint32_t)(g > 0xFFFFFFFFull ? 0xFFFFFFFFull : g);
-  a.partials[t].bgap_lo = lo_p;
+  *gap = (uint32_t)(g > 0xFFFFFFFFull ? 0xFFFFFFFFull : g);
+  *gap_lo = lo_p;
   const bool cand = a.large_min_gap ? (g >= a.large_min_gap) : (g > 100);
   if (a.want_large && cand && !crossing) {
     const double merit_d = (double)g / log((double)lo_p);
@@ -1348,95 +1347,126 @@ __global__ void stitch_kernel(SieveArgs a) {
   }
 }
 
-// One block per interval: first/last prime and the first maximal gap.
-__global__ void reduce_kernel(SieveArgs a, IntervalOut* out) {
-  const uint32_t ivx = blockIdx.x;
-  if (ivx >= a.n_intervals) return;
+// The seams of a launch with many tiles per interval, a thread per tile (kept in the partials).
+__global__ void stitch_kernel(SieveArgs a) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= a.n_tiles) return;
+  const TilePartial P = a.partials[t];
+  if (P.count == 0) return;
+  const uint32_t ivx = find_interval(a, t);
   const IntervalDev iv = a.iv[ivx];
-  __shared__ uint32_t s_first, s_last, s_gap;
-  __shared__ unsigned long long s_lo;
+  uint32_t gap;
+  uint64_t gap_lo;
+  tile_seam(a, iv, ivx, t, P, &gap, &gap_lo);
+  a.partials[t].bgap = gap;
+  a.partials[t].bgap_lo = gap_lo;
+}
+
+// One block per interval, after its tiles: the seams between them (unless stitch_kernel ran), first
+// and last prime, the first maximal gap; with `stats`, the accumulators folded into
+// voss_interval_stats, so that only the result crosses to the host (lo, hi and the primes 2, 3, 5
+// are filled in there).  One launch instead of three of 2 to 5 us each, which a launch of a few
+// tiles notices.
+constexpr int kTailBlock = 256;
+
+__global__ void __launch_bounds__(kTailBlock) tail_kernel(SieveArgs a, bool stitched, IntervalOut* out,
+                                                          voss_interval_stats* stats, const uint32_t* out_index) {
+  const uint32_t ivx = blockIdx.x;
+  const IntervalDev iv = a.iv[ivx];
+  __shared__ uint32_t s_first, s_last;
+  __shared__ unsigned long long s_gap[kTailBlock / 32], s_lo[kTailBlock / 32];
   if (threadIdx.x == 0) {
     s_first = kNone;
     s_last = 0;
-    s_gap = 0;
-    s_lo = ~0ull;
   }
   __syncthreads();
-  uint32_t my_first = kNone, my_last = 0, my_gap = 0;
-  for (uint32_t i = threadIdx.x; i < iv.n_tiles; i += blockDim.x) {
+  uint32_t my_first = kNone, my_last = 0;
+  unsigned long long my_gap = 0, my_lo = ~0ull;
+  auto longer = [&](unsigned long long g, unsigned long long lo) {  // ties: the smaller lower prime
+    if (g > my_gap || (g == my_gap && lo < my_lo)) {
+      my_gap = g;
+      my_lo = lo;
+    }
+  };
+  for (uint32_t i = threadIdx.x; i < iv.n_tiles; i += kTailBlock) {
     const TilePartial P = a.partials[iv.tile_begin + i];
     if (!P.count) continue;
     my_first = min(my_first, i);
     my_last = max(my_last, i + 1);
-    my_gap = max(my_gap, max(P.max_gap, P.bgap));
+    uint32_t bgap = P.bgap;
+    uint64_t bgap_lo = P.bgap_lo;
+    if (!stitched) tile_seam(a, iv, ivx, iv.tile_begin + i, P, &bgap, &bgap_lo);
+    if (P.max_gap) longer(P.max_gap, 30ull * (iv.k0 + 4ull * a.tile_words * i) + P.max_lo);
+    if (bgap) longer(bgap, bgap_lo);
   }
   atomicMin(&s_first, my_first);
   atomicMax(&s_last, my_last);
-  atomicMax(&s_gap, my_gap);
-  __syncthreads();
-  const uint32_t G = s_gap;
-  unsigned long long my_lo = ~0ull;
-  if (G) {
-    for (uint32_t i = threadIdx.x; i < iv.n_tiles; i += blockDim.x) {
-      const TilePartial P = a.partials[iv.tile_begin + i];
-      if (!P.count) continue;
-      const uint64_t vt = 30ull * (iv.k0 + 4ull * a.tile_words * i);
-      if (P.max_gap == G) my_lo = min(my_lo, (unsigned long long)(vt + P.max_lo));
-      if (P.bgap == G) my_lo = min(my_lo, (unsigned long long)P.bgap_lo);
-    }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const unsigned long long g = __shfl_down_sync(0xFFFFFFFFu, my_gap, d);
+    const unsigned long long lo = __shfl_down_sync(0xFFFFFFFFu, my_lo, d);
+    longer(g, lo);
   }
-  atomicMin(&s_lo, my_lo);
+  if ((threadIdx.x & 31) == 0) {
+    s_gap[threadIdx.x >> 5] = my_gap;
+    s_lo[threadIdx.x >> 5] = my_lo;
+  }
+  __threadfence();  // the seams of the block are in the accumulators
   __syncthreads();
+  voss_interval_stats* s = stats ? stats + (out_index ? out_index[ivx] : ivx) : nullptr;
+  const unsigned long long* A = a.acc + (size_t)ivx * kAccStride;
   if (threadIdx.x == 0) {
+    for (int w = 1; w < kTailBlock / 32; ++w) longer(s_gap[w], s_lo[w]);
     IntervalOut o;
-    if (s_first == kNone) {
-      o.first = o.last = 0;
-    } else {
+    o.first = o.last = 0;
+    if (s_first != kNone) {
       const TilePartial F = a.partials[iv.tile_begin + s_first];
       const TilePartial L = a.partials[iv.tile_begin + s_last - 1];
       o.first = 30ull * (iv.k0 + 4ull * a.tile_words * s_first) + F.first;
       o.last = 30ull * (iv.k0 + 4ull * a.tile_words * (s_last - 1)) + L.last;
     }
-    o.max_gap = G;
-    o.max_gap_lo = G ? s_lo : 0;
+    o.max_gap = my_gap;
+    o.max_gap_lo = my_gap ? my_lo : 0;
     out[ivx] = o;
+    if (s) {
+      s->lo = 0;
+      s->hi = 0;
+      s->prime_count = __ldcg(A + kAccCount);
+      s->first_prime = o.first;
+      s->last_prime = o.last;
+      s->max_gap = o.max_gap;
+      s->max_gap_lo = o.max_gap_lo;
+      s->gap_overflow = __ldcg(A + kAccHistOver);
+    }
   }
-}
-
-// One block per interval: fold the accumulators into voss_interval_stats on the device, so
-// that only the result (not the raw counters) crosses to the host.  lo/hi and the primes
-// 2, 3, 5 are filled in on the host.
-__global__ void interval_finalize_kernel(SieveArgs a, const IntervalOut* io, voss_interval_stats* out,
-                                         const uint32_t* out_index) {
-  const uint32_t ivx = blockIdx.x;
-  if (ivx >= a.n_intervals) return;
-  const unsigned long long* A = a.acc + (size_t)ivx * kAccStride;
-  voss_interval_stats* s = out + (out_index ? out_index[ivx] : ivx);
-  for (uint32_t b = threadIdx.x; b < (uint32_t)VOSS_IHIST; b += blockDim.x) {
+  if (!s) return;
+  for (uint32_t b = threadIdx.x; b < (uint32_t)VOSS_IHIST; b += kTailBlock) {
     unsigned long long v = 0;
     if (b > 0) {
-      v = A[kAccHist + b];
+      v = __ldcg(A + kAccHist + b);
       if (b < (uint32_t)kModqBins)
-        for (uint32_t o = 0; o < 8; ++o) v += A[kAccModq + o * kModqBins + b];
+        for (uint32_t o = 0; o < 8; ++o) v += __ldcg(A + kAccModq + o * kModqBins + b);
     }
     s->gap_hist[b] = v;
   }
-  if (threadIdx.x == 0) {
-    s->lo = 0;
-    s->hi = 0;
-    s->prime_count = A[kAccCount];
-    s->first_prime = io[ivx].first;
-    s->last_prime = io[ivx].last;
-    s->max_gap = io[ivx].max_gap;
-    s->max_gap_lo = io[ivx].max_gap_lo;
-    s->gap_overflow = A[kAccHistOver];
-  }
 }
 
-int launch_interval_finalize(const SieveArgs& a, const IntervalOut* io, voss_interval_stats* out,
-                             const uint32_t* out_index, void* stream) {
-  if (a.n_intervals == 0) return 0;
-  interval_finalize_kernel<<<a.n_intervals, 256, 0, (cudaStream_t)stream>>>(a, io, out, out_index);
+// Zeroes the launch's counters and accumulators and fills its large-prime bitmap with ones in one
+// launch (a memset of each takes about as long).
+__global__ void init_kernel(uint4* zero, size_t n_zero, uint32_t* ones, size_t n_ones) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (size_t i = first; i < n_zero; i += stride) zero[i] = make_uint4(0, 0, 0, 0);
+  uint4* ones4 = reinterpret_cast<uint4*>(ones);
+  for (size_t i = first; i < n_ones / 4; i += stride) ones4[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+  for (size_t i = (n_ones & ~(size_t)3) + first; i < n_ones; i += stride) ones[i] = ~0u;
+}
+
+int launch_init(void* zero, size_t zero_bytes, uint32_t* ones, size_t n_ones, int sm_count, void* stream) {
+  const size_t n_zero = zero_bytes / sizeof(uint4);
+  const size_t want = (std::max(n_zero, n_ones / 4) + 255) / 256 + 1;
+  const int grid = (int)std::min<size_t>(want, (size_t)sm_count * 16);
+  init_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((uint4*)zero, n_zero, ones, n_ones);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1679,16 +1709,15 @@ int launch_sieve_emit(const SieveArgs& a, int grid, int block, size_t smem, void
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int launch_stitch(const SieveArgs& a, void* stream) {
-  if (a.n_tiles == 0) return 0;
-  const int blk = 256;
-  stitch_kernel<<<(a.n_tiles + blk - 1) / blk, blk, 0, (cudaStream_t)stream>>>(a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-int launch_reduce(const SieveArgs& a, IntervalOut* out, void* stream) {
+int launch_tail(const SieveArgs& a, uint32_t max_tiles, IntervalOut* out, voss_interval_stats* stats,
+                const uint32_t* out_index, void* stream, uint32_t* kernels) {
   if (a.n_intervals == 0) return 0;
-  reduce_kernel<<<a.n_intervals, 256, 0, (cudaStream_t)stream>>>(a, out);
+  // one interval of few tiles: its block takes the seams along.  In a batch the intervals' numbers of
+  // tiles differ by thousands, and a thread per tile evens them out.
+  const bool stitched = a.n_tiles > 0 && (a.n_intervals > 1 || max_tiles > 8u * kTailBlock);
+  if (stitched) stitch_kernel<<<(a.n_tiles + 255) / 256, 256, 0, (cudaStream_t)stream>>>(a);
+  tail_kernel<<<a.n_intervals, kTailBlock, 0, (cudaStream_t)stream>>>(a, stitched, out, stats, out_index);
+  *kernels += stitched ? 2 : 1;
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

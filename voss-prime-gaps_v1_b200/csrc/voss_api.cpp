@@ -282,14 +282,12 @@ int plan_intervals(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, ui
 
 
 int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPlan& P, bool want_large,
-                   uint64_t large_cap, bool emit, cudaStream_t s, uint32_t min_gap, SieveArgs* args_out) {
+                   uint64_t large_cap, bool emit, cudaStream_t s, uint32_t min_gap, voss_interval_stats* stats,
+                   const uint32_t* out_index, uint32_t* kernels) {
   const uint32_t n_iv = (uint32_t)P.iv.size();
   int rc;
-  if ((rc = W.iv.ensure(sizeof(IntervalDev) * std::max<size_t>(1, n_iv)))) return rc;
   if ((rc = W.partials.ensure(sizeof(TilePartial) * std::max<size_t>(1, P.n_tiles)))) return rc;
-  if ((rc = W.acc.ensure(sizeof(unsigned long long) * kAccStride * std::max<size_t>(1, n_iv)))) return rc;
-  if ((rc = W.out.ensure(sizeof(IntervalOut) * std::max<size_t>(1, n_iv)))) return rc;
-  if ((rc = W.counters.ensure(sizeof(uint32_t) * kCtrWords))) return rc;
+  if ((rc = W.state.ensure(state_bytes(n_iv)))) return rc;
   if ((rc = W.over.ensure(sizeof(OverflowGap) * kOverCap))) return rc;
   const uint64_t cap = want_large ? std::min(std::max(large_cap, (uint64_t)1), kMaxLargeCap) : 1;
   if ((rc = W.large.ensure(sizeof(LargeGapDev) * cap))) return rc;
@@ -307,7 +305,6 @@ int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPl
   std::memcpy(a.cls_first, c->cls_first, sizeof(a.cls_first));
   a.n_cls_blocks = c->n_cls_blocks;
   a.pretab = c->d_pretab.as<uint32_t>();
-  a.iv = W.iv.as<IntervalDev>();
   a.n_intervals = n_iv;
   a.n_tiles = P.n_tiles;
   a.tile_words = c->tune.block_threads * P.shape.chunk_words;
@@ -318,13 +315,14 @@ int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPl
   a.want_large = want_large ? 1u : 0u;
   a.large_min_gap = min_gap;
   a.b_mode = c->tune.medium_mode;
-  uint32_t* ctr = W.counters.as<uint32_t>();
+  const LaunchState L = state_of(W, n_iv);
+  uint32_t* ctr = L.ctr;
   a.tile_counter = ctr + kCtrTile;
   a.large_count = ctr + kCtrLarge;
   a.over_count = ctr + kCtrOver;
   a.error = ctr + kCtrError;
   a.partials = W.partials.as<TilePartial>();
-  a.acc = W.acc.as<unsigned long long>();
+  a.acc = L.acc;
   a.large = W.large.as<LargeGapDev>();
   a.large_iv = W.large_iv.as<uint32_t>();
   a.large_cap = (uint32_t)cap;
@@ -393,62 +391,76 @@ int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPl
                 [](const IntervalScatter& x, const IntervalScatter& y) { return x.sqrt_hi > y.sqrt_hi; });
       w.j1 = (uint32_t)(std::upper_bound(c->primes.begin(), c->primes.end(), sc[w.off].sqrt_hi) - c->primes.begin());
     }
-    if ((rc = W.gbm.ensure(gbm_bytes)) || (rc = W.scat.ensure(sizeof(IntervalScatter) * sc.size()))) return rc;
+    if ((rc = W.gbm.ensure(gbm_bytes))) return rc;
     a.gbm = W.gbm.as<uint32_t>();
     a.scatter_first = j0;
   }
   // Tiles of a launch of many intervals find their interval in a table (one load) rather than
   // by a binary search of the interval descriptors in the tile header.
-  std::vector<uint32_t> tiv;
-  if (n_iv > 1 && P.n_tiles) {
-    tiv.resize(P.n_tiles);
+  const size_t n_tiv = n_iv > 1 ? P.n_tiles : 0;
+  // the descriptors cross in one copy: intervals | pre-pass intervals | interval of each tile
+  std::vector<char> desc(desc_bytes(n_iv, sc.size(), n_tiv));
+  const size_t sc_off = desc_bytes(n_iv, 0, 0), tiv_off = desc_bytes(n_iv, sc.size(), 0);
+  if ((rc = W.desc.ensure(std::max<size_t>(desc.size(), 1)))) return rc;
+  a.iv = reinterpret_cast<const IntervalDev*>(W.desc.as<char>());
+  const IntervalScatter* d_scat = reinterpret_cast<const IntervalScatter*>(W.desc.as<char>() + sc_off);
+  if (n_iv) std::memcpy(desc.data(), P.iv.data(), sizeof(IntervalDev) * n_iv);
+  if (!sc.empty()) std::memcpy(desc.data() + sc_off, sc.data(), sizeof(IntervalScatter) * sc.size());
+  uint32_t max_tiles = 0;
+  for (uint32_t i = 0; i < n_iv; ++i) max_tiles = std::max(max_tiles, P.iv[i].n_tiles);
+  if (n_tiv) {
+    uint32_t* tiv = reinterpret_cast<uint32_t*>(desc.data() + tiv_off);
     for (uint32_t i = 0; i < n_iv; ++i)
       for (uint32_t t = 0; t < P.iv[i].n_tiles; ++t) tiv[P.iv[i].tile_begin + t] = i;
-    if ((rc = W.tile_iv.ensure(sizeof(uint32_t) * P.n_tiles))) return rc;
-    a.tile_iv = W.tile_iv.as<uint32_t>();
+    a.tile_iv = reinterpret_cast<const uint32_t*>(W.desc.as<char>() + tiv_off);
   }
   // Device work of the launch, all of it after ev0 (the host planning above is done first, so
   // the GPU never waits on the host inside the events).
+  uint32_t k = 0;
   CUDA_TRY(cudaEventRecord(E.ev0, s));
-  if (n_iv) CUDA_TRY(cudaMemcpyAsync(W.iv.p, P.iv.data(), sizeof(IntervalDev) * n_iv, cudaMemcpyHostToDevice, s));
-  if (!tiv.empty())
-    CUDA_TRY(cudaMemcpyAsync(W.tile_iv.p, tiv.data(), sizeof(uint32_t) * tiv.size(), cudaMemcpyHostToDevice, s));
-  if (!emit) CUDA_TRY(cudaMemsetAsync(W.acc.p, 0, sizeof(unsigned long long) * kAccStride * std::max<size_t>(1, n_iv), s));
-  CUDA_TRY(cudaMemsetAsync(W.counters.p, 0, sizeof(uint32_t) * kCtrWords, s));
+  if (!desc.empty()) CUDA_TRY(cudaMemcpyAsync(W.desc.p, desc.data(), desc.size(), cudaMemcpyHostToDevice, s));
+  const size_t zero_bytes = emit ? kCtrBytes : L.bytes;
   if (scatter) {
-    CUDA_TRY(cudaMemsetAsync(W.gbm.p, 0xFF, gbm_bytes, s));
-    CUDA_TRY(cudaMemcpyAsync(W.scat.p, sc.data(), sizeof(IntervalScatter) * sc.size(), cudaMemcpyHostToDevice, s));
+    if (launch_init(W.state.p, zero_bytes, W.gbm.as<uint32_t>(), gbm_bytes / 4, c->sm_count, s))
+      return fail(VOSS_ERR_CUDA, "launch set-up failed");
+    ++k;
+  } else {
+    CUDA_TRY(cudaMemsetAsync(W.state.p, 0, zero_bytes, s));
   }
-  for (const Window& w : wins)
-    if (launch_scatter_large(a.primes, a.magic, j0, w.j1, W.scat.as<IntervalScatter>() + w.off, w.n,
-                             W.gbm.as<uint32_t>(), c->sm_count, s))
+  for (const Window& w : wins) {
+    if (launch_scatter_large(a.primes, a.magic, j0, w.j1, d_scat + w.off, w.n, W.gbm.as<uint32_t>(), c->sm_count, s))
       return fail(VOSS_ERR_CUDA, "large-prime pre-pass launch failed");
+    ++k;
+  }
   if (E.evp) CUDA_TRY(cudaEventRecord(E.evp, s));
   if (P.n_tiles) {
     int lr = emit ? launch_sieve_emit(a, grid, (int)c->tune.block_threads, smem, s)
                   : launch_sieve_stats(a, grid, (int)c->tune.block_threads, smem, s);
     if (lr) return fail(VOSS_ERR_CUDA, "sieve launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+    ++k;
   }
   CUDA_TRY(cudaEventRecord(E.ev1, s));
-  if (!emit) {
-    if (launch_stitch(a, s)) return fail(VOSS_ERR_CUDA, "stitch launch failed");
-    if (launch_reduce(a, W.out.as<IntervalOut>(), s)) return fail(VOSS_ERR_CUDA, "reduce launch failed");
+  if (!emit && launch_tail(a, max_tiles, L.out, stats, out_index, s, &k))
+    return fail(VOSS_ERR_CUDA, "tail launch failed");
+  if (want_large) {  // short lists are sorted where the host need not know their length yet
+    if ((rc = W.ls_sorted.ensure(sizeof(LargeGapDev) * kSmallSort))) return rc;
+    if (launch_large_sort_small(a.large, a.large_count, a.large_cap, W.ls_sorted.as<LargeGapDev>(), s))
+      return fail(VOSS_ERR_CUDA, "large-gap sort launch failed");
+    ++k;
   }
   CUDA_TRY(cudaEventRecord(E.ev2, s));
-  if (&W == &c->ws)  // the context's own launches (server slots keep their own workspaces)
-    c->last_kernels = (uint32_t)wins.size() + (P.n_tiles ? 1u : 0u) + (emit ? 0u : 2u);
-  if (args_out) *args_out = a;
+  *kernels = k;
   return VOSS_OK;
 }
 
 int launch_plan(voss_ctx* c, const RunPlan& P, bool want_large, uint64_t large_cap, bool emit, cudaStream_t s,
-                uint32_t min_gap = 0, SieveArgs* args_out = nullptr) {
+                uint32_t min_gap = 0) {
   LaunchEvents E;
   E.ev0 = c->ev0;
   E.evp = c->evp;
   E.ev1 = c->ev1;
   E.ev2 = c->ev2;
-  return launch_plan_ws(c, c->ws, E, P, want_large, large_cap, emit, s, min_gap, args_out);
+  return launch_plan_ws(c, c->ws, E, P, want_large, large_cap, emit, s, min_gap, nullptr, nullptr, &c->last_kernels);
 }
 
 // memcpy split over host threads: one thread copies from pageable memory at a fraction of the
@@ -639,23 +651,20 @@ int launch_routed(voss_ctx* c, Workspace& W, const LaunchEvents& E, const Interv
     const TileShape shape = choose_shape(c, R.lo.data(), R.hi.data(), (uint32_t)R.lo.size(),
                                          W.gbm_fixed ? W.partials.bytes / sizeof(TilePartial) : 0);
     if ((rc = plan_intervals(c, R.lo.data(), R.hi.data(), (uint32_t)R.lo.size(), 0, shape, &P))) return rc;
-    SieveArgs a;
-    if ((rc = launch_plan_ws(c, W, E, P, false, 0, false, s, 0, &a))) return rc;
-    k = (uint32_t)(&W == &c->ws ? c->last_kernels : 3) + 1;
     const bool identity = R.lo.size() == n;
     if (!identity) {
       if ((rc = W.sh_map.ensure(sizeof(uint32_t) * R.map.size()))) return rc;
       CUDA_TRY(cudaMemcpyAsync(W.sh_map.p, R.map.data(), sizeof(uint32_t) * R.map.size(), cudaMemcpyHostToDevice, s));
     }
-    if (launch_interval_finalize(a, W.out.as<IntervalOut>(), W.istats.as<voss_interval_stats>(),
-                                 identity ? nullptr : W.sh_map.as<uint32_t>(), s))
-      return fail(VOSS_ERR_CUDA, "interval finalize launch failed");
+    if ((rc = launch_plan_ws(c, W, E, P, false, 0, false, s, 0, W.istats.as<voss_interval_stats>(),
+                             identity ? nullptr : W.sh_map.as<uint32_t>(), &k)))
+      return rc;
   } else {
     // no sieve launch: the events bracket the Miller-Rabin path alone
-    if ((rc = W.counters.ensure(sizeof(uint32_t) * kCtrWords))) return rc;
+    if ((rc = W.state.ensure(kCtrBytes))) return rc;
     for (cudaEvent_t e : {E.ev0, E.evp, E.ev1})
       if (e) CUDA_TRY(cudaEventRecord(e, s));
-    CUDA_TRY(cudaMemsetAsync(W.counters.p, 0, sizeof(uint32_t) * kCtrWords, s));
+    CUDA_TRY(cudaMemsetAsync(W.state.p, 0, kCtrBytes, s));
   }
   if (!R.sv.empty()) {
     NvtxRange r("short intervals by Miller-Rabin");
@@ -813,26 +822,24 @@ void finalize_range(const unsigned long long* acc, const IntervalOut& o, uint64_
   }
 }
 
-int fetch_common(voss_ctx* c, uint32_t n_iv, std::vector<unsigned long long>& acc,
-                 std::vector<IntervalOut>& outs, uint32_t* ctr, std::vector<OverflowGap>& over,
-                 bool want_acc) {
+// State of the context's last one-interval launch, and the first of its sorted large gaps, in the
+// context's pinned buffer: one round trip.
+int fetch_state(voss_ctx* c, uint64_t large_cap, const uint32_t** ctr, const IntervalOut** out,
+                const unsigned long long** acc, const voss_large_gap** large) {
   NvtxRange r("fetch statistics");
   cudaStream_t s = c->stream;
-  CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.counters.p, sizeof(uint32_t) * kCtrWords, cudaMemcpyDeviceToHost, s));
-  outs.resize(std::max<uint32_t>(1, n_iv));
-  CUDA_TRY(cudaMemcpyAsync(outs.data(), c->ws.out.p, sizeof(IntervalOut) * n_iv, cudaMemcpyDeviceToHost, s));
-  if (want_acc) {
-    acc.resize((size_t)kAccStride * std::max<uint32_t>(1, n_iv));
-    CUDA_TRY(cudaMemcpyAsync(acc.data(), c->ws.acc.p, sizeof(unsigned long long) * kAccStride * n_iv,
-                             cudaMemcpyDeviceToHost, s));
-  }
+  const size_t bytes = state_bytes(1);
+  char* h = c->h_fetch;
+  CUDA_TRY(cudaMemcpyAsync(h, c->ws.state.p, bytes, cudaMemcpyDeviceToHost, s));
+  const size_t n = std::min<uint64_t>(large_cap, kFetchRecords);
+  if (n)
+    CUDA_TRY(cudaMemcpyAsync(h + bytes, c->ws.ls_sorted.p, sizeof(voss_large_gap) * n, cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));
-  int rc = check_device_error(ctr);
-  if (rc) return rc;
-  const uint32_t no = std::min(ctr[kCtrOver], kOverCap);
-  over.resize(no);
-  if (no) CUDA_TRY(cudaMemcpy(over.data(), c->ws.over.p, sizeof(OverflowGap) * no, cudaMemcpyDeviceToHost));
-  return VOSS_OK;
+  *ctr = reinterpret_cast<const uint32_t*>(h);
+  *out = reinterpret_cast<const IntervalOut*>(h + kCtrBytes);
+  *acc = reinterpret_cast<const unsigned long long*>(h + kCtrBytes + sizeof(IntervalOut));
+  *large = reinterpret_cast<const voss_large_gap*>(h + bytes);
+  return check_device_error(*ctr);
 }
 
 int run_range_device(voss_ctx* c, uint64_t lo, uint64_t hi, uint32_t flags, uint64_t seg_num,
@@ -889,6 +896,11 @@ int stage_large_sorted(voss_ctx* c, uint64_t n, uint64_t hi, voss_large_gap** ou
   NvtxRange r("sort and copy large gaps");
   Workspace& W = c->ws;
   cudaStream_t s = c->stream;
+  if (n <= kSmallSort) {  // sorted behind the launch already
+    CUDA_TRY(cudaMemcpyAsync(c->h_large, W.ls_sorted.p, sizeof(voss_large_gap) * n, cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    return VOSS_OK;
+  }
   const int end_bit = hi > 1 ? 64 - __builtin_clzll(hi - 1) : 1;  // bits in which positions can differ
   const size_t tb = large_sort_temp_bytes((uint32_t)n, end_bit);
   int rc;
@@ -906,25 +918,31 @@ int stage_large_sorted(voss_ctx* c, uint64_t n, uint64_t hi, voss_large_gap** ou
 int fetch_range(voss_ctx* c, voss_range_stats* st, voss_large_gap* large, uint64_t large_cap,
                 uint64_t* written) {
   if (!c->have_range) return fail(VOSS_ERR_STATE, "no range has been sieved on this context");
-  std::vector<unsigned long long> acc;
-  std::vector<IntervalOut> outs;
-  std::vector<OverflowGap> over;
-  uint32_t ctr[kCtrWords];
-  int rc = fetch_common(c, 1, acc, outs, ctr, over, true);
+  const uint32_t* ctr;
+  const IntervalOut* out;
+  const unsigned long long* acc;
+  const voss_large_gap* lg;
+  int rc = fetch_state(c, std::min<uint64_t>(c->r_large_cap, large ? large_cap : 0), &ctr, &out, &acc, &lg);
   if (rc) return rc;
+  std::vector<OverflowGap> over(std::min(ctr[kCtrOver], kOverCap));
+  if (!over.empty())
+    CUDA_TRY(cudaMemcpy(over.data(), c->ws.over.p, sizeof(OverflowGap) * over.size(), cudaMemcpyDeviceToHost));
   cudaEventElapsedTime(&c->sieve_ms, c->ev0, c->ev1);
   cudaEventElapsedTime(&c->total_ms, c->ev0, c->ev2);
   {
     NvtxRange r("finalize statistics");
-    finalize_range(acc.data(), outs[0], c->r_lo, c->r_hi, c->r_flags, c->r_seg, over, st);
+    finalize_range(acc, *out, c->r_lo, c->r_hi, c->r_flags, c->r_seg, over, st);
   }
   const uint64_t found = ctr[kCtrLarge];
   st->large_total = found;
   const uint64_t ondev = std::min<uint64_t>(found, c->r_large_cap);
   const uint64_t w = std::min<uint64_t>(ondev, large ? large_cap : 0);
   if (w) {
-    voss_large_gap* lg = nullptr;
-    if ((rc = stage_large_sorted(c, ondev, c->r_hi, &lg))) return rc;
+    voss_large_gap* staged = nullptr;
+    if (ondev > kFetchRecords) {
+      if ((rc = stage_large_sorted(c, ondev, c->r_hi, &staged))) return rc;
+      lg = staged;
+    }
     std::memcpy(large, lg, sizeof(voss_large_gap) * w);
   }
   if (written) *written = w;
@@ -979,6 +997,10 @@ VOSS_API int voss_ctx_create(int device, uint64_t max_hi, voss_ctx** out) {
       cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
       cudaEventCreate(&c->ev2) != cudaSuccess || cudaEventCreate(&c->evp) != cudaSuccess)
     return bail(fail(VOSS_ERR_CUDA, "stream/event creation failed"));
+  if (cudaMallocHost(&c->h_fetch, kFetchBytes) != cudaSuccess) {
+    c->h_fetch = nullptr;
+    return bail(fail(VOSS_ERR_NOMEM, "cudaMallocHost of the result buffer failed"));
+  }
   c->primes = base_primes(isqrt_u64(max_hi - 1));
   const size_t np = std::max<size_t>(1, c->primes.size());
   int rc;
@@ -1019,6 +1041,7 @@ VOSS_API void voss_ctx_destroy(voss_ctx* c) {
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   if (c->ev_copy) cudaEventDestroy(c->ev_copy);
   if (c->h_large) cudaFreeHost(c->h_large);
+  if (c->h_fetch) cudaFreeHost(c->h_fetch);
   for (int b = 0; b < 2; ++b) {
     if (c->h_stage[b]) cudaFreeHost(c->h_stage[b]);
     if (c->ev_stage[b]) cudaEventDestroy(c->ev_stage[b]);
@@ -1142,20 +1165,23 @@ VOSS_API int voss_sieve_intervals(voss_ctx* c, const uint64_t* lo, const uint64_
   if ((rc = W.istats.ensure(sizeof(voss_interval_stats) * n))) return rc;
   if ((rc = launch_routed(c, W, E, R, n, s, &kernels))) return rc;
   c->last_kernels = kernels;
-  uint32_t ctr[kCtrWords];
-  CUDA_TRY(cudaMemcpyAsync(ctr, W.counters.p, sizeof(ctr), cudaMemcpyDeviceToHost, s));
-  // large results (8 KB per interval) come back through pinned staging, copied out by host threads
-  // (two halves over the two buffers: the second crosses while the first is copied out)
+  // the counters and small results cross through the pinned buffer; large results (8 KB per interval)
+  // through pinned staging, copied out by host threads (two halves over the two buffers: the second
+  // crosses while the first is copied out)
+  CUDA_TRY(cudaMemcpyAsync(c->h_fetch, W.state.p, kCtrBytes, cudaMemcpyDeviceToHost, s));
   const size_t res_bytes = sizeof(voss_interval_stats) * n;
-  const bool staged = res_bytes >= (8u << 20);
-  if (staged) {
+  const bool pinned = res_bytes <= kFetchBytes - kCtrBytes;
+  if (pinned) {
+    CUDA_TRY(cudaMemcpyAsync(c->h_fetch + kCtrBytes, W.istats.p, res_bytes, cudaMemcpyDeviceToHost, s));
+  } else if (res_bytes >= (8u << 20)) {
     if ((rc = ensure_stage(c, (res_bytes + 15) / 16))) return rc;
     if ((rc = stage_out(c, out, W.istats.p, res_bytes, s))) return rc;
   } else {
     CUDA_TRY(cudaMemcpyAsync(out, W.istats.p, res_bytes, cudaMemcpyDeviceToHost, s));
   }
   CUDA_TRY(cudaStreamSynchronize(s));
-  if ((rc = check_device_error(ctr))) return rc;
+  if ((rc = check_device_error(reinterpret_cast<const uint32_t*>(c->h_fetch)))) return rc;
+  if (pinned) std::memcpy(out, c->h_fetch + kCtrBytes, res_bytes);
   cudaEventElapsedTime(&c->sieve_ms, c->ev0, c->ev1);
   cudaEventElapsedTime(&c->total_ms, c->ev0, c->ev2);
   for (uint32_t i = 0; i < n; ++i) add_small_primes(out[i], lo[i], hi[i]);
@@ -1176,17 +1202,21 @@ VOSS_API int voss_gaps_at_least(voss_ctx* c, uint64_t lo, uint64_t hi, uint32_t 
   const uint64_t devcap = std::min<uint64_t>(std::max<uint64_t>(cap, 1), kMaxLargeCap);
   rc = launch_plan(c, P, true, devcap, false, c->stream, min_gap);
   if (rc) return rc;
-  uint32_t ctr[kCtrWords];
-  CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.counters.p, sizeof(ctr), cudaMemcpyDeviceToHost, c->stream));
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
-  if ((rc = check_device_error(ctr))) return rc;
+  const uint32_t* ctr;
+  const IntervalOut* iv_out;
+  const unsigned long long* acc;
+  const voss_large_gap* lg;
+  if ((rc = fetch_state(c, cap ? devcap : 0, &ctr, &iv_out, &acc, &lg))) return rc;
   const uint64_t found = ctr[kCtrLarge];
   *count = found;
-  const uint64_t w = std::min<uint64_t>(std::min<uint64_t>(found, devcap), cap);
+  const uint64_t ondev = std::min<uint64_t>(found, devcap), w = std::min<uint64_t>(ondev, cap);
   if (w) {
-    voss_large_gap* v = nullptr;
-    if ((rc = stage_large_sorted(c, std::min<uint64_t>(found, devcap), hi, &v))) return rc;
-    std::memcpy(out, v, sizeof(voss_large_gap) * w);
+    voss_large_gap* staged = nullptr;
+    if (ondev > kFetchRecords) {
+      if ((rc = stage_large_sorted(c, ondev, hi, &staged))) return rc;
+      lg = staged;
+    }
+    std::memcpy(out, lg, sizeof(voss_large_gap) * w);
   }
   return VOSS_OK;
 }
@@ -1209,7 +1239,7 @@ VOSS_API int voss_primes_range(voss_ctx* c, uint64_t lo, uint64_t hi, uint64_t* 
   if (P.n_tiles)
     CUDA_TRY(cudaMemcpyAsync(parts.data(), c->ws.partials.p, sizeof(TilePartial) * P.n_tiles, cudaMemcpyDeviceToHost, s));
   uint32_t ctr[kCtrWords];
-  CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.counters.p, sizeof(ctr), cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.state.p, sizeof(ctr), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));
   if ((rc = check_device_error(ctr))) return rc;
   std::vector<unsigned long long> offs(std::max<uint32_t>(1, P.n_tiles));
@@ -1234,7 +1264,7 @@ VOSS_API int voss_primes_range(voss_ctx* c, uint64_t lo, uint64_t hi, uint64_t* 
   rc = launch_plan(c, P, false, 0, true, s);
   if (rc) return rc;
   CUDA_TRY(cudaMemcpyAsync(out + k, c->ws.emit.p, sizeof(uint64_t) * room, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.counters.p, sizeof(ctr), cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.state.p, sizeof(ctr), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));
   return check_device_error(ctr);
 }

@@ -34,13 +34,13 @@ int count_tiles(voss_ctx* c, uint64_t lo, uint64_t hi, RunPlan* P, std::vector<u
   int rc = plan_intervals(c, &a, &hi, 1, 0, choose_shape(c, &a, &hi, 1, 0), P);
   if (rc) return rc;
   LaunchEvents E{c->ev0, c->ev1, c->ev2, c->evp};
-  rc = launch_plan_ws(c, c->ws, E, *P, false, 0, false, s, 0, nullptr);
+  rc = launch_plan_ws(c, c->ws, E, *P, false, 0, false, s, 0, nullptr, nullptr, &c->last_kernels);
   if (rc) return rc;
   std::vector<TilePartial> parts(P->n_tiles);
   uint32_t ctr[kCtrWords];
   if (P->n_tiles)
     CUDA_TRY(cudaMemcpyAsync(parts.data(), c->ws.partials.p, sizeof(TilePartial) * P->n_tiles, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.counters.p, sizeof(ctr), cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.state.p, sizeof(ctr), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));
   if ((rc = check_device_error(ctr))) return rc;
   prefix->assign(P->n_tiles + 1, 0);
@@ -75,12 +75,12 @@ int emit_window(voss_ctx* c, const RunPlan& P, const std::vector<uint64_t>& pref
     return rc;
   CUDA_TRY(cudaMemcpyAsync(c->ws.offsets.p, offs.data(), sizeof(unsigned long long) * Q.n_tiles, cudaMemcpyHostToDevice, s));
   LaunchEvents E{c->ev0, c->ev1, c->ev2, c->evp};
-  rc = launch_plan_ws(c, c->ws, E, Q, false, 0, true, s, 0, nullptr);
+  rc = launch_plan_ws(c, c->ws, E, Q, false, 0, true, s, 0, nullptr, nullptr, &c->last_kernels);
   if (rc) return rc;
   out->resize(n);
   uint32_t ctr[kCtrWords];
   CUDA_TRY(cudaMemcpyAsync(out->data(), c->ws.emit.p, sizeof(uint64_t) * n, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.counters.p, sizeof(ctr), cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.state.p, sizeof(ctr), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));
   return check_device_error(ctr);
 }

@@ -63,9 +63,10 @@ struct DevBuf {
 
 // Device memory of one launch of the tile kernel (and of Miller-Rabin batches).
 struct Workspace {
-  DevBuf iv, partials, acc, out, large, large_iv, over, counters, istats, offsets, emit, mr_in, mr_out;
-  DevBuf gbm, scat;  // large-prime pre-pass: bitmap of the launch and its interval descriptors
-  DevBuf tile_iv;    // interval of each tile, for launches of more than one interval
+  DevBuf state;  // counters, IntervalOut and accumulators of a launch (state_of), zeroed and read as one
+  DevBuf desc;   // what a launch copies in: intervals, pre-pass intervals, interval of each tile
+  DevBuf partials, large, large_iv, over, istats, offsets, emit, mr_in, mr_out;
+  DevBuf gbm;    // large-prime bitmap of the launch
   DevBuf pg_pa, pg_gap, pg_ok;  // gap proofs: inputs and verdicts (endpoints use mr_in / mr_out)
   DevBuf sha_data, sha_off, sha_out;  // certificate hashing: messages, offsets, digests
   DevBuf ls_keys, ls_idx, ls_temp, ls_sorted;  // large-gap list sorted by position (large_sort.cu)
@@ -98,6 +99,33 @@ struct RunPlan {
 };
 
 enum { kCtrTile = 0, kCtrLarge = 1, kCtrOver = 2, kCtrError = 3, kCtrWords = 8 };
+
+constexpr size_t kCtrBytes = 64;  // counters at the front of Workspace::state
+// The parts of Workspace::state in a launch of n intervals.
+struct LaunchState {
+  uint32_t* ctr;
+  voss::IntervalOut* out;
+  unsigned long long* acc;
+  size_t bytes;
+};
+inline LaunchState state_of(const Workspace& W, size_t n) {
+  char* p = static_cast<char*>(W.state.p);
+  const size_t acc = kCtrBytes + sizeof(voss::IntervalOut) * n;
+  return LaunchState{reinterpret_cast<uint32_t*>(p), reinterpret_cast<voss::IntervalOut*>(p + kCtrBytes),
+                     reinterpret_cast<unsigned long long*>(p + acc),
+                     acc + sizeof(unsigned long long) * voss::kAccStride * n};
+}
+inline size_t state_bytes(size_t n) {
+  return kCtrBytes + (sizeof(voss::IntervalOut) + sizeof(unsigned long long) * voss::kAccStride) * n;
+}
+// Bytes of Workspace::desc: n intervals, n_scat pre-pass intervals, n_tiles tiles.
+inline size_t desc_bytes(size_t n, size_t n_scat, size_t n_tiles) {
+  return ((sizeof(voss::IntervalDev) * n + 15) & ~(size_t)15) + sizeof(voss::IntervalScatter) * n_scat +
+         sizeof(uint32_t) * n_tiles;
+}
+// Records of the sorted large-gap list that come to the host together with the state.
+constexpr uint32_t kFetchRecords = 4096;
+constexpr size_t kFetchBytes = 128u << 10;  // voss_ctx::h_fetch
 
 constexpr uint64_t kMaxHi = 1ull << 62;
 constexpr uint32_t kOverCap = 1u << 16;
@@ -143,6 +171,8 @@ struct voss_ctx {
   // host side of the large-gap list: pinned, grow-only staging for the device-to-host copy of
   // the list (sorted on the device), so that repeated calls touch no fresh pages
   voss_large_gap* h_large = nullptr;
+  // pinned: the state of a one-interval launch and the first kFetchRecords large gaps, or a small result
+  char* h_fetch = nullptr;
   size_t h_large_cap = 0;
   // pinned staging of large host batches (Miller-Rabin candidates in, verdicts out): two
   // buffers, one filled by host threads while the other crosses; ev_stage[b] marks the end of
@@ -166,10 +196,11 @@ TileShape choose_shape(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi
 // Cut intervals [lo_i, hi_i) into tiles; intervals without wheel integers get no tiles.
 int plan_intervals(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, uint32_t n, uint64_t seg_k,
                    const TileShape& shape, RunPlan* P);
-// Queue the tile kernel (+ stitch and reduce unless emit) for plan P on stream s, using the
-// workspace W and events E.
+// Queue plan P on stream s, using the workspace W and events E: the tile kernel, and unless emit the
+// tail (with `stats`: of interval statistics at stats[out_index[i]]).  *kernels: how many ran.
 int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPlan& P, bool want_large,
-                   uint64_t large_cap, bool emit, cudaStream_t s, uint32_t min_gap, voss::SieveArgs* args_out);
+                   uint64_t large_cap, bool emit, cudaStream_t s, uint32_t min_gap, voss_interval_stats* stats,
+                   const uint32_t* out_index, uint32_t* kernels);
 // A batch of intervals split between the sieve (lo, hi, map = their positions in the batch)
 // and the Miller-Rabin path for short intervals at high starts (sv, n_cand candidates).
 struct IntervalRoute {

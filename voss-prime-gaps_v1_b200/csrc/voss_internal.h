@@ -199,14 +199,16 @@ struct LaunchShape {
 size_t sieve_smem_bytes(uint32_t tile_words);
 int launch_sieve_stats(const SieveArgs& a, int grid, int block, size_t smem, void* stream);
 int launch_sieve_emit(const SieveArgs& a, int grid, int block, size_t smem, void* stream);
-int launch_stitch(const SieveArgs& a, void* stream);
-int launch_reduce(const SieveArgs& a, IntervalOut* out, void* stream);
+// Zero `zero_bytes` (a multiple of 16) at `zero` and set n_ones words at `ones` (16-byte aligned).
+int launch_init(void* zero, size_t zero_bytes, uint32_t* ones, size_t n_ones, int sm_count, void* stream);
 }  // namespace voss
 struct voss_interval_stats;
 namespace voss {
-// out_index (nullptr: identity) gives each launch interval's position in `out`.
-int launch_interval_finalize(const SieveArgs& a, const IntervalOut* io, voss_interval_stats* out,
-                             const uint32_t* out_index, void* stream);
+// Seams, first/last prime and maximal gap of every interval (of at most max_tiles tiles each) into
+// `out`, and the interval statistics into `stats` (nullptr: not wanted); out_index (nullptr:
+// identity) gives each launch interval's position in `stats`.  Adds the kernels launched.
+int launch_tail(const SieveArgs& a, uint32_t max_tiles, IntervalOut* out, voss_interval_stats* stats,
+                const uint32_t* out_index, void* stream, uint32_t* kernels);
 // Short intervals by Miller-Rabin (short_iv.cu): candidates into d_cand (n_cand), verdicts into
 // d_ok, results at d_out[out_index].
 int launch_short_intervals(const ShortInterval* d_iv, uint32_t n_iv, uint32_t n_seg, uint64_t n_cand,
@@ -216,6 +218,10 @@ int launch_scatter_large(const uint32_t* primes, const uint64_t* magic, uint32_t
                          const IntervalScatter* iv, uint32_t n_iv, uint32_t* gbm, int sm_count, void* stream);
 int sieve_kernel_attrs(int block, size_t smem, int* max_ctas_per_sm);
 // Large-gap list sorted by position on the device (large_sort.cu): keys and idx hold 2n entries.
+constexpr uint32_t kSmallSort = 16384;
+// Sorts min(*count, cap) records when they are at most kSmallSort (else does nothing).
+int launch_large_sort_small(const LargeGapDev* in, const uint32_t* count, uint32_t cap, LargeGapDev* out,
+                            void* stream);
 size_t large_sort_temp_bytes(uint32_t n, int end_bit);
 int launch_large_sort(const LargeGapDev* in, uint32_t n, int end_bit, unsigned long long* keys, uint32_t* idx,
                       void* temp, size_t temp_bytes, LargeGapDev* out, int sm_count, void* stream);

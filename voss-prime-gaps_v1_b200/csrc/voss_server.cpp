@@ -28,8 +28,6 @@
 #include "voss_host.h"
 
 using namespace voss_host;
-using voss::IntervalOut;
-using voss::SieveArgs;
 
 namespace {
 
@@ -145,7 +143,7 @@ int launch_batch(voss_server* S, Slot& sl) {
     if (rc) return rc;
     CUDA_TRY(cudaMemcpyAsync(sl.h_istats, sl.ws.istats.p, sizeof(voss_interval_stats) * sl.n_iv,
                              cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaMemcpyAsync(sl.h_ctr, sl.ws.counters.p, sizeof(uint32_t) * kCtrWords, cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaMemcpyAsync(sl.h_ctr, sl.ws.state.p, sizeof(uint32_t) * kCtrWords, cudaMemcpyDeviceToHost, s));
     S->launches += kernels;
   } else {
     std::memset(sl.h_ctr, 0, sizeof(uint32_t) * kCtrWords);
@@ -301,10 +299,8 @@ Slot* make_slot(voss_server* S, int* rc) {
     return bad(fail(VOSS_ERR_CUDA, "server slot stream/event creation failed"));
   Workspace& W = sl->ws;
   int e;
-  if ((e = W.iv.ensure(sizeof(voss::IntervalDev) * nreq)) || (e = W.partials.ensure(sizeof(voss::TilePartial) * C.max_batch_tiles)) ||
-      (e = W.tile_iv.ensure(sizeof(uint32_t) * C.max_batch_tiles)) ||
-      (e = W.acc.ensure(sizeof(unsigned long long) * voss::kAccStride * nreq)) ||
-      (e = W.out.ensure(sizeof(IntervalOut) * nreq)) || (e = W.counters.ensure(sizeof(uint32_t) * kCtrWords)) ||
+  if ((e = W.partials.ensure(sizeof(voss::TilePartial) * C.max_batch_tiles)) || (e = W.state.ensure(state_bytes(nreq))) ||
+      (e = W.desc.ensure(desc_bytes(nreq, nreq + C.max_batch_bitmap_bytes / kScatterWindowBytes + 1, C.max_batch_tiles))) ||
       (e = W.over.ensure(sizeof(voss::OverflowGap) * kOverCap)) || (e = W.large.ensure(sizeof(voss::LargeGapDev))) ||
       (e = W.large_iv.ensure(sizeof(uint32_t))) || (e = W.istats.ensure(sizeof(voss_interval_stats) * nreq)) ||
       (e = W.mr_in.ensure(8 * (C.max_batch_candidates + 1))) || (e = W.mr_out.ensure(C.max_batch_candidates + 1)))
@@ -312,8 +308,7 @@ Slot* make_slot(voss_server* S, int* rc) {
   // the large-prime pre-pass bitmap: fixed size, never grown while serving
   W.gbm_budget = C.max_batch_bitmap_bytes;
   W.gbm_fixed = true;
-  if (W.gbm_budget && ((e = W.gbm.ensure(W.gbm_budget)) || (e = W.scat.ensure(sizeof(voss::IntervalScatter) * (nreq + W.gbm_budget / kScatterWindowBytes + 1)))))
-    return bad(e);
+  if (W.gbm_budget && (e = W.gbm.ensure(W.gbm_budget))) return bad(e);
   if ((e = W.sh_iv.ensure(sizeof(voss::ShortInterval) * nreq)) || (e = W.sh_map.ensure(sizeof(uint32_t) * nreq)) ||
       (e = W.sh_seg.ensure(sizeof(voss::ShortSegment) * (C.max_batch_candidates / voss::kShortSeg + nreq + 1))))
     return bad(e);
