@@ -15,6 +15,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <exception>
+#include <memory>
 #include <string>
 #include <thread>
 #include <vector>
@@ -526,6 +527,68 @@ void parallel_gather(void* dst, const CopySeg* seg, size_t n_seg, size_t min_par
   for (auto& t : th) t.join();
 }
 
+CopyTeam::CopyTeam(size_t total_bytes) {
+  const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+  const size_t parts = std::min<size_t>(std::min(hw, 8u), total_bytes / kStagePart + 1);
+  for (size_t i = 1; i < parts; ++i) {
+    try {
+      th_.emplace_back([this, i] { work(i); });
+    } catch (const std::exception&) {
+      break;  // the copies are split over those that started
+    }
+  }
+}
+
+CopyTeam::~CopyTeam() {
+  stop_ = true;
+  post();
+  for (auto& t : th_) t.join();
+}
+
+void CopyTeam::post() {
+  {
+    std::lock_guard<std::mutex> lk(mu_);
+    job_.fetch_add(1, std::memory_order_release);
+  }
+  cv_.notify_all();
+}
+
+void CopyTeam::copy_part(size_t i) const {
+  const size_t step = ((bytes_ / (th_.size() + 1)) + 64) & ~(size_t)63;
+  const size_t a = std::min(bytes_, i * step), b = std::min(bytes_, a + step);
+  if (a < b) std::memcpy((char*)dst_ + a, (const char*)src_ + a, b - a);
+}
+
+void CopyTeam::work(size_t i) {
+  uint64_t seen = 0;
+  for (;;) {
+    // the next copy of a pipelined transfer comes within a fraction of a millisecond
+    for (int k = 0; k < 2000 && job_.load(std::memory_order_acquire) == seen; ++k) std::this_thread::yield();
+    if (job_.load(std::memory_order_acquire) == seen) {
+      std::unique_lock<std::mutex> lk(mu_);
+      cv_.wait(lk, [&] { return job_.load(std::memory_order_acquire) != seen; });
+    }
+    seen = job_.load(std::memory_order_acquire);
+    if (stop_) return;
+    copy_part(i);
+    left_.fetch_sub(1, std::memory_order_release);
+  }
+}
+
+void CopyTeam::copy(void* dst, const void* src, size_t bytes) {
+  if (th_.empty() || bytes < kStagePart / 4) {
+    std::memcpy(dst, src, bytes);
+    return;
+  }
+  dst_ = dst;
+  src_ = src;
+  bytes_ = bytes;
+  left_.store(th_.size(), std::memory_order_relaxed);
+  post();
+  copy_part(0);
+  while (left_.load(std::memory_order_acquire)) std::this_thread::yield();
+}
+
 // The context's two pinned staging buffers, ready for host writes: every transfer that may
 // still use them (left queued by an earlier call that returned early) has finished.  They hold
 // min(entries, stage_limit) 64-bit words each (grow-only); callers move data in chunks of
@@ -553,14 +616,14 @@ int ensure_stage(voss_ctx* c, size_t entries) {
 // Host -> device through the staging buffers on stream s: chunk i is filled by host threads
 // into buffer i & 1 once that buffer's previous transfer is done, then crosses while chunk
 // i + 1 is filled.  Returns once the last chunk is queued.
-int stage_in(voss_ctx* c, void* d_dst, const void* src, size_t bytes, cudaStream_t s) {
-  const size_t chunk = c->h_stage_cap * sizeof(uint64_t);
+int stage_in(voss_ctx* c, void* d_dst, const void* src, size_t bytes, cudaStream_t s, CopyTeam& team) {
+  const size_t chunk = std::min(c->h_stage_cap * sizeof(uint64_t), kStageChunk);
   size_t i = 0;
   for (size_t off = 0; off < bytes; off += chunk, ++i) {
     const size_t k = std::min(chunk, bytes - off);
     const int b = (int)(i & 1);
     CUDA_TRY(cudaEventSynchronize(c->ev_stage[b]));
-    parallel_copy(c->h_stage[b], (const char*)src + off, k);
+    team.copy(c->h_stage[b], (const char*)src + off, k);
     CUDA_TRY(cudaMemcpyAsync((char*)d_dst + off, c->h_stage[b], k, cudaMemcpyHostToDevice, s));
     CUDA_TRY(cudaEventRecord(c->ev_stage[b], s));
   }
@@ -569,8 +632,8 @@ int stage_in(voss_ctx* c, void* d_dst, const void* src, size_t bytes, cudaStream
 
 // Device -> host through the staging buffers, after the work queued on s: chunk j crosses into
 // buffer j & 1 while host threads copy chunk j - 1 out.  Returns with every byte in dst.
-int stage_out(voss_ctx* c, void* dst, const void* d_src, size_t bytes, cudaStream_t s) {
-  const size_t chunk = c->h_stage_cap * sizeof(uint64_t);
+int stage_out(voss_ctx* c, void* dst, const void* d_src, size_t bytes, cudaStream_t s, CopyTeam& team) {
+  const size_t chunk = std::min(c->h_stage_cap * sizeof(uint64_t), kStageChunk);
   size_t prev_off = 0, prev_k = 0, j = 0;
   for (size_t off = 0; off < bytes; off += chunk, ++j) {
     const size_t k = std::min(chunk, bytes - off);
@@ -580,14 +643,14 @@ int stage_out(voss_ctx* c, void* dst, const void* d_src, size_t bytes, cudaStrea
     CUDA_TRY(cudaEventRecord(c->ev_stage[b], s));
     if (j > 0) {
       CUDA_TRY(cudaEventSynchronize(c->ev_stage[b ^ 1]));
-      parallel_copy((char*)dst + prev_off, c->h_stage[b ^ 1], prev_k);
+      team.copy((char*)dst + prev_off, c->h_stage[b ^ 1], prev_k);
     }
     prev_off = off;
     prev_k = k;
   }
   if (j > 0) {
     CUDA_TRY(cudaEventSynchronize(c->ev_stage[(j - 1) & 1]));
-    parallel_copy((char*)dst + prev_off, c->h_stage[(j - 1) & 1], prev_k);
+    team.copy((char*)dst + prev_off, c->h_stage[(j - 1) & 1], prev_k);
   }
   return VOSS_OK;
 }
@@ -991,7 +1054,8 @@ VOSS_API int voss_ctx_create(int device, uint64_t max_hi, voss_ctx** out) {
   c->sm_count = prop.multiProcessorCount;
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&c->ev_copy, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_out[0], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_out[1], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_stage[0], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_stage[1], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
@@ -1039,12 +1103,12 @@ VOSS_API void voss_ctx_destroy(voss_ctx* c) {
   if (c->evp) cudaEventDestroy(c->evp);
   if (c->stream) cudaStreamDestroy(c->stream);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
-  if (c->ev_copy) cudaEventDestroy(c->ev_copy);
   if (c->h_large) cudaFreeHost(c->h_large);
   if (c->h_fetch) cudaFreeHost(c->h_fetch);
   for (int b = 0; b < 2; ++b) {
     if (c->h_stage[b]) cudaFreeHost(c->h_stage[b]);
     if (c->ev_stage[b]) cudaEventDestroy(c->ev_stage[b]);
+    if (c->ev_out[b]) cudaEventDestroy(c->ev_out[b]);
   }
   delete c;
 }
@@ -1166,16 +1230,15 @@ VOSS_API int voss_sieve_intervals(voss_ctx* c, const uint64_t* lo, const uint64_
   if ((rc = launch_routed(c, W, E, R, n, s, &kernels))) return rc;
   c->last_kernels = kernels;
   // the counters and small results cross through the pinned buffer; large results (8 KB per interval)
-  // through pinned staging, copied out by host threads (two halves over the two buffers: the second
-  // crosses while the first is copied out)
+  // through pinned staging, one chunk crossing while host threads copy the one before it out
   CUDA_TRY(cudaMemcpyAsync(c->h_fetch, W.state.p, kCtrBytes, cudaMemcpyDeviceToHost, s));
   const size_t res_bytes = sizeof(voss_interval_stats) * n;
   const bool pinned = res_bytes <= kFetchBytes - kCtrBytes;
   if (pinned) {
     CUDA_TRY(cudaMemcpyAsync(c->h_fetch + kCtrBytes, W.istats.p, res_bytes, cudaMemcpyDeviceToHost, s));
   } else if (res_bytes >= (8u << 20)) {
-    if ((rc = ensure_stage(c, (res_bytes + 15) / 16))) return rc;
-    if ((rc = stage_out(c, out, W.istats.p, res_bytes, s))) return rc;
+    CopyTeam team(res_bytes);
+    if ((rc = ensure_stage(c, kStageChunk / 8)) || (rc = stage_out(c, out, W.istats.p, res_bytes, s, team))) return rc;
   } else {
     CUDA_TRY(cudaMemcpyAsync(out, W.istats.p, res_bytes, cudaMemcpyDeviceToHost, s));
   }
@@ -1263,8 +1326,15 @@ VOSS_API int voss_primes_range(voss_ctx* c, uint64_t lo, uint64_t hi, uint64_t* 
   // pass 2: write (out_cap is the buffer size, which may exceed `room`)
   rc = launch_plan(c, P, false, 0, true, s);
   if (rc) return rc;
-  CUDA_TRY(cudaMemcpyAsync(out + k, c->ws.emit.p, sizeof(uint64_t) * room, cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaMemcpyAsync(ctr, c->ws.state.p, sizeof(ctr), cudaMemcpyDeviceToHost, s));
+  if (room * sizeof(uint64_t) >= kStageChunk) {  // long lists through pinned staging, copied out by host threads
+    CopyTeam team(room * sizeof(uint64_t));
+    if ((rc = ensure_stage(c, kStageChunk / 8)) ||
+        (rc = stage_out(c, out + k, c->ws.emit.p, room * sizeof(uint64_t), s, team)))
+      return rc;
+  } else {
+    CUDA_TRY(cudaMemcpyAsync(out + k, c->ws.emit.p, sizeof(uint64_t) * room, cudaMemcpyDeviceToHost, s));
+  }
   CUDA_TRY(cudaStreamSynchronize(s));
   return check_device_error(ctr);
 }
@@ -1292,43 +1362,49 @@ VOSS_API int voss_mr_verify(voss_ctx* c, const uint64_t* n, uint64_t count, uint
   cudaStream_t s = c->stream;
   Workspace& W = c->ws;
   int rc;
-  // context-owned, grow-only buffers: repeated calls do not allocate.  The candidates cross in
-  // chunks on the copy stream while the previous chunk is tested on `stream`.  Large batches go
-  // through two pinned staging buffers that host threads fill (chunk i + 1 is copied in while
-  // chunk i crosses and chunk i - 1 is tested), and the verdicts come back the same way; small
-  // ones are copied straight from the caller's memory.
-  const bool staged = count >= (1ull << 20);
-  if (staged && (rc = ensure_stage(c, std::min<uint64_t>(count, 1ull << 24)))) return rc;
-  const uint64_t kChunk = staged ? c->h_stage_cap : (1ull << 24);  // candidates per launch
+  // context-owned, grow-only buffers: repeated calls do not allocate.  Small batches are copied
+  // straight from and to the caller's memory; large ones go through the two pinned staging buffers
+  // chunk by chunk: while chunk i is filled in by host threads, chunk i - 1 crosses on the copy
+  // stream and is tested on `stream`, and the verdicts of chunk i - 2 are copied out.
   if ((rc = W.mr_in.ensure(count * 8)) || (rc = W.mr_out.ensure(count))) return rc;
   uint64_t* d_in = W.mr_in.as<uint64_t>();
   uint8_t* d_out = W.mr_out.as<uint8_t>();
-  uint64_t i = 0;
-  for (uint64_t off = 0; off < count; off += kChunk, ++i) {
-    const uint64_t k = std::min(kChunk, count - off);
-    if (staged) {
-      const int b = (int)(i & 1);
-      CUDA_TRY(cudaEventSynchronize(c->ev_stage[b]));  // buffer b's previous transfer is done
-      parallel_copy(c->h_stage[b], n + off, k * 8);
-      CUDA_TRY(cudaMemcpyAsync(d_in + off, c->h_stage[b], k * 8, cudaMemcpyHostToDevice, c->copy_stream));
-      CUDA_TRY(cudaEventRecord(c->ev_stage[b], c->copy_stream));
-    } else {
-      CUDA_TRY(cudaMemcpyAsync(d_in + off, n + off, k * 8, cudaMemcpyHostToDevice, c->copy_stream));
-    }
-    CUDA_TRY(cudaEventRecord(c->ev_copy, c->copy_stream));
-    CUDA_TRY(cudaStreamWaitEvent(s, c->ev_copy, 0));
-    if (launch_mr(d_in + off, k, d_out + off, s, c->sm_count))
+  if (count < (1ull << 20)) {
+    CUDA_TRY(cudaMemcpyAsync(d_in, n, count * 8, cudaMemcpyHostToDevice, s));
+    if (launch_mr(d_in, count, d_out, s, c->sm_count))
       return fail(VOSS_ERR_CUDA, "Miller-Rabin launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-  }
-  if (!staged) {
     CUDA_TRY(cudaMemcpyAsync(is_prime, d_out, count, cudaMemcpyDeviceToHost, s));
     CUDA_TRY(cudaStreamSynchronize(s));
     return VOSS_OK;
   }
-  // verdicts: chunk j crosses into buffer j & 1 while chunk j - 1 is copied out by host threads
-  // (the input transfers are complete: every launch on `stream` waited for them)
-  if ((rc = stage_out(c, is_prime, d_out, count, s))) return rc;
-  CUDA_TRY(cudaStreamSynchronize(s));
+  CopyTeam team(count * 8);
+  // a buffer holds a chunk's candidates and, behind them, its verdicts
+  if ((rc = ensure_stage(c, kMrChunk + kMrChunk / 8))) return rc;
+  const uint64_t chunk = std::min<uint64_t>(kMrChunk, c->h_stage_cap * 8 / 9);
+  const uint64_t n_chunks = (count + chunk - 1) / chunk;
+  auto verdicts = [&](uint64_t i) { return reinterpret_cast<uint8_t*>(c->h_stage[i & 1] + chunk); };
+  auto collect = [&](uint64_t i) {  // copy chunk i's verdicts out
+    const uint64_t off = i * chunk, k = std::min(chunk, count - off);
+    CUDA_TRY(cudaEventSynchronize(c->ev_out[i & 1]));
+    team.copy(is_prime + off, verdicts(i), k);
+    return (int)VOSS_OK;
+  };
+  for (uint64_t i = 0; i < n_chunks; ++i) {
+    const uint64_t off = i * chunk, k = std::min(chunk, count - off);
+    const int b = (int)(i & 1);
+    // the buffer's previous chunk has been tested (its verdicts crossed behind it) and copied out
+    if (i >= 2 && (rc = collect(i - 2))) return rc;
+    team.copy(c->h_stage[b], n + off, k * 8);
+    CUDA_TRY(cudaMemcpyAsync(d_in + off, c->h_stage[b], k * 8, cudaMemcpyHostToDevice, c->copy_stream));
+    CUDA_TRY(cudaEventRecord(c->ev_stage[b], c->copy_stream));
+    CUDA_TRY(cudaStreamWaitEvent(s, c->ev_stage[b], 0));
+    if (launch_mr(d_in + off, k, d_out + off, s, c->sm_count))
+      return fail(VOSS_ERR_CUDA, "Miller-Rabin launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+    CUDA_TRY(cudaMemcpyAsync(verdicts(i), d_out + off, k, cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaEventRecord(c->ev_out[b], s));
+  }
+  for (uint64_t i = n_chunks >= 2 ? n_chunks - 2 : 0; i < n_chunks; ++i)
+    if ((rc = collect(i))) return rc;
   return VOSS_OK;
 }
 
@@ -1348,9 +1424,11 @@ VOSS_API int voss_prove_gaps(voss_ctx* c, const uint64_t* p_after, const int32_t
     return rc;
   // large batches cross through the pinned staging buffers (filled and emptied by host threads)
   const bool staged = count >= (1ull << 20);
+  std::unique_ptr<CopyTeam> team;
   if (staged) {
-    if ((rc = ensure_stage(c, (count + 1) / 2)) || (rc = stage_in(c, W.pg_pa.p, p_after, count * 8, s)) ||
-        (rc = stage_in(c, W.pg_gap.p, gap, count * 4, s)))
+    team = std::make_unique<CopyTeam>(count * 12);
+    if ((rc = ensure_stage(c, kStageChunk / 8)) || (rc = stage_in(c, W.pg_pa.p, p_after, count * 8, s, *team)) ||
+        (rc = stage_in(c, W.pg_gap.p, gap, count * 4, s, *team)))
       return rc;
   } else {
     CUDA_TRY(cudaMemcpyAsync(W.pg_pa.p, p_after, count * 8, cudaMemcpyHostToDevice, s));
@@ -1360,7 +1438,7 @@ VOSS_API int voss_prove_gaps(voss_ctx* c, const uint64_t* p_after, const int32_t
                         W.mr_in.as<uint64_t>(), W.mr_out.as<uint8_t>(), s, c->sm_count))
     return fail(VOSS_ERR_CUDA, "gap proof launch failed");
   if (staged) {
-    if ((rc = stage_out(c, ok, W.pg_ok.p, count, s))) return rc;
+    if ((rc = stage_out(c, ok, W.pg_ok.p, count, s, *team))) return rc;
   } else {
     CUDA_TRY(cudaMemcpyAsync(ok, W.pg_ok.p, count, cudaMemcpyDeviceToHost, s));
   }

@@ -5,7 +5,11 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <atomic>
+#include <condition_variable>
 #include <cstdint>
+#include <mutex>
+#include <thread>
 #include <vector>
 
 #include "voss.h"
@@ -139,6 +143,13 @@ constexpr uint64_t kDefaultLargeCap = 1ull << 22;
 #endif
 constexpr uint64_t kScatterWindowBytes = (uint64_t)VOSS_SCATTER_WINDOW_MB << 20;
 constexpr uint64_t kScatterWindowWords = kScatterWindowBytes / 4;
+// Large host transfers: bytes per chunk through a pinned buffer, bytes per copying host thread at
+// least, and Miller-Rabin candidates per chunk.  10^7 candidates take 3.5 ms per call at 2^20 per
+// chunk, 4.2 at 2^19 and 4.2 at 2^21 (6.3 ms in one chunk); 6*10^6 primes (48 MB) 3.7 ms in 8 MB
+// chunks, 4.9 in 4 MB, 3.7 in 16 MB (11.5 ms straight to pageable memory).
+constexpr size_t kStageChunk = 8u << 20;
+constexpr size_t kStagePart = 1u << 20;
+constexpr uint64_t kMrChunk = 1ull << 20;
 constexpr uint64_t kMaxLargeCap = 50000000ull;  // MAX_LARGE_GAPS, src/voss_v7_live.cu:34
 
 }  // namespace voss_host
@@ -148,7 +159,6 @@ struct voss_ctx {
   int sm_count = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;  // host-to-device copies overlapped with work on `stream`
-  cudaEvent_t ev_copy = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, evp = nullptr;
   uint64_t max_hi = 0;
   std::vector<uint32_t> primes;  // >= 37
@@ -180,6 +190,7 @@ struct voss_ctx {
   uint64_t* h_stage[2] = {nullptr, nullptr};
   size_t h_stage_cap = 0;  // 64-bit entries per buffer
   cudaEvent_t ev_stage[2] = {nullptr, nullptr};
+  cudaEvent_t ev_out[2] = {nullptr, nullptr};  // a Miller-Rabin chunk's verdicts are in buffer b
   // most 64-bit entries a staging buffer may hold (larger transfers cross in chunks); the
   // environment variable VOSS_STAGE_LIMIT lowers it when the context is created, so tests can
   // drive the chunked paths with small batches
@@ -220,6 +231,30 @@ int launch_routed(voss_ctx* c, Workspace& W, const LaunchEvents& E, const Interv
 int check_device_error(const uint32_t* ctr_host);
 // memcpy split over up to 8 host threads, in parts of at least min_part bytes.
 void parallel_copy(void* dst, const void* src, size_t bytes, size_t min_part = 8u << 20);
+// Up to 8 host threads that copy together for the duration of one call: a chunked transfer starts
+// them once (a thread costs tens of microseconds) and hands them each chunk.
+class CopyTeam {
+ public:
+  explicit CopyTeam(size_t total_bytes);  // a thread per kStagePart bytes at most
+  ~CopyTeam();
+  CopyTeam(const CopyTeam&) = delete;
+  CopyTeam& operator=(const CopyTeam&) = delete;
+  void copy(void* dst, const void* src, size_t bytes);  // memcpy, returns when all of it is done
+
+ private:
+  void work(size_t i);
+  void copy_part(size_t i) const;
+  void post();
+  std::vector<std::thread> th_;
+  std::mutex mu_;
+  std::condition_variable cv_;
+  std::atomic<uint64_t> job_{0};
+  std::atomic<size_t> left_{0};
+  bool stop_ = false;  // written before the last post()
+  void* dst_ = nullptr;
+  const void* src_ = nullptr;
+  size_t bytes_ = 0;
+};
 struct CopySeg {
   const void* src;
   size_t bytes;
