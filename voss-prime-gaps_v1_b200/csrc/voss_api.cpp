@@ -375,13 +375,12 @@ int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPl
         }
         IntervalScatter I;
         I.vbase = 30ull * (d.k0 + 4ull * w0);
-        I.span = 120ull * nw;
         I.gword = d.gword + w0;
-        I.sqrt_hi = (uint32_t)std::min<uint64_t>(isqrt_u64(std::min(d.hi, I.vbase + I.span) - 1), 0xFFFFFFFFull);
+        I.sqrt_hi = (uint32_t)std::min<uint64_t>(isqrt_u64(std::min<uint64_t>(d.hi, I.vbase + 120ull * nw) - 1), 0xFFFFFFFFull);
         I.vbase_d = (double)I.vbase;
         I.vbase_lo = (uint32_t)I.vbase;
-        I.span32 = (uint32_t)std::min<uint64_t>(I.span, 0xFFFFFFFFull);
-        I.lt32 = I.span / 30 < (1ull << 31) ? (uint32_t)(I.span / 30) : 0u;
+        I.span32 = (uint32_t)(120ull * nw);
+        I.lt32 = (uint32_t)(4ull * nw);
         sc.push_back(I);
         wbytes += 4ull * nw;
         wins.back().n++;
@@ -429,9 +428,8 @@ int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPl
     CUDA_TRY(cudaMemsetAsync(W.state.p, 0, zero_bytes, s));
   }
   for (const Window& w : wins) {
-    if (launch_scatter_large(a.primes, a.magic, j0, w.j1, d_scat + w.off, w.n, W.gbm.as<uint32_t>(), c->sm_count, s))
+    if (launch_scatter_large(a.primes, j0, w.j1, d_scat + w.off, w.n, W.gbm.as<uint32_t>(), c->sm_count, s, &k))
       return fail(VOSS_ERR_CUDA, "large-prime pre-pass launch failed");
-    ++k;
   }
   if (E.evp) CUDA_TRY(cudaEventRecord(E.evp, s));
   if (P.n_tiles) {

@@ -88,11 +88,10 @@ struct __align__(16) IntervalScatter {
   // Read for every (prime, interval) pair: 16 B
   double vbase_d;     // vbase rounded to double (for the quotient estimate of vbase mod p)
   uint32_t vbase_lo;  // low 32 bits of vbase (the remainder needs only those, see scatter_large_kernel)
-  uint32_t span32;    // min(span, 2^32 - 1)
+  uint32_t span32;    // integers covered by the interval's words (120 per word): at most a window's
   // read once per prime (how many intervals it reaches) or when a multiple of p may lie inside
   uint32_t sqrt_hi;   // isqrt(hi - 1), capped to 2^32 - 1
-  uint32_t lt32;      // bytes of the interval's bitmap (span / 30) when below 2^31, else 0
-  uint64_t span;      // integers covered by the interval's words (120 per word)
+  uint32_t lt32;      // bytes of the interval's bitmap (span / 30)
   uint64_t gword;     // first word in the large-prime bitmap
   uint64_t vbase;     // for primes >= 2^30 (hi above 2^60)
 };
@@ -214,8 +213,8 @@ int launch_tail(const SieveArgs& a, uint32_t max_tiles, IntervalOut* out, voss_i
 int launch_short_intervals(const ShortInterval* d_iv, uint32_t n_iv, uint32_t n_seg, uint64_t n_cand,
                            uint64_t* d_cand, uint8_t* d_ok, ShortSegment* d_seg, voss_interval_stats* d_out,
                            int sm_count, void* stream);
-int launch_scatter_large(const uint32_t* primes, const uint64_t* magic, uint32_t j0, uint32_t j1,
-                         const IntervalScatter* iv, uint32_t n_iv, uint32_t* gbm, int sm_count, void* stream);
+int launch_scatter_large(const uint32_t* primes, uint32_t j0, uint32_t j1, const IntervalScatter* iv, uint32_t n_iv,
+                         uint32_t* gbm, int sm_count, void* stream, uint32_t* kernels);
 int sieve_kernel_attrs(int block, size_t smem, int* max_ctas_per_sm);
 // Large-gap list sorted by position on the device (large_sort.cu): keys and idx hold 2n entries.
 constexpr uint32_t kSmallSort = 16384;
