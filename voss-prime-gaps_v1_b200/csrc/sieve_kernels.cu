@@ -195,7 +195,7 @@ __device__ __forceinline__ uint32_t find_interval(const SieveArgs& a, uint32_t t
 // instructions per clear (11.8 instructions against 6 for the hits of clear_class_primes).
 struct TileBits {
   uint32_t* bm;
-  uint32_t spare;  // byte offset of the lane's word behind the tile (kSpareWords follow every tile)
+  uint32_t spare;  // byte offset of the lane's first word behind the tile (kSpareWords follow every tile)
   uint32_t nw;     // words of this tile
   uint32_t* err;
 
@@ -203,15 +203,15 @@ struct TileBits {
     VOSS_SM_GUARD(off >> 2, nw + kSpareWords)
     atomicAnd(reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(bm) + off), mask);
   }
-  // the same, or a word behind the tile when off >= 4 nw (an offset below zero is a large unsigned)
-  __device__ __forceinline__ void clear_word_or_spare(uint32_t off, uint32_t mask) const {
-    clear(min(off, spare), mask);
+  // Byte offset of byte x's word, or of the lane's k-th spare word (k < kSpareRows) when x >= 4 nw (an x
+  // below zero is a large unsigned).  Clears that follow each other take different spare words: on one
+  // word a warp's atomics in close succession serialise (the small primes' starts and ends, unrolled
+  // by four, took 61k wavefronts per tile instead of 47k).
+  __device__ __forceinline__ uint32_t word_or_spare(uint32_t x, int k) const {
+    return __viaddmin_u32(spare, 128u * (uint32_t)k, x) & ~3u;
   }
-  // bit x of the tile, or some bit of a spare word when x >= 32 nw
-  __device__ __forceinline__ void clear_bit_or_spare(uint32_t x) const {
-    const uint32_t word = min(x, 8u * spare) >> 5;
-    VOSS_SM_GUARD(word, nw + kSpareWords)
-    atomicAnd(bm + word, __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, x));
+  __device__ __forceinline__ void clear_word_or_spare(uint32_t off, uint32_t mask, int k) const {
+    clear(__viaddmin_u32(spare, 128u * (uint32_t)k, off), mask);
   }
 };
 
@@ -267,13 +267,21 @@ __device__ __forceinline__ void clear_small_prime(const TileBits& T, uint32_t re
   const int x_out = __reduce_min_sync(kFull, left);    // up to here none has finished,
   const int x_end = __reduce_max_sync(kFull, left);    // and here all have
   int x = 0;
-  for (; x < x_in; x += step, w += (uint32_t)step) T.clear_word_or_spare(w, mask);
+#pragma unroll 1
+  for (; x < x_in; x += 4 * step) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j, w += (uint32_t)step) T.clear_word_or_spare(w, mask, j);
+  }
 #pragma unroll 1
   for (const int x_8 = x_out - 7 * step; x < x_8; x += 8 * step) {
 #pragma unroll
     for (int j = 0; j < 8; ++j, w += (uint32_t)step) T.clear(w, mask);
   }
-  for (; x < x_end; x += step, w += (uint32_t)step) T.clear_word_or_spare(w, mask);
+#pragma unroll 1
+  for (; x < x_end; x += 4 * step) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j, w += (uint32_t)step) T.clear_word_or_spare(w, mask, j);
+  }
 }
 
 // Clears bit `bit` of bytes byte, byte + p, byte + 2p, ... below Lt (p odd).  Four consecutive
@@ -301,9 +309,9 @@ __device__ __forceinline__ void clear_progression(const TileBits& T, uint32_t by
       w0 += step;
     } while (w0 < lim);
   }
-  T.clear_word_or_spare(w0, m0);
-  T.clear_word_or_spare(w0 + d1, m1);
-  T.clear_word_or_spare(w0 + d2, m2);
+  T.clear_word_or_spare(w0, m0, 0);
+  T.clear_word_or_spare(w0 + d1, m1, 1);
+  T.clear_word_or_spare(w0 + d2, m2, 2);
 }
 
 struct ClassStep {  // c_cls_step of one class
@@ -317,9 +325,11 @@ struct ClassStep {  // c_cls_step of one class
 // then rounds of eight predicated clears, each round one period p further.  For primes above the
 // tile length one round does it.  The class is the warp's, so corr_j and the bits are the same
 // for all lanes: nothing is looked up per hit, and nothing branches but the round loop.
-// Bound by issue slots: 52 instructions per round of eight clears and about 100 around them (loads,
-// remainder, first hits), against 451k per tile near 10^12 of a walk from multiple to multiple
-// whose steps depend on the lane's own class; shared-memory wavefronts are next (3.2 per clear).
+// Bound by shared-memory wavefronts (3.6 per clear, random banks) and issue slots alike (84 and 77 % of
+// their peaks): 343k warp instructions per tile near 10^12, against 451k of a walk from multiple to
+// multiple whose steps depend on the lane's own class.  kOneRound (pmin >= Lt) clears each hit where
+// it is found: 17.9 against 18.4 ms for the 10^11 integers below 10^12.
+template <bool kOneRound>
 __device__ __forceinline__ void clear_class_primes(const TileBits& T, uint32_t p, uint32_t r, uint32_t pmin,
                                                    const ClassStep& C, uint32_t Lt) {
   const uint32_t a = p / 30u, a2 = 2u * a, a4 = 2u * a2, a6 = a4 + a2;
@@ -329,13 +339,16 @@ __device__ __forceinline__ void clear_class_primes(const TileBits& T, uint32_t p
   for (int j = 0; j < 8; ++j) {
     constexpr uint32_t gap[8] = {1, 6, 4, 2, 4, 2, 4, 6};  // W30[j] - W30[j - 1]
     t += (gap[j] == 1 ? a : gap[j] == 2 ? a2 : gap[j] == 4 ? a4 : a6) + C.corr[j];
-    x[j] = 8u * min(t, t + p) + C.bit[j];  // t mod p: a negative t is a large unsigned
+    const uint32_t s = __viaddmin_u32(t, p, t);  // t mod p: a negative t is a large unsigned
+    if (kOneRound) T.clear(T.word_or_spare(s, j), bit_mask(s, C.bit[j]));
+    else x[j] = 8u * s + C.bit[j];
   }
+  if (kOneRound) return;
   const uint32_t period = 8u * p;
   for (uint32_t start = 0; start < Lt; start += pmin) {  // no hit of round start / pmin lies below byte start
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      T.clear_bit_or_spare(x[j]);
+      T.clear(T.word_or_spare(x[j] >> 3, j), __funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, x[j]));
       x[j] += period;
     }
   }
@@ -980,7 +993,9 @@ sieve_tiles_kernel(SieveArgs a) {
               inv = pi[i];
             }
             const uint32_t r = mod_by_inv(ktile, kd, p_now, inv_now);
-            clear_class_primes(T, p_now, r, __shfl_sync(0xFFFFFFFFu, p_now, 0), C, Lt);
+            const uint32_t pmin = __shfl_sync(0xFFFFFFFFu, p_now, 0);
+            if (pmin >= Lt) clear_class_primes<true>(T, p_now, r, pmin, C, Lt);
+            else clear_class_primes<false>(T, p_now, r, pmin, C, Lt);
             if (k >= k_end) break;
           }
         }

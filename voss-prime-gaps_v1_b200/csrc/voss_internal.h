@@ -29,7 +29,7 @@ constexpr uint32_t kPreMod[kPreGroups] = {1001u /*7*11*13*/, 323u /*17*19*/, 667
                                           31u /*31*/};
 constexpr uint32_t kPreOff[kPreGroups] = {0u, 1001u, 1324u, 1991u};
 constexpr uint32_t kPreWords = 2022u;
-constexpr uint32_t kSpareWords = 32u;  // behind every tile in shared memory: one word per lane (TileBits)
+constexpr uint32_t kSpareRows = 8u, kSpareWords = 32u * kSpareRows;  // behind every tile in shared memory (TileBits)
 constexpr uint32_t kClsBlock = 256u;
 // mult_factor * tile bytes, the end of the primes that tiles take by class, is at most 64 * 252,252
 constexpr uint32_t kClsLimit = 1u << 24;
