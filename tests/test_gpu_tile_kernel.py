@@ -103,3 +103,10 @@ def test_gap_lists_of_every_sort_in_order(gpu_ctx, ln):
     np.testing.assert_array_equal(got["position"], p[1:][d >= 150])
     np.testing.assert_array_equal(got["gap"], d[d >= 150])
     assert gpu_ctx.gaps_at_least(lo, lo + ln, 150, cap=max(1, got.size)).size == got.size
+
+
+@pytest.mark.parametrize("lo,hi", [(1, 10**6), (10**4, 10**7), (9 * 10**6, 15 * 10**6), (99_000_000, 101_000_000)])
+def test_low_ranges_under_a_context_for_high_ones(gpu_ctx_big, lo, hi):
+    """The base primes of a context for 10^18 fill the tiles below 10^9; only those that struck
+    themselves out are restored."""
+    assert_range_equal(gpu_ctx_big.sieve_range(lo, hi), O.sieve_range(lo, hi))

@@ -538,43 +538,62 @@ struct BlockScratch {
   int32_t warp_max[BLOCK / 32];
   int32_t warp_prefix[BLOCK / 32];
   int32_t block_max;
+  uint32_t block_sum;
   uint32_t warp_sum[BLOCK / 32];
   unsigned long long warp_key[BLOCK / 32];
   bool redo;
 };
 
-// Exclusive max-scan of `v` over thread order; returns the exclusive prefix and, through
-// *total, the max over the block.
+// Exclusive sum-scan of `v` and max-scan of `m` over thread order in one pass, with the totals.
 template <int BLOCK>
-__device__ __forceinline__ int32_t block_excl_max(int32_t v, BlockScratch<BLOCK>& S, int32_t* total) {
+__device__ __forceinline__ void block_excl_sum_max(uint32_t v, int32_t m, BlockScratch<BLOCK>& S, uint32_t* sum_before,
+                                                   uint32_t* sum, int32_t* max_before, int32_t* max_all) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int32_t incl = v;
+  uint32_t vi = v;
+  int32_t mi = m;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    int32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-    if (lane >= d) incl = max(incl, t);
+    const uint32_t tv = __shfl_up_sync(0xFFFFFFFFu, vi, d);
+    const int32_t tm = __shfl_up_sync(0xFFFFFFFFu, mi, d);
+    if (lane >= d) {
+      vi += tv;
+      mi = max(mi, tm);
+    }
   }
-  if (lane == 31) S.warp_max[warp] = incl;
+  if (lane == 31) {
+    S.warp_sum[warp] = vi;
+    S.warp_max[warp] = mi;
+  }
   __syncthreads();
   if (warp == 0) {
-    int32_t x = lane < BLOCK / 32 ? S.warp_max[lane] : -1;
-    int32_t y = x;
+    const uint32_t x = lane < BLOCK / 32 ? S.warp_sum[lane] : 0;
+    uint32_t xi = x;
+    int32_t yi = lane < BLOCK / 32 ? S.warp_max[lane] : -1;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      int32_t t = __shfl_up_sync(0xFFFFFFFFu, y, d);
-      if (lane >= d) y = max(y, t);
+      const uint32_t tv = __shfl_up_sync(0xFFFFFFFFu, xi, d);
+      const int32_t tm = __shfl_up_sync(0xFFFFFFFFu, yi, d);
+      if (lane >= d) {
+        xi += tv;
+        yi = max(yi, tm);
+      }
     }
-    int32_t ex = __shfl_up_sync(0xFFFFFFFFu, y, 1);
-    if (lane == 0) ex = -1;
-    if (lane < BLOCK / 32) S.warp_prefix[lane] = ex;
-    if (lane == BLOCK / 32 - 1) S.block_max = y;
+    const int32_t ye = __shfl_up_sync(0xFFFFFFFFu, yi, 1);
+    if (lane < BLOCK / 32) {
+      S.warp_sum[lane] = xi - x;  // exclusive over the warps
+      S.warp_prefix[lane] = lane == 0 ? -1 : ye;
+    }
+    if (lane == BLOCK / 32 - 1) {
+      S.block_sum = xi;
+      S.block_max = yi;
+    }
   }
   __syncthreads();
-  int32_t ex = __shfl_up_sync(0xFFFFFFFFu, incl, 1);
-  if (lane == 0) ex = -1;
-  ex = max(ex, S.warp_prefix[warp]);
-  *total = S.block_max;
-  return ex;
+  const int32_t me = __shfl_up_sync(0xFFFFFFFFu, mi, 1);
+  *sum_before = vi - v + S.warp_sum[warp];
+  *max_before = max(lane == 0 ? -1 : me, S.warp_prefix[warp]);
+  *sum = S.block_sum;
+  *max_all = S.block_max;
 }
 
 template <int BLOCK>
@@ -649,6 +668,10 @@ __device__ __forceinline__ uint32_t acc_index(uint32_t i) {
 
 // Small primes' records (prime, remainder, residue class) take 13 + 13 + 3 bits of a word.
 constexpr uint32_t kSmallPrimeEnd = 1u << 13;
+// Lanes per prime of the progressions.  A warp's item is then 16 primes, and the longest item (640
+// clears in a row for 32 primes above tile/80) no longer outlasts the others where few primes follow:
+// [1, 10^9] 280 -> 252 us of tiles, one interval of 10^6 33 -> 28 us; 4 and 8 lanes cost long runs 1 and 2 %.
+constexpr uint32_t kProgLanes = 2;
 
 constexpr uint32_t kFlushEvery = 2048;  // tiles between counter flushes (u32 headroom)
 
@@ -718,10 +741,16 @@ __device__ __forceinline__ void tile_header(TileHdr& H, CtaState& St, const Siev
       const uint32_t w_max = __reduce_max_sync(0xFFFFFFFFu, w_n);
       const uint32_t w_item = w_max >= 4096u ? 256u : (w_max >= 1024u ? 128u : 32u);
       const uint32_t w_items = 8u * ((w_max + w_item - 1u) / w_item);
+      // base primes that lie in the tile and may have been struck out as their own multiple: up to the
+      // interval's root (the pre-pass), rounded up to a kClsBlock as above.  Below 2^24, where blocks
+      // are in use, kClsBlock primes span less than 2^16; a context for 10^16 holds primes up to 10^8,
+      // and restoring all of a tile's near 10^7 took 80 us.
       uint32_t r0 = a.n_primes, r1 = a.n_primes;
-      if (vbase <= a.p_max) {
+      const uint64_t root = vbase <= a.p_max ? isqrt_u64(iv.hi - 1) : 0;
+      if (vbase <= a.p_max && vbase <= root + 65536u) {
+        const uint32_t used = count_le_warp(a.primes, a.n_primes, root, ln) + kClsBlock;
         r0 = count_lt_warp(a.primes, a.n_primes, vbase, ln);
-        r1 = count_lt_warp(a.primes, a.n_primes, vbase + 30ull * lt, ln);
+        r1 = min(count_lt_warp(a.primes, a.n_primes, vbase + 30ull * lt, ln), used);
       }
       if (ln == 0) {
         H.ktile = ktile;
@@ -936,23 +965,27 @@ sieve_tiles_kernel(SieveArgs a) {
       VOSS_PHASE(3)
       // medium primes
       if (a.b_mode == 0) {
-        // a thread per prime, 8 residue progressions; warps claim 32 consecutive primes at a time
+        // kProgLanes lanes per prime, each some of its 8 residue progressions; warps claim 32 / kProgLanes
+        // consecutive primes at a time
+        constexpr uint32_t kPrimes = 32u / kProgLanes, kRes = 8u / kProgLanes;
+        const uint32_t part = (uint32_t)lane / kPrimes;
         for (;;) {
           uint32_t base = 0;
-          if (lane == 0) base = atomicAdd(&H.b_ctr, 32u);
+          if (lane == 0) base = atomicAdd(&H.b_ctr, kPrimes);
           base = __shfl_sync(0xFFFFFFFFu, base, 0);
           if (base >= iw - ia) break;
-          const uint32_t i = ia + base + (uint32_t)lane;
+          const uint32_t i = ia + base + (uint32_t)lane % kPrimes;
           if (i < iw) {
             const uint32_t p = a.primes[i];
             const uint64_t m = a.magic[i];
             const uint32_t r = fma_mod ? mod_by_magic_fma(ktile, ks, p, m) : mod_barrett(ktile, p, m);
             const uint32_t pa = p / 30u, bi = (uint32_t)s_rb[p - 30u * pa];
-            const uint2 st8 = reinterpret_cast<const uint2*>(s_step)[bi];  // the prime's 8 entries
+            const uint64_t st = *reinterpret_cast<const uint64_t*>(s_step + 8u * bi) >> (8u * kRes * part);
+            const uint64_t wr = kW30Packed >> (8u * kRes * part);
 #pragma unroll
-            for (uint32_t o = 0; o < 8; ++o) {
-              const uint32_t e = ((o < 4u ? st8.x : st8.y) >> (8u * (o & 3u))) & 0xFFu;
-              const uint32_t delta = pa * w30(o) + (e & 31u);
+            for (uint32_t o = 0; o < kRes; ++o) {
+              const uint32_t e = (uint32_t)(st >> (8u * o)) & 0xFFu;
+              const uint32_t delta = pa * ((uint32_t)(wr >> (8u * o)) & 0xFFu) + (e & 31u);
               clear_progression(T, delta >= r ? delta - r : delta + p - r, p, e >> 5, Lt);
             }
           }
@@ -1044,7 +1077,7 @@ sieve_tiles_kernel(SieveArgs a) {
     VOSS_PHASE(5)
 
     // ---- 3. restore primes lying in the tile ---------------------------------------------
-    {
+    if (H.vbase < 32 || H.r0 < H.r1) {
       const uint64_t vbase = H.vbase, vlo = H.vlo, vhi = H.vhi, vend = vbase + 30ull * Lt;
       if (vbase < 32 && tid < 8) {
         const uint32_t sp[8] = {7, 11, 13, 17, 19, 23, 29, 31};
@@ -1062,8 +1095,8 @@ sieve_tiles_kernel(SieveArgs a) {
             atomicOr(bm + (k >> 2), 1u << (((k & 3u) << 3) | (uint32_t)s_rb[off - 30u * k]));
         }
       }
+      __syncthreads();
     }
-    __syncthreads();
     VOSS_PHASE(6)
 
     // ---- 4. extract -----------------------------------------------------------------------
@@ -1106,10 +1139,9 @@ sieve_tiles_kernel(SieveArgs a) {
           break;
         }
       }
-      uint32_t tile_cnt;
-      const uint32_t rank0 = block_excl_sum<BLOCK>(pc, S, &tile_cnt);
-      int32_t tile_last;
-      const int32_t before = block_excl_max<BLOCK>(my_last, S, &tile_last);
+      uint32_t tile_cnt, rank0;
+      int32_t tile_last, before;
+      block_excl_sum_max<BLOCK>(pc, my_last, S, &rank0, &tile_cnt, &before, &tile_last);
       s_rank[tid] = rank0;
       s_mid[tid] = (uint16_t)pc_half;
       s_before[tid] = before;
@@ -1162,7 +1194,7 @@ sieve_tiles_kernel(SieveArgs a) {
       // The walk works in bitmap bits (bit 8k + o of the tile = integer 30k + W30[o]): one counter
       // per (distance d, residue of the lower prime), no conversion to integers.  Only gaps of at
       // least t_far bits are looked at closer (far_gap): t_far is such that every large-gap
-      // candidate is one (a gap of g holds at least 8g/30 - 0.87 bits), and about sixteen others of
+      // candidate is one (a gap of g holds at least 8g/30 - 0.87 bits), and about thirty others of
       // the tile, so that the longest gap is found among them.  If it is not clear that it was (a
       // gap below t_far bits is below 3.75 t_far), the tile's gaps are gone through again.
       // Bound by issue slots: 205k warp instructions per tile of 218,000 primes (near 10^12), against
@@ -1171,7 +1203,7 @@ sieve_tiles_kernel(SieveArgs a) {
       uint32_t t_far;
       {
         const float bits = 32.0f * (float)nw / (float)(tile_cnt | 1u);
-        const float t = bits * __logf((float)(tile_cnt | 1u) * (1.0f / 16.0f));
+        const float t = bits * __logf((float)(tile_cnt | 1u) * (1.0f / 32.0f));
         t_far = t < 1.0f ? 1u : (t > (float)kGapBits ? kGapBits : (uint32_t)t);
         if (cthr < 2u * kGapBits * 15u / 8u) t_far = min(t_far, max(1u, 8u * cthr / 30u));
       }

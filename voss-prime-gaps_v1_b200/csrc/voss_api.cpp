@@ -199,10 +199,10 @@ TileShape default_shape(const voss_ctx* c) {
 //  - the pre-pass, which spreads over all SMs: at 40 sqrt(integers) the tiles' share of the
 //    remaining primes costs about what the pre-pass's bitmap atomics do (best of a sweep over
 //    2^11..2^19: 8192, 32768, 131072, 524288 for 10^5..10^8 integers);
-//  - in a single wave, small primes up to tile/20: a warp each instead of a lane each, whose few
-//    dozen clears in a row were the longest chain of such a launch.
-// Device time before and after: 10^6 integers at 10^12 115 -> 62 us, 10^7 203 -> 73, 10^8 201 -> 121,
-// 10^9 365 -> 317; [1, 10^8] 306 -> 92, [1, 10^9] 307 -> 266.
+//  - in a single wave of short chunks, small primes up to tile/40: a warp each instead of two lanes
+//    each, whose clears in a row are the longest chain of such a launch ([1, 10^7] 67 -> 57 us).
+// Device time in the default tile and so: 10^6 integers at 10^12 115 -> 62 us, 10^7 203 -> 70,
+// 10^8 201 -> 117, 10^9 354 -> 272; [1, 10^8] 306 -> 85, [1, 10^9] 251 -> 219.
 TileShape choose_shape(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, uint32_t n, uint64_t max_tiles) {
   constexpr uint64_t kMaxWaves = 6;
   constexpr double kTileSetup = 40.0;
@@ -225,7 +225,7 @@ TileShape choose_shape(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi
     return max_tiles && tiles > max_tiles ? 0 : (tiles + slots - 1) / slots;
   };
   uint64_t best = dflt.chunk_words, best_waves = waves_of(best);
-  double cost = 0.95 * (double)best_waves * ((double)best + kTileSetup);  // at least 5 % better
+  double cost = 0.98 * (double)best_waves * ((double)best + kTileSetup);  // at least 2 % better
   for (uint64_t k = 1; k <= kMaxWaves; ++k) {
     const uint64_t chunk = ((total + block * k * slots - 1) / (block * k * slots)) | 1;
     if (chunk >= dflt.chunk_words) continue;
@@ -241,7 +241,7 @@ TileShape choose_shape(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi
   s.chunk_words = (uint32_t)best;
   const double reach = 40.0 * std::sqrt(120.0 * (double)total);
   s.p_large = (uint32_t)std::min<double>(dflt.p_large, std::max(8192.0, reach));
-  if (best_waves == 1) s.coop_div = std::max(1u, dflt.coop_div / 4);
+  if (best_waves == 1 && best < 10) s.coop_div = std::max(1u, dflt.coop_div / 2);
   return s;
 }
 
