@@ -923,18 +923,29 @@ sieve_tiles_kernel(SieveArgs a) {
           return m;
         };
         uint32_t w = c;
-        if (gbm || w < w_in) {
-          for (; w < nw; w += 1001u) {
-            uint32_t m = mask();
-            if (gbm) m &= gbm[w];
-            if (w < w_in || w >= w_out) m &= edge_mask(vbase + 120ull * w, vlo, vhi);
-            bm[w] = m;
+        auto edge = [&](uint32_t end) {  // words that reach out of the interval
+          for (; w < end; w += 1001u) {
+            const uint32_t m = mask() & edge_mask(vbase + 120ull * w, vlo, vhi);
+            bm[w] = gbm ? m & gbm[w] : m;
           }
+        };
+        edge(min(w_in, nw));
+        if (gbm) {
+          // the pre-pass's words, eight loads in flight per thread: one at a time they cost a tile 51
+          // trips to L2 (4.7e9 integers near 10^15: 1172 -> 1095 us of tiles)
+          for (; w + 7u * 1001u < w_out; w += 8u * 1001u) {
+            uint32_t g[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) g[k] = __ldcg(gbm + w + 1001u * (uint32_t)k);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) bm[w + 1001u * (uint32_t)k] = mask() & g[k];
+          }
+          for (; w < w_out; w += 1001u) bm[w] = mask() & __ldcg(gbm + w);
         } else {
 #pragma unroll 4
           for (; w < w_out; w += 1001u) bm[w] = mask();
-          for (; w < nw; w += 1001u) bm[w] = mask() & edge_mask(vbase + 120ull * w, vlo, vhi);
         }
+        edge(nw);
       }
     }
     __syncthreads();
