@@ -110,3 +110,14 @@ def test_low_ranges_under_a_context_for_high_ones(gpu_ctx_big, lo, hi):
     """The base primes of a context for 10^18 fill the tiles below 10^9; only those that struck
     themselves out are restored."""
     assert_range_equal(gpu_ctx_big.sieve_range(lo, hi), O.sieve_range(lo, hi))
+
+
+@pytest.mark.parametrize("lo", [26 * 10**11, 8 * 10**12, 16 * 10**12, 17 * 10**12])
+def test_long_ranges_around_the_prepass_rule(lo):
+    """Ranges whose root lies just above the pre-pass's bound sieve those primes in the tiles; the
+    same range through the pre-pass."""
+    import voss
+    with voss.Context(2 * 10**13) as ctx:
+        r = ctx.sieve_range(lo, lo + 3 * 10**9)
+        ctx.set_tuning(mult_factor=8)  # a fixed shape: its pre-pass bound is 8 tile lengths
+        assert_range_equal(ctx.sieve_range(lo, lo + 3 * 10**9), r)

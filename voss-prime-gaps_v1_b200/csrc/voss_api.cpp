@@ -209,6 +209,18 @@ TileShape choose_shape(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi
   const TileShape dflt = default_shape(c);
   const uint64_t slots = (uint64_t)c->sm_count * c->ctas_per_sm, block = c->tune.block_threads;
   if (!c->auto_shape || n > kMaxWaves * slots) return dflt;
+  // A long range whose root is up to 2.5 times the pre-pass's bound (twice for two or three waves)
+  // does without the pre-pass: its clears are atomics in L2 (2.4e11 per second), its bitmap is filled and read back,
+  // and the tiles take those primes by class for less (2*10^10 integers at 3, 10 and 16*10^12:
+  // 5.43 -> 4.35, 6.36 -> 5.57, 6.84 -> 6.26 ms; at 23*10^12 6.88 -> 6.90).
+  auto without_prepass = [&](TileShape s, uint64_t waves) {
+    if (n == 1 && waves >= 2 && hi[0] > 1) {
+      const uint64_t root = isqrt_u64(hi[0] - 1);
+      if (root >= s.p_large && 2 * root <= (waves >= 4 ? 5ull : 4ull) * dflt.p_large && root < kClsLimit)
+        s.p_large = (uint32_t)root + 1u;
+    }
+    return s;
+  };
   std::vector<uint64_t> words;
   words.reserve(n);
   uint64_t total = 0;
@@ -218,7 +230,8 @@ TileShape choose_shape(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi
     words.push_back(((hi[i] - 1) / 30 - ((a / 30) & ~3ull)) / 4 + 1);
     total += words.back();
   }
-  if (total == 0 || total > kMaxWaves * slots * block * dflt.chunk_words) return dflt;
+  if (total == 0) return dflt;
+  if (total > kMaxWaves * slots * block * dflt.chunk_words) return without_prepass(dflt, kMaxWaves);
   auto waves_of = [&](uint64_t chunk) -> uint64_t {
     uint64_t tiles = 0;
     for (uint64_t w : words) tiles += (w + block * chunk - 1) / (block * chunk);
@@ -236,13 +249,13 @@ TileShape choose_shape(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi
       cost = (double)waves * ((double)chunk + kTileSetup);
     }
   }
-  if (best == dflt.chunk_words) return dflt;
+  if (best == dflt.chunk_words) return without_prepass(dflt, best_waves);
   TileShape s = dflt;
   s.chunk_words = (uint32_t)best;
   const double reach = 40.0 * std::sqrt(120.0 * (double)total);
   s.p_large = (uint32_t)std::min<double>(dflt.p_large, std::max(8192.0, reach));
   if (best_waves == 1 && best < 10) s.coop_div = std::max(1u, dflt.coop_div / 2);
-  return s;
+  return without_prepass(s, best_waves);
 }
 
 // Cut intervals [lo_i, hi_i) into tiles; intervals without wheel integers get no tiles.
