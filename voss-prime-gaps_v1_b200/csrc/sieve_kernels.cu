@@ -354,16 +354,18 @@ __device__ __forceinline__ void clear_class_primes(const TileBits& T, uint32_t p
   }
 }
 
-// x = *p (shared memory) if `yes`, as a predicated load.
-__device__ __forceinline__ void load_if(uint32_t& x, const uint32_t* p, bool yes) {
+// The word at shared-memory address p + 4 into x, and p on to it, if x is used up (zero): one
+// predicated step, without a branch.
+__device__ __forceinline__ void next_word_if_spent(uint32_t& x, uint32_t& p) {
   asm volatile(
       "{\n\t"
-      ".reg .pred yes;\n\t"
-      "setp.ne.u32 yes, %2, 0;\n\t"
-      "@yes ld.shared.u32 %0, [%1];\n\t"
+      ".reg .pred spent;\n\t"
+      "setp.eq.u32 spent, %0, 0;\n\t"
+      "@spent add.u32 %1, %1, 4;\n\t"
+      "@spent ld.shared.u32 %0, [%1];\n\t"
       "}"
-      : "+r"(x)
-      : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"((uint32_t)yes)
+      : "+r"(x), "+r"(p)
+      :
       : "memory");
 }
 
@@ -1208,8 +1210,10 @@ sieve_tiles_kernel(SieveArgs a) {
       // candidate is one (a gap of g holds at least 8g/30 - 0.87 bits), and about thirty others of
       // the tile, so that the longest gap is found among them.  If it is not clear that it was (a
       // gap below t_far bits is below 3.75 t_far), the tile's gaps are gone through again.
-      // Bound by issue slots: 205k warp instructions per tile of 218,000 primes (near 10^12), against
-      // 294k with positions as integers, a branch per reload and the longest gap tracked per prime.
+      // Bound by issue slots: 294k warp instructions per tile of 218,000 primes (near 10^12) with positions
+      // as integers, a branch per reload and the longest gap tracked per prime; 205k with bit distances and
+      // one vote; the step to the next word as one predicated sequence on its address took another 5 %
+      // off the whole kernel (17.7 -> 16.9 ms for the 10^11 integers below 10^12).
       const uint32_t cthr = H.cthr;
       uint32_t t_far;
       {
@@ -1219,7 +1223,9 @@ sieve_tiles_kernel(SieveArgs a) {
         if (cthr < 2u * kGapBits * 15u / 8u) t_far = min(t_far, max(1u, 8u * cthr / 30u));
       }
       uint32_t mg = 0, mlo = 0;
-      auto value = [&](uint32_t bit) { return 120u * (bit >> 5) + s_pos[bit & 31u]; };
+      // bits are counted from shared-memory address 0, so a word's address gives its first bit
+      const uint32_t sb = (uint32_t)__cvta_generic_to_shared(bm), bit0 = 8u * sb;
+      auto value = [&](uint32_t bit) { return 120u * ((bit - bit0) >> 5) + s_pos[(bit - bit0) & 31u]; };
       auto far_gap = [&](uint32_t lo_bit, uint32_t hi_bit, bool crossing) {
         const uint32_t pv = value(lo_bit), pos = value(hi_bit), g = pos - pv;
         if (crossing || hi_bit - lo_bit >= kGapBits) {  // not counted in shared memory
@@ -1247,36 +1253,34 @@ sieve_tiles_kernel(SieveArgs a) {
           }
         }
       };
-      uint32_t it0 = 0;
+      uint32_t left = n_mine;
+      uint32_t wp = sb + 4u * w;  // address of the word that x comes from
+      if (n_mine)
+        while (x == 0u) next_word_if_spent(x, wp);  // the tile holds this thread's primes: wp stays inside it
       if (prev < 0 && n_mine) {
         // the tile's first prime: no predecessor in the tile (exactly one thread)
-        while (x == 0u) x = bm[++w];
-        const uint32_t b = (uint32_t)__ffs(x) - 1u;
+        prev = (int32_t)(8u * (wp - sb) + (uint32_t)__ffs(x) - 1u);
         x &= x - 1u;
-        prev = (int32_t)(32u * w + b);
-        H.first = value((uint32_t)prev);
-        it0 = 1;
+        H.first = value(bit0 + (uint32_t)prev);
+        --left;
+        if (left)
+          while (x == 0u) next_word_if_spent(x, wp);
       }
-      if (n_mine > it0)
-        while (x == 0u) x = bm[++w];  // the tile holds primes of this thread: w stays inside it
-      uint32_t pv = (uint32_t)prev;
-      const uint32_t vb = H.vb == kNone ? kNone : 8u * (H.vb / 30u);  // the boundary's first bit
+      uint32_t pv = bit0 + (uint32_t)prev;
+      const uint32_t vb = H.vb == kNone ? kNone : bit0 + 8u * (H.vb / 30u);  // the boundary's first bit
       // Instantiated twice: in a tile without a segment boundary (nearly all of them) the crossing
       // test drops out of the loop.
       auto walk = [&](auto cross_tag) {
         constexpr bool kCross = decltype(cross_tag)::value;
-        uint32_t left = n_mine - it0;
         // All but the last prime, the warp's lanes side by side: the next word is a predicated load,
         // and one vote covers what is rare, a far gap or a word without primes (a branch of its own
         // for the reload diverges at nearly every prime).
         const uint32_t common = __reduce_min_sync(0xFFFFFFFFu, left);
 #pragma unroll 4
         for (uint32_t it = 1; it < common; ++it) {
-          const uint32_t bit = 32u * w + (uint32_t)__ffs(x) - 1u;
+          const uint32_t bit = 8u * wp + (uint32_t)__ffs(x) - 1u;
           x &= x - 1u;
-          const bool spent = x == 0u;
-          w += spent ? 1u : 0u;
-          load_if(x, bm + w, spent);
+          next_word_if_spent(x, wp);
           const uint32_t d = bit - pv;
           const bool crossing = kCross && (pv < vb) && (bit >= vb);
           const uint32_t slot = min(8u * d + (pv & 7u), (uint32_t)kSmSpare);
@@ -1284,14 +1288,14 @@ sieve_tiles_kernel(SieveArgs a) {
           const bool far = d >= t_far || crossing;
           if (__any_sync(0xFFFFFFFFu, far || x == 0u)) {
             if (far) far_gap(pv, bit, crossing);
-            while (x == 0u) x = bm[++w];  // this lane has primes left: w stays inside the tile
+            while (x == 0u) next_word_if_spent(x, wp);  // this lane has primes left
           }
           pv = bit;
         }
         left -= common ? common - 1u : 0u;
         for (; left; --left) {
-          while (x == 0u) x = bm[++w];
-          const uint32_t bit = 32u * w + (uint32_t)__ffs(x) - 1u;
+          while (x == 0u) next_word_if_spent(x, wp);
+          const uint32_t bit = 8u * wp + (uint32_t)__ffs(x) - 1u;
           x &= x - 1u;
           const uint32_t d = bit - pv;
           const bool crossing = kCross && (pv < vb) && (bit >= vb);
@@ -1309,7 +1313,7 @@ sieve_tiles_kernel(SieveArgs a) {
       auto store_partial = [&](unsigned long long key) {
         TilePartial P;
         P.first = tile_cnt ? H.first : kNone;
-        P.last = tile_cnt ? value((uint32_t)tile_last) : kNone;
+        P.last = tile_cnt ? value(bit0 + (uint32_t)tile_last) : kNone;
         P.count = tile_cnt;
         P.max_gap = (uint32_t)(key >> 32);
         P.max_lo = key ? 0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFull) : 0u;
@@ -1335,7 +1339,7 @@ sieve_tiles_kernel(SieveArgs a) {
           for (uint32_t y = bm[ww]; y; y &= y - 1u) {
             const uint32_t bit = 32u * ww + (uint32_t)__ffs(y) - 1u;
             if (pb >= 0) {
-              const uint32_t lo_v = value((uint32_t)pb), g = value(bit) - lo_v;
+              const uint32_t lo_v = value(bit0 + (uint32_t)pb), g = value(bit0 + bit) - lo_v;
               mlo = g > mg ? lo_v : mlo;
               mg = g > mg ? g : mg;
             }
