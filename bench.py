@@ -6,7 +6,7 @@ reference's statistics in reference-compat mode: pi(N), the gap histogram, mod-4
 counts, the per-residue gap histogram, the large-gap list and the maximal gap.  Metric:
 range/s = integers sieved per second (higher is better).
 
-  value      device time of the sieve+stitch+reduce kernels per step (CUDA events on the
+  value      device time of the sieve and tail kernels per step (CUDA events on the
              launching stream, L2 flushed between steps outside the timed events), max over
              ranks; inputs (base-prime table) resident in HBM.
   e2e        the same step through the public C ABI call voss_sieve_range with host result
@@ -265,12 +265,12 @@ _MR_BASES = (2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37)
 
 
 def mr_mulmods(sample) -> tuple[int, int]:
-    """Montgomery products the Miller-Rabin kernels' algorithm needs for these candidates,
-    (moduli below 2^63, moduli above): per candidate that trial division by 2..37 leaves open,
+    """Montgomery products the reference's method (strong tests to the prime bases) needs for these
+    candidates, (moduli below 2^63, moduli above): per candidate that trial division by 2..37 leaves open,
     for each base in order up to the first that fails, or up to as many bases as n's size needs
     (6, 7, 9 or 12): one squaring per bit of the odd part d, one product per set bit of d (none
     for base 2, whose products are doublings), and the squarings of the r - 1 follow-up steps
-    up to the first -1.  The lanes' padding in the warp-uniform loops is overhead, not counted."""
+    up to the first -1.  mr_products counts what the kernel's own method needs."""
     small = full = 0
     for n in map(int, sample):
         if n < 2 or n % 2 == 0 or any(n == b or n % b == 0 for b in _MR_BASES[1:]):
@@ -298,6 +298,42 @@ def mr_mulmods(sample) -> tuple[int, int]:
         else:
             full += cnt
     return small, full
+
+
+_MR_DOUBLE_END = 1 << 49  # below it the kernel's products are in double precision
+_FP64_OPS_PER_PRODUCT = 6
+_FP64_LANES_PER_CYCLE_SM = 62.0  # fp64 fma, measured on a B200
+
+
+def mr_products(sample) -> tuple[int, int, int]:
+    """Modular products the primality kernel's method needs for these candidates, (moduli below
+    2^49, from 2^49 to 2^63, above): per candidate that trial division by 2..37 leaves open, a
+    strong test to base 2 (one squaring per bit of the odd part of n - 1, then squarings up to the
+    first -1), and for its survivors an extra strong Lucas test (two products per bit of the odd
+    part of n + 1, then squarings up to the first 0; only primes get there but for a few
+    pseudoprimes, so the ladder is counted in full).  Lanes padded to a warp's trip count are
+    overhead, not counted."""
+    cnt = [0, 0, 0]
+    for n in map(int, sample):
+        if n < 2 or n % 2 == 0 or any(n == b or n % b == 0 for b in _MR_BASES[1:]):
+            continue
+        d = n - 1
+        r = (d & -d).bit_length() - 1
+        d >>= r
+        k = d.bit_length()
+        x = pow(2, d, n)
+        ok = x == 1 or x == n - 1
+        for _ in range(r - 1):
+            if ok:
+                break
+            x = x * x % n
+            k += 1
+            ok = x == n - 1
+        if ok:
+            e = n + 1
+            k += 2 * (e // (e & -e)).bit_length()
+        cnt[0 if n < _MR_DOUBLE_END else 1 if n < 1 << 63 else 2] += k
+    return cnt[0], cnt[1], cnt[2]
 
 
 # ---------------------------------------------------------------------------------------
@@ -507,7 +543,7 @@ def mr_candidates(ctx, half: int, seed: int = 20261203):
 
 
 def run_mr(a) -> dict:
-    """Batched verification: 1e8 candidates through deterministic Miller-Rabin (12 bases), and
+    """Batched verification: 1e8 candidates through the deterministic primality kernel, and
     the interior-composite proof of every gap >= 200 below 1e12."""
     import numpy as np
     import torch
@@ -534,14 +570,17 @@ def run_mr(a) -> dict:
     torch.cuda.synchronize()
     clk = clocks.stop()
     ms = statistics.mean(e0.elapsed_time(e1) for e0, e1 in ev)
-    # roofline: Montgomery products the algorithm needs (counted on a seeded sample of the
-    # batch, scaled) against this GPU's measured product rate, per modulus class
+    # roofline: modular products the kernel's method needs (counted on a seeded sample of the
+    # batch, scaled) against this GPU's product rate, per modulus class
     msample = n[: min(n.size, 100_000)]
-    m_small, m_full = mr_mulmods(msample)
     scale = n.size / msample.size
-    m_small, m_full = m_small * scale, m_full * scale
+    m_dbl, m_small, m_full = (k * scale for k in mr_products(msample))
+    m_all = m_dbl + m_small + m_full
     peak_full, peak_small = ctx.probe_mulmod()
-    t_ideal = m_small / peak_small + m_full / peak_full
+    sm_hz = 1e6 * (clk["sm_mhz"] or 1965.0)
+    peak_dbl = (_FP64_LANES_PER_CYCLE_SM / _FP64_OPS_PER_PRODUCT * sm_hz
+                * torch.cuda.get_device_properties(0).multi_processor_count)
+    t_ideal = m_dbl / peak_dbl + m_small / peak_small + m_full / peak_full
     t_meas = ms * 1e-3
     got = d_out.cpu().numpy()
     # e2e through the host-buffer entry point
@@ -582,7 +621,8 @@ def run_mr(a) -> dict:
         "value": n.size / (ms * 1e-3), "unit": "candidates/s", "n_gpus": 1, "steps": a.steps, "warmup": a.warmup,
         "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "u64",
         "data": "synthetic: sieved primes + PCG64 seed 20261203 odd values",
-        "config": {"workload": "batched Miller-Rabin, bases 2..37, 64-bit Montgomery", "candidates": int(n.size),
+        "config": {"workload": "batched deterministic primality of 64-bit integers (trial division 2..37, "
+                               "strong test to base 2, extra strong Lucas test)", "candidates": int(n.size),
                    "known_primes": int(known.sum())},
         "e2e": {"value": n.size / e2e, "unit": "candidates/s", "h2d_bytes_per_step": 8 * int(n.size),
                 "d2h_bytes_per_step": int(n.size), "api": "voss_mr_verify (host buffers)"},
@@ -593,20 +633,24 @@ def run_mr(a) -> dict:
                          "sample": f"first {sample.size} candidates through verify_cpp.cpp is_prime_u64",
                          "matches_gpu": match},
         "gap_proofs": proofs,
-        "roofline": {"bound": "int", "achieved": (m_small + m_full) / t_meas / 1e9,
-                     "peak": (m_small + m_full) / t_ideal / 1e9, "unit": "G Montgomery products/s",
+        "roofline": {"bound": "fp64+int", "achieved": m_all / t_meas / 1e9,
+                     "peak": m_all / t_ideal / 1e9, "unit": "G modular products/s",
                      "frac": t_ideal / t_meas, "traffic": None,
-                     "kernel": "mr_sieve_kernel + mr_finish_kernel (one call)", "kernel_ms": ms,
-                     "products_per_candidate": (m_small + m_full) / n.size,
-                     "products_small_modulus": m_small, "products_full_modulus": m_full,
-                     "peak_small_per_s": peak_small, "peak_full_per_s": peak_full,
-                     "peak_source": "voss_probe_mulmod: independent Montgomery squaring chains on this GPU in "
-                                    "this run (moduli < 2^63 and >= 2^63); peak = the products' time-weighted rate",
+                     "kernel": "mr_kernel (one launch per call)", "kernel_ms": ms,
+                     "products_per_candidate": m_all / n.size,
+                     "products_below_2_49": m_dbl, "products_2_49_to_2_63": m_small,
+                     "products_from_2_63": m_full,
+                     "peak_below_2_49_per_s": peak_dbl, "peak_small_per_s": peak_small,
+                     "peak_full_per_s": peak_full,
+                     "peak_source": "below 2^49: six fp64 operations per product at the fp64 pipe's measured "
+                                    "rate; above: voss_probe_mulmod, independent Montgomery squaring chains on "
+                                    "this GPU in this run (moduli < 2^63 and >= 2^63); peak = the products' "
+                                    "time-weighted rate",
                      "count_sample": int(msample.size),
-                     "traffic_note": "8 B read + 1 B written per candidate; mr_finish_kernel DRAM figures in "
-                                     "profiles/mr_finish_kernel_2e6.md"},
+                     "traffic_note": "8 B read + 1 B written per candidate; DRAM figures in "
+                                     "profiles/mr_kernel_2e6.md"},
         "clocks": clk,
-        "gpu_launches": 2 * a.steps,
+        "gpu_launches": a.steps,
     }
     del ctx
     return out

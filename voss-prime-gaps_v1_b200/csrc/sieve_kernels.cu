@@ -106,18 +106,6 @@ __device__ __forceinline__ uint32_t mod_by_inv(uint64_t x, double xd, uint32_t p
   return min(r, r + p);  // a negative remainder is a large unsigned
 }
 
-// x mod p from a double-precision estimate of the quotient, for p >= 2^11 and x < 2^62:
-// xd = x and inv = 1/p rounded to double, so xd * inv is within (x/p) * 3 * 2^-53 < 2^-1 of x/p
-// and its truncation is floor(x/p) - 1, floor(x/p) or floor(x/p) + 1; one signed correction
-// finishes the remainder.
-__device__ __forceinline__ uint32_t mod_by_estimate(uint64_t x, double xd, uint32_t p, double inv) {
-  const uint64_t q = __double2ull_rz(xd * inv);
-  int64_t r = (int64_t)(x - q * (uint64_t)p);
-  if (r < 0) r += p;
-  else if (r >= (int64_t)p) r -= p;
-  return (uint32_t)r;
-}
-
 __device__ __forceinline__ uint64_t isqrt_u64(uint64_t x) {
   uint64_t s = (uint64_t)sqrt((double)x);
   if (s > 0xFFFFFFFFull) s = 0xFFFFFFFFull;
