@@ -124,9 +124,9 @@ typedef struct voss_tuning {
   uint32_t walk_sixteenths; /* mode 0: primes p >= walk_sixteenths*tile_bytes/16 are taken by residue class
                                mod 30 instead of 8 residue progressions each (>= 16*mult_factor: never;
                                0 = default 2) */
-  uint32_t mr_route;        /* voss_sieve_intervals: an interval whose base primes >= mult_factor*tile_bytes
-                               outnumber mr_route times its length is tested by Miller-Rabin instead of
-                               sieved (0 = default 25; 0xFFFFFFFF = never) */
+  uint32_t mr_route;        /* voss_sieve_intervals: an interval whose base primes outnumber mr_route times
+                               its length is tested by Miller-Rabin instead of sieved (0 = default 25;
+                               0xFFFFFFFF = never) */
 } voss_tuning;
 
 typedef struct voss_ctx voss_ctx;

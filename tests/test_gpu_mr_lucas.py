@@ -48,3 +48,15 @@ def test_batch_sizes(gpu_ctx, count):
     n = rng.integers(0, 2**63, size=count, dtype=np.uint64) * 2 + 1
     n[::3] >>= np.uint64(20)
     check(gpu_ctx, n)
+
+
+@pytest.mark.parametrize("extra", [0, 1])
+def test_both_sides_of_the_line_between_inlined_and_called_tests(gpu_ctx, extra):
+    # one pass of every block (8 blocks of 256 per SM), and one candidate more
+    import torch
+    count = torch.cuda.get_device_properties(0).multi_processor_count * 8 * 256 + extra
+    rng = np.random.default_rng(count)
+    n = rng.integers(0, 2**63, size=count, dtype=np.uint64) * 2 + 1
+    n[::2] >>= np.uint64(16)
+    n[::5] = (np.uint64(1) << np.uint64(49)) + np.arange(n[::5].size, dtype=np.uint64) - np.uint64(n[::5].size // 2)
+    check(gpu_ctx, n)

@@ -321,6 +321,17 @@ __device__ __forceinline__ bool test_lucas(uint64_t n) {
   return ok && P != 0;
 }
 
+// The same as calls: one copy of each test instead of one at every place that drains a queue.
+template <bool kDouble>
+__device__ __noinline__ bool call_base2(uint64_t n) {
+  return test_base2<kDouble>(n);
+}
+
+template <bool kDouble>
+__device__ __noinline__ bool call_lucas(uint64_t n) {
+  return test_lucas<kDouble>(n);
+}
+
 // Trial division for every candidate (a lane per candidate); the undecided wait in the warp's
 // shared-memory queues, one per size class for the base-2 test and one for the Lucas test of its
 // survivors, and each time a queue holds 32 they are tested together.  Lanes whose candidate is
@@ -359,28 +370,35 @@ struct MrQueues {  // of one size class
   uint32_t n_base2, n_lucas;
 };
 
-template <bool kDouble>
+template <bool kDouble, bool kCalls>
 __device__ __forceinline__ void drain_lucas(const uint64_t* __restrict__ cand, uint8_t* __restrict__ out, MrQueues& Q,
                                             uint32_t lane) {
   bool live;
   const uint32_t i = queue_take(Q.lucas, Q.n_lucas, lane, live);
-  const bool ok = test_lucas<kDouble>(cand[i]);
+  const bool ok = kCalls ? call_lucas<kDouble>(cand[i]) : test_lucas<kDouble>(cand[i]);
   if (live) out[i] = ok ? 1 : 0;
 }
 
-template <bool kDouble>
+template <bool kDouble, bool kCalls>
 __device__ __forceinline__ void drain_base2(const uint64_t* __restrict__ cand, uint8_t* __restrict__ out, MrQueues& Q,
                                             uint32_t lane) {
   bool live;
   const uint32_t i = queue_take(Q.base2, Q.n_base2, lane, live);
-  const bool ok = test_base2<kDouble>(cand[i]);
+  const bool ok = kCalls ? call_base2<kDouble>(cand[i]) : test_base2<kDouble>(cand[i]);
   if (live && !ok) out[i] = 0;
   queue_add(Q.lucas, Q.n_lucas, lane, i, live && ok);
-  if (Q.n_lucas >= 32u) drain_lucas<kDouble>(cand, out, Q, lane);
+  if (Q.n_lucas >= 32u) drain_lucas<kDouble, kCalls>(cand, out, Q, lane);
 }
 
-__global__ void __launch_bounds__(kMrBlock) mr_kernel(const uint64_t* __restrict__ cand, uint64_t count,
-                                                      uint8_t* __restrict__ out) {
+// kCalls: for batches that give every block more than one pass.  Inlined, the tests stand at four
+// places each, and a block whose candidates lie on both sides of 2^49 runs through more code than the
+// instruction cache holds (ncu: 2.4 warps waiting for an instruction per issue); as calls there is one
+// copy, and five blocks fit an SM.  10^7 candidates, half of them below 10^12 and half 64-bit: 1031 ->
+// 920 us, 10^6 of them 150 -> 138, 4*10^6 of 48 bits 134 -> 125; 5*10^6 primes below 10^12 490 -> 488 and
+// 4*10^6 64-bit ones 327 -> 335; but 1000 candidates, in calls, 22.7 -> 25.2 us.
+template <bool kCalls>
+__global__ void __launch_bounds__(kMrBlock, kCalls ? 5 : 1) mr_kernel(const uint64_t* __restrict__ cand, uint64_t count,
+                                                                      uint8_t* __restrict__ out) {
   __shared__ uint32_t s_q[kMrBlock / 32][4][kMrQueue];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   MrQueues qd = {s_q[warp][0], s_q[warp][1], 0, 0}, qm = {s_q[warp][2], s_q[warp][3], 0, 0};
@@ -399,8 +417,8 @@ __global__ void __launch_bounds__(kMrBlock) mr_kernel(const uint64_t* __restrict
     }
     queue_add(qd.base2, qd.n_base2, lane, (uint32_t)i, open && dbl);
     queue_add(qm.base2, qm.n_base2, lane, (uint32_t)i, open && !dbl);
-    if (qd.n_base2 >= 32u) drain_base2<true>(cand, out, qd, lane);
-    if (qm.n_base2 >= 32u) drain_base2<false>(cand, out, qm, lane);
+    if (qd.n_base2 >= 32u) drain_base2<true, kCalls>(cand, out, qd, lane);
+    if (qm.n_base2 >= 32u) drain_base2<false, kCalls>(cand, out, qm, lane);
   }
   // What is left in the queues (up to 31 each) is put together over the block, so that the last
   // tests run on full warps: at 4,000,001 candidates a warp sees 422 and leaves half a warp of
@@ -428,14 +446,15 @@ __global__ void __launch_bounds__(kMrBlock) mr_kernel(const uint64_t* __restrict
     return true;
   };
   constexpr uint32_t kWarps = kMrBlock / 32;
-  for (uint32_t c = warp; take(0, c, qd.base2, qd.n_base2); c += kWarps) drain_base2<true>(cand, out, qd, lane);
-  for (uint32_t c = warp; take(1, c, qm.base2, qm.n_base2); c += kWarps) drain_base2<false>(cand, out, qm, lane);
+  for (uint32_t c = warp; take(0, c, qd.base2, qd.n_base2); c += kWarps) drain_base2<true, kCalls>(cand, out, qd, lane);
+  for (uint32_t c = warp; take(1, c, qm.base2, qm.n_base2); c += kWarps)
+    drain_base2<false, kCalls>(cand, out, qm, lane);
   put(2, qd.lucas, qd.n_lucas);
   put(3, qm.lucas, qm.n_lucas);
   __syncthreads();
-  for (uint32_t c = warp; take(2, c, qd.lucas, qd.n_lucas); c += kWarps) drain_lucas<true>(cand, out, qd, lane);
+  for (uint32_t c = warp; take(2, c, qd.lucas, qd.n_lucas); c += kWarps) drain_lucas<true, kCalls>(cand, out, qd, lane);
   for (uint32_t c = kWarps - 1 - warp; take(3, c, qm.lucas, qm.n_lucas); c += kWarps)
-    drain_lucas<false>(cand, out, qm, lane);
+    drain_lucas<false, kCalls>(cand, out, qm, lane);
 }
 
 // Gap proofs: one warp per gap.  Interior integers are split over the lanes; an interior odd
@@ -556,8 +575,8 @@ int launch_mr(const uint64_t* d_n, uint64_t count, uint8_t* d_out, void* stream,
   cudaStream_t s = (cudaStream_t)stream;
   const uint64_t want = (count + kMrBlock - 1) / kMrBlock;
   const uint64_t most = (uint64_t)sm_count * kMrBlocksPerSm;
-  const int grid = (int)(want < most ? want : most);
-  mr_kernel<<<grid, kMrBlock, 0, s>>>(d_n, count, d_out);
+  if (want > most) mr_kernel<true><<<(int)most, kMrBlock, 0, s>>>(d_n, count, d_out);
+  else mr_kernel<false><<<(int)want, kMrBlock, 0, s>>>(d_n, count, d_out);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

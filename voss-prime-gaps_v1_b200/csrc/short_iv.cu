@@ -4,8 +4,7 @@
 // is 5.76e6 reductions however short the interval, and at 10^18 50.8e6.  Testing the
 // interval's wheel integers (coprime to 30) with the deterministic Miller-Rabin kernels costs
 // about 30 products per integer instead, so voss_sieve_intervals sends an interval
-// here when its base primes above the large-prime threshold outnumber mr_route times its
-// length.  The verdicts are exact for every n < 2^64 (mr_kernels.cu), so the statistics are the
+// here when its base primes outnumber mr_route times its length.  The verdicts are exact for every n < 2^64 (mr_kernels.cu), so the statistics are the
 // ones the sieve gives: primes >= 7 of [lo, hi), their gap histogram (bin g/2), first and last
 // prime, and the first maximal gap.
 #include <cuda_runtime.h>
