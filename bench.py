@@ -507,7 +507,7 @@ def run_intervals(a) -> dict:
             "bound": "int", "pairs": work["prepass_pairs"],
             "pairs_per_s": work["prepass_pairs"] / (pre_ms * 1e-3) if pre_ms > 0 else None,
             "ms": pre_ms, "clears": work["prepass_hits"],
-            "issue_frac_ncu": 0.722, "alu_frac_ncu": 0.587,
+            "issue_frac_ncu": 0.674, "alu_frac_ncu": 0.442,
             "source": "issue and ALU-pipe fractions of peak (active cycles) of scatter_large_kernel from the "
                       "committed capture profiles/scatter_large_kernel_intervals.md; one 64-bit reduction per "
                       "(prime, interval) pair, ms includes the batch's copies and bitmap memset"},
