@@ -28,48 +28,68 @@ __global__ void large_gather_kernel(const LargeGapDev* __restrict__ in, const ui
 }
 
 // Lists of up to kSmallSort records, in the stream behind the tiles and before the host knows how
-// many there are: every record counts the positions below its own (they are distinct) and is written
-// to that place.  A block ranks 64 records; its four warp pairs count in a quarter of the keys each,
-// 1024 keys at a time in shared memory.  One launch and no second round trip instead of nine launches
-// after one (a bitonic sort in one block took 8 us for 300 records and 50 us for 2000, on its
-// barriers); beyond 16,384 records the radix sort is the faster one.
-constexpr int kRankBlock = 256, kRankRecords = 64;
-constexpr uint32_t kRankKeys = 1024;  // per round, a quarter of them per warp pair
+// many there are: block b of G places the records of the b-th G-th of [lo, hi).  It goes over all positions once,
+// counts those below its part and lists those in it (a 148th of the records: gaps lie evenly over a
+// range), ranks the list against itself and writes each record to its place.  A part with more
+// records than the list holds is taken in halves; the positions are distinct, so that ends.
+// Bound by the latency of its reads, n per block from L2, where ranking every record against all n was
+// bound by n^2 compares: with the launch's other closing work 17.4 us for 10,602 records, 47.9 before,
+// 17.2 us for 15,826, 64.4 before, 11.4 us for 308, 15.1 before.  One launch and no second round trip
+// instead of nine launches after one; beyond 16,384 records the radix sort.
+constexpr int kRankBlock = 1024;
+constexpr uint32_t kRankList = 2048;
 
-__global__ void __launch_bounds__(kRankBlock) large_rank_kernel(const LargeGapDev* __restrict__ in,
-                                                                const uint32_t* __restrict__ count, uint32_t cap,
-                                                                LargeGapDev* __restrict__ out) {
-  __shared__ __align__(16) unsigned long long s_key[kRankKeys];
-  __shared__ uint32_t s_rank[kRankRecords];
+__global__ void __launch_bounds__(kRankBlock, 1)
+large_rank_kernel(const LargeGapDev* __restrict__ in, const uint32_t* __restrict__ count, uint32_t cap,
+                  unsigned long long lo, unsigned long long hi, LargeGapDev* __restrict__ out) {
+  __shared__ unsigned long long s_key[kRankList];
+  __shared__ uint32_t s_idx[kRankList];
+  __shared__ uint32_t s_below, s_listed;
   const uint32_t n = *count < cap ? *count : cap;
-  const uint32_t r = threadIdx.x % kRankRecords, part = threadIdx.x / kRankRecords;
-  const uint32_t first = kRankRecords * blockIdx.x;
-  if (n > kSmallSort || first >= n) return;
-  const LargeGapDev mine = in[min(first + r, n - 1)];
-  if (threadIdx.x < kRankRecords) s_rank[threadIdx.x] = 0;
-  uint32_t rank = 0;
-  for (uint32_t base = 0; base < n; base += kRankKeys) {
-    __syncthreads();
-#pragma unroll
-    for (uint32_t k = threadIdx.x; k < kRankKeys; k += kRankBlock)
-      s_key[k] = base + k < n ? in[base + k].position : ~0ull;
-    __syncthreads();
-    const ulonglong2* keys = reinterpret_cast<const ulonglong2*>(s_key + part * (kRankKeys / 4));
-#pragma unroll 8
-    for (uint32_t k = 0; k < kRankKeys / 8; ++k) {
-      const ulonglong2 x = keys[k];
-      rank += (x.x < mine.position) + (x.y < mine.position);
+  if (n > kSmallSort) return;
+  const unsigned long long span = hi - lo, width = span / gridDim.x + 1ull, b = blockIdx.x;
+  unsigned long long from = b == 0 ? 0ull : lo + min(b * width, span);
+  const unsigned long long end = b + 1 == gridDim.x ? ~0ull : lo + min((b + 1) * width, span);
+  while (from < end) {
+    unsigned long long to = end;
+    while (true) {
+      __syncthreads();
+      if (threadIdx.x == 0) s_below = s_listed = 0;
+      __syncthreads();
+      uint32_t below = 0;
+#pragma unroll 4
+      for (uint32_t k = threadIdx.x; k < n; k += kRankBlock) {
+        const unsigned long long p = in[k].position;
+        below += p < from;
+        if (p >= from && p < to) {
+          const uint32_t at = atomicAdd(&s_listed, 1u);
+          if (at < kRankList) {
+            s_key[at] = p;
+            s_idx[at] = k;
+          }
+        }
+      }
+      below = __reduce_add_sync(0xFFFFFFFFu, below);
+      if (threadIdx.x % 32 == 0 && below) atomicAdd(&s_below, below);
+      __syncthreads();
+      if (s_listed <= kRankList || to - from < 2ull) break;
+      to = from + (to - from) / 2ull;
     }
+    const uint32_t m = min(s_listed, kRankList);
+    for (uint32_t i = threadIdx.x; i < m; i += kRankBlock) {
+      const unsigned long long mine = s_key[i];
+      uint32_t rank = s_below;
+#pragma unroll 8
+      for (uint32_t k = 0; k < m; ++k) rank += s_key[k] < mine;
+      out[rank] = in[s_idx[i]];
+    }
+    from = to;
   }
-  atomicAdd(&s_rank[r], rank);
-  __syncthreads();
-  if (part == 0 && first + r < n) out[s_rank[r]] = mine;
 }
 
-int launch_large_sort_small(const LargeGapDev* in, const uint32_t* count, uint32_t cap, LargeGapDev* out,
-                            void* stream) {
-  const uint32_t most = cap < kSmallSort ? cap : kSmallSort;
-  large_rank_kernel<<<(most + kRankRecords - 1) / kRankRecords, kRankBlock, 0, (cudaStream_t)stream>>>(in, count, cap, out);
+int launch_large_sort_small(const LargeGapDev* in, const uint32_t* count, uint32_t cap, uint64_t lo, uint64_t hi,
+                            LargeGapDev* out, int sm_count, void* stream) {
+  large_rank_kernel<<<sm_count, kRankBlock, 0, (cudaStream_t)stream>>>(in, count, cap, lo, hi < lo ? lo : hi, out);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -456,7 +456,13 @@ int launch_plan_ws(voss_ctx* c, Workspace& W, const LaunchEvents& E, const RunPl
     return fail(VOSS_ERR_CUDA, "tail launch failed");
   if (want_large) {  // short lists are sorted where the host need not know their length yet
     if ((rc = W.ls_sorted.ensure(sizeof(LargeGapDev) * kSmallSort))) return rc;
-    if (launch_large_sort_small(a.large, a.large_count, a.large_cap, W.ls_sorted.as<LargeGapDev>(), s))
+    uint64_t lo = ~0ull, hi = 0;
+    for (const IntervalDev& I : P.iv) {
+      lo = std::min(lo, I.lo);
+      hi = std::max(hi, I.hi);
+    }
+    if (launch_large_sort_small(a.large, a.large_count, a.large_cap, lo, hi, W.ls_sorted.as<LargeGapDev>(), c->sm_count,
+                                s))
       return fail(VOSS_ERR_CUDA, "large-gap sort launch failed");
     ++k;
   }

@@ -218,9 +218,10 @@ int launch_scatter_large(const uint32_t* primes, uint32_t j0, uint32_t j1, const
 int sieve_kernel_attrs(int block, size_t smem, int* max_ctas_per_sm);
 // Large-gap list sorted by position on the device (large_sort.cu): keys and idx hold 2n entries.
 constexpr uint32_t kSmallSort = 16384;
-// Sorts min(*count, cap) records when they are at most kSmallSort (else does nothing).
-int launch_large_sort_small(const LargeGapDev* in, const uint32_t* count, uint32_t cap, LargeGapDev* out,
-                            void* stream);
+// Sorts min(*count, cap) records with distinct positions in [lo, hi) when they are at most kSmallSort
+// (else does nothing).
+int launch_large_sort_small(const LargeGapDev* in, const uint32_t* count, uint32_t cap, uint64_t lo, uint64_t hi,
+                            LargeGapDev* out, int sm_count, void* stream);
 size_t large_sort_temp_bytes(uint32_t n, int end_bit);
 int launch_large_sort(const LargeGapDev* in, uint32_t n, int end_bit, unsigned long long* keys, uint32_t* idx,
                       void* temp, size_t temp_bytes, LargeGapDev* out, int sm_count, void* stream);
