@@ -2,11 +2,11 @@
 //
 // Sieving [lo, hi) reduces lo modulo every base prime up to isqrt(hi - 1): at hi = 10^16 that
 // is 5.76e6 reductions however short the interval, and at 10^18 50.8e6.  Testing the
-// interval's wheel integers (coprime to 30) with the deterministic Miller-Rabin kernels costs
+// interval's wheel integers (coprime to 30) with the deterministic primality kernel costs
 // about 30 products per integer instead, so voss_sieve_intervals sends an interval
-// here when its base primes outnumber mr_route times its length.  The verdicts are exact for every n < 2^64 (mr_kernels.cu), so the statistics are the
-// ones the sieve gives: primes >= 7 of [lo, hi), their gap histogram (bin g/2), first and last
-// prime, and the first maximal gap.
+// here when its base primes outnumber mr_route times its length.  The verdicts are exact for
+// every n < 2^64 (mr_kernels.cu), so the statistics are the ones the sieve gives: primes >= 7 of
+// [lo, hi), their gap histogram (bin g/2), first and last prime, and the first maximal gap.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -27,7 +27,8 @@ __device__ __forceinline__ uint64_t wheel_value(const ShortInterval& I, uint32_t
 }
 
 // The intervals are worked on in segments of kShortSeg candidates, a block each, so that one long
-// interval fills the GPU as well as many short ones.  Segment b belongs to the last interval with seg_begin <= b; every interval has at least one.
+// interval fills the GPU as well as many short ones.  Segment b belongs to the last interval with
+// seg_begin <= b; every interval has at least one.
 __device__ __forceinline__ uint32_t interval_of(const ShortInterval* __restrict__ iv, uint32_t n_iv, uint32_t b) {
   uint32_t lo = 0, hi = n_iv;
   while (hi - lo > 1u) {
