@@ -428,6 +428,7 @@ __global__ void __launch_bounds__(kMrBlock, kCalls ? 5 : 1) mr_kernel(const uint
   if (threadIdx.x < 4) s_n[threadIdx.x] = 0;
   __syncthreads();
   auto put = [&](int k, const uint32_t* q, uint32_t nq) {
+    __syncwarp();  // the entries come from other lanes (queue_add); its ballot does not order shared memory
     uint32_t at = 0;
     if (lane == 0 && nq) at = atomicAdd(&s_n[k], nq);
     at = __shfl_sync(0xFFFFFFFFu, at, 0);
