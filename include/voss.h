@@ -200,8 +200,7 @@ VOSS_API int voss_mr_verify_device(voss_ctx* ctx, const uint64_t* d_n, uint64_t 
  * It takes no context and allocates nothing; it needs no scratch memory either, so
  *   - count may not exceed 4194304 (1 << 22) per call; larger counts return VOSS_ERR_ARG;
  *   - calls may overlap on the GPU (different streams or host threads);
- *   - the first call on a device uploads the trial-division constant tables on the calling
- *     thread's current device; make that first call before any stream capture.
+ *   - the first call on a device loads the kernels there; make it before any stream capture.
  * d_n and d_is_prime are device pointers on the current device; `stream` is a cudaStream_t or
  * NULL for the legacy default stream.  The call is asynchronous on `stream`. */
 VOSS_API int voss_mr_verify_noalloc(const uint64_t* d_n, uint64_t count, uint8_t* d_is_prime,

@@ -7,11 +7,10 @@
 // zeros and the 64-bit big-endian bit length; the 64-round compression with the message
 // schedule kept in a 16-word ring; initial hash value and round constants taken as the first 32
 // bits of the fractional parts of the square roots of the first 8 primes and of the cube roots of
-// the first 64 primes, which the host computes exactly in integer arithmetic at set-up.
+// the first 64 primes, computed exactly in integer arithmetic at compile time.
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstdint>
 #include <cstring>
 
@@ -20,13 +19,8 @@
 
 namespace voss {
 
-__constant__ uint32_t c_sha_k[64];
-__constant__ uint32_t c_sha_h0[8];
-
-static std::atomic<uint64_t> g_sha_ready{0};  // per device ordinal
-
 // floor(x^(1/k)) for k = 2, 3 and x < 2^120, by bisection on 128-bit integers.
-static uint64_t iroot(unsigned __int128 x, int k) {
+constexpr uint64_t iroot(unsigned __int128 x, int k) {
   uint64_t lo = 0, hi = 1ull << 41;
   while (hi - lo > 1) {
     const uint64_t mid = lo + (hi - lo) / 2;
@@ -37,27 +31,27 @@ static uint64_t iroot(unsigned __int128 x, int k) {
   return lo;
 }
 
-static int ensure_sha_tables() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-  const uint64_t bit = 1ull << dev;
-  if (g_sha_ready.load() & bit) return 0;
-  uint32_t primes[64];
+// Constant-initialised: the tables come with the kernel's module, so that no launch on any stream can run
+// ahead of an upload.
+struct ShaTables {
+  uint32_t k[64], h0[8];
+};
+
+constexpr ShaTables make_sha_tables() {
+  uint32_t primes[64] = {};
   for (int n = 2, c = 0; c < 64; ++n) {
     bool pr = true;
     for (int d = 2; d * d <= n; ++d)
       if (n % d == 0) pr = false;
     if (pr) primes[c++] = (uint32_t)n;
   }
-  uint32_t k[64], h0[8];
+  ShaTables t{};
   // fractional bits: floor(p^(1/3) * 2^32) = floor((p * 2^96)^(1/3)); keep the low 32 bits
-  for (int i = 0; i < 64; ++i) k[i] = (uint32_t)iroot((unsigned __int128)primes[i] << 96, 3);
-  for (int i = 0; i < 8; ++i) h0[i] = (uint32_t)iroot((unsigned __int128)primes[i] << 64, 2);
-  if (cudaMemcpyToSymbol(c_sha_k, k, sizeof(k)) != cudaSuccess) return -1;
-  if (cudaMemcpyToSymbol(c_sha_h0, h0, sizeof(h0)) != cudaSuccess) return -1;
-  g_sha_ready.fetch_or(bit);
-  return 0;
+  for (int i = 0; i < 64; ++i) t.k[i] = (uint32_t)iroot((unsigned __int128)primes[i] << 96, 3);
+  for (int i = 0; i < 8; ++i) t.h0[i] = (uint32_t)iroot((unsigned __int128)primes[i] << 64, 2);
+  return t;
 }
+__constant__ ShaTables c_sha = make_sha_tables();
 
 __device__ __forceinline__ uint32_t rotr(uint32_t x, uint32_t n) { return __funnelshift_r(x, x, n); }
 
@@ -70,7 +64,7 @@ __global__ void sha256_batch_kernel(const uint8_t* __restrict__ data, const uint
     const uint8_t* m = data + base;
     uint32_t h[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) h[j] = c_sha_h0[j];
+    for (int j = 0; j < 8; ++j) h[j] = c_sha.h0[j];
     const uint64_t nblk = (len + 9 + 63) / 64;
     const uint64_t bits = len * 8;
     for (uint64_t blk = 0; blk < nblk; ++blk) {
@@ -103,7 +97,7 @@ __global__ void sha256_batch_kernel(const uint8_t* __restrict__ data, const uint
         }
         const uint32_t S1 = rotr(e, 6) ^ rotr(e, 11) ^ rotr(e, 25);
         const uint32_t ch = (e & f) ^ (~e & g);
-        const uint32_t t1 = hh + S1 + ch + c_sha_k[t] + w[t & 15];
+        const uint32_t t1 = hh + S1 + ch + c_sha.k[t] + w[t & 15];
         const uint32_t S0 = rotr(a, 2) ^ rotr(a, 13) ^ rotr(a, 22);
         const uint32_t mj = (a & b) ^ (a & c) ^ (b & c);
         const uint32_t t2 = S0 + mj;
@@ -155,7 +149,6 @@ VOSS_API int voss_sha256_batch(voss_ctx* c, const uint8_t* data, const uint64_t*
   const uint64_t bytes = offsets[count];
   if (bytes && !data) return fail(VOSS_ERR_ARG, "NULL data");
   cudaSetDevice(c->device);
-  if (voss::ensure_sha_tables()) return fail(VOSS_ERR_CUDA, "SHA-256 constant upload failed");
   cudaStream_t s = c->stream;
   Workspace& W = c->ws;  // context-owned, grow-only buffers
   int rc;

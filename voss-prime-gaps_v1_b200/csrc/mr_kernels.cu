@@ -23,7 +23,6 @@
 // test and size, and each time a queue holds 32 they are tested together, a lane each.
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <mutex>
@@ -34,12 +33,25 @@
 
 namespace voss {
 
-__constant__ uint64_t c_base_inv[12];  // B^-1 mod 2^64 (odd B), for the divisibility test
-__constant__ uint64_t c_base_lim[12];  // floor((2^64-1)/B)
+// Divisibility of n by the odd bases B (index 0, for 2, is not used): n B^-1 mod 2^64 is at most
+// floor((2^64-1)/B) exactly when B | n.  Constant-initialised: the tables come with the kernel's module, so that
+// no launch on any stream can run ahead of an upload.
+struct TrialTables {
+  uint64_t inv[12], lim[12];
+};
 
-// Constant memory is per device: the tables are uploaded once for each device ordinal.
-static std::atomic<uint64_t> g_mr_ready{0};
-static const uint64_t kBases[12] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37};
+constexpr TrialTables make_trial_tables() {
+  constexpr uint64_t bases[12] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37};
+  TrialTables t{};
+  for (int i = 1; i < 12; ++i) {
+    uint64_t x = bases[i];  // its own inverse mod 2^3
+    for (int k = 0; k < 5; ++k) x *= 2ull - bases[i] * x;
+    t.inv[i] = x;
+    t.lim[i] = ~0ull / bases[i];
+  }
+  return t;
+}
+__constant__ TrialTables c_trial = make_trial_tables();
 
 struct Mont {
   uint64_t n, inv, ninv, one, mone;  // inv = n^-1, ninv = -n^-1 (mod 2^64); one = 2^64 mod n, mone = n - one
@@ -108,7 +120,7 @@ __device__ __forceinline__ int trial_phase(uint64_t n) {
     const uint64_t B = i == 1 ? 3 : i == 2 ? 5 : i == 3 ? 7 : i == 4 ? 11 : i == 5 ? 13 : i == 6 ? 17
                      : i == 7 ? 19 : i == 8 ? 23 : i == 9 ? 29 : i == 10 ? 31 : 37;
     if (n == B) return 1;
-    if (n * c_base_inv[i] <= c_base_lim[i]) return 0;
+    if (n * c_trial.inv[i] <= c_trial.lim[i]) return 0;
   }
   if (n < 1681) return 1;
   return -1;
@@ -546,31 +558,7 @@ __global__ void __launch_bounds__(kProveBlock) prove_interior_kernel(const uint6
   }
 }
 
-static int ensure_mr_tables() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-  const uint64_t bit = 1ull << dev;
-  if (g_mr_ready.load() & bit) return 0;
-  uint64_t inv[12], lim[12];
-  for (int i = 0; i < 12; ++i) {
-    const uint64_t b = kBases[i];
-    uint64_t x = b;
-    if (b & 1) {
-      for (int k = 0; k < 5; ++k) x *= 2ull - b * x;
-    } else {
-      x = 0;
-    }
-    inv[i] = x;
-    lim[i] = ~0ull / b;
-  }
-  if (cudaMemcpyToSymbol(c_base_inv, inv, sizeof(inv)) != cudaSuccess) return -1;
-  if (cudaMemcpyToSymbol(c_base_lim, lim, sizeof(lim)) != cudaSuccess) return -1;
-  g_mr_ready.fetch_or(bit);
-  return 0;
-}
-
 int launch_mr(const uint64_t* d_n, uint64_t count, uint8_t* d_out, void* stream, int sm_count) {
-  if (ensure_mr_tables()) return -1;
   if (count == 0) return 0;
   if (count > 0xFFFFFFFFull) return -1;
   cudaStream_t s = (cudaStream_t)stream;
@@ -583,7 +571,6 @@ int launch_mr(const uint64_t* d_n, uint64_t count, uint8_t* d_out, void* stream,
 
 int launch_prove_gaps(const uint64_t* d_p_after, const int32_t* d_gap, uint64_t count, uint8_t* d_ok,
                       uint64_t* d_ends, uint8_t* d_ends_ok, void* stream, int sm_count) {
-  if (ensure_mr_tables()) return -1;
   if (count == 0) return 0;
   if (count > 0x7FFFFFFFull) return -1;
   cudaStream_t s = (cudaStream_t)stream;

@@ -28,7 +28,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <type_traits>
@@ -38,28 +37,86 @@
 
 namespace voss {
 
+// The wheel tables are constant-initialised: they come with the kernels' module, so that no launch on any
+// stream can run ahead of an upload.
+template <class T, int N>
+struct Table {
+  T v[N];
+};
+
+constexpr uint32_t wheel_residue(int o) { return (uint32_t)(kW30Packed >> (8 * o)) & 0xFFu; }
+
+// residue r (mod 30) -> wheel bit index, or -1 when gcd(r, 30) > 1.
+constexpr Table<int8_t, 32> make_res_bit() {
+  Table<int8_t, 32> t{};
+  for (int r = 0; r < 32; ++r) t.v[r] = -1;
+  for (int o = 0; o < 8; ++o) t.v[wheel_residue(o)] = (int8_t)o;
+  return t;
+}
+constexpr Table<int8_t, 32> kResBit = make_res_bit();
+__constant__ Table<int8_t, 32> c_res_bit = make_res_bit();
+
 // [bi*8 + o]: for a prime p = 30a + b (b = W30[bi]) and multiplier residue w = W30[o],
 // p*w = 30*(a*w + D) + W30[B] with D = floor(b*w/30), stored as D | (B << 5).
-__constant__ uint8_t c_wheel_step[64];
-// residue r (mod 30) -> wheel bit index, or -1 when gcd(r, 30) > 1.
-__constant__ int8_t c_res_bit[32];
+constexpr Table<uint8_t, 64> make_wheel_step() {
+  Table<uint8_t, 64> t{};
+  for (int i = 0; i < 64; ++i) {
+    const uint32_t bw = wheel_residue(i / 8) * wheel_residue(i % 8);
+    t.v[i] = (uint8_t)(bw / 30u | (uint32_t)kResBit.v[bw % 30u] << 5);
+  }
+  return t;
+}
+__constant__ Table<uint8_t, 64> c_wheel_step = make_wheel_step();
+
 // Wheel walk of a prime p = 30a + W30[bi] over its multiples p*m with gcd(m, 30) = 1.
 // [bi*30 + t]: t = (offset of the first multiple of p at or above a tile's start) mod 30 gives
 // m mod 30 = t * p^-1 (mod 30); stored: (steps to the next m coprime to 30) | (its wheel index << 3).
-__constant__ uint8_t c_walk_start[240];
+constexpr Table<uint8_t, 240> make_walk_start() {
+  Table<uint8_t, 240> t{};
+  for (int bi = 0; bi < 8; ++bi) {
+    uint32_t pinv = 1;
+    while (wheel_residue(bi) * pinv % 30u != 1u) ++pinv;
+    for (uint32_t k = 0; k < 30; ++k) {
+      const uint32_t u = k * pinv % 30u;
+      uint32_t adv = 0;
+      while (kResBit.v[(u + adv) % 30u] < 0) ++adv;
+      t.v[bi * 30 + (int)k] = (uint8_t)(adv | (uint32_t)kResBit.v[(u + adv) % 30u] << 3);
+    }
+  }
+  return t;
+}
+__constant__ Table<uint8_t, 240> c_walk_start = make_walk_start();
+
 // [bi*8 + j]: from m = 30c + W30[j] to the next coprime m, the byte index of p*m grows by
 // a*gap_j + corr (gap_j = W30[j+1] - W30[j], W30[8] = 31); stored: .x = ~(1 << bit of p*m)
 // (rotated left by 8 * (byte & 3) it is the clear mask of that byte's lane in its word; the
 // funnel shift takes its count mod 32, so byte << 3 is that rotation),
 // .y = gap_j | corr << 16.
-__constant__ uint2 c_walk_step[64];
+constexpr Table<uint2, 64> make_walk_step() {
+  Table<uint2, 64> t{};
+  for (int bi = 0; bi < 8; ++bi)
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t w = wheel_residue(bi), m = wheel_residue(j), next = j < 7 ? wheel_residue(j + 1) : 31u;
+      t.v[bi * 8 + j].x = ~(1u << kResBit.v[w * m % 30u]);
+      t.v[bi * 8 + j].y = (next - m) | (w * next / 30u - w * m / 30u) << 16;
+    }
+  return t;
+}
+__constant__ Table<uint2, 64> c_walk_step = make_walk_step();
+
 // [bi*8 + j], for the primes that a tile takes by class: .x = D_j - D_{j-1} (D_j = floor(W30[bi] W30[j] / 30),
 // D_{-1} = 0), .y = the bit of W30[bi] * W30[j].
-__constant__ uint2 c_cls_step[64];
-static int ensure_tables();
-
-// Constant memory is per device: the tables are uploaded once for each device ordinal.
-static std::atomic<uint64_t> g_tables_ready{0};
+constexpr Table<uint2, 64> make_cls_step() {
+  Table<uint2, 64> t{};
+  for (int bi = 0; bi < 8; ++bi)
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t w = wheel_residue(bi), m = wheel_residue(j);
+      t.v[bi * 8 + j].x = w * m / 30u - (j ? w * wheel_residue(j - 1) / 30u : 0u);
+      t.v[bi * 8 + j].y = (uint32_t)kResBit.v[w * m % 30u];
+    }
+  return t;
+}
+__constant__ Table<uint2, 64> c_cls_step = make_cls_step();
 
 __device__ __forceinline__ uint32_t w30(uint32_t o) {
   return (uint32_t)((kW30Packed >> (8u * o)) & 0xFFu);
@@ -812,8 +869,8 @@ sieve_tiles_kernel(SieveArgs a) {
 
   const int tid = threadIdx.x, lane = tid & 31;
   for (uint32_t i = tid; i < kPreWords; i += BLOCK) pre[i] = a.pretab[i];
-  if (tid < 64) s_step[tid] = c_wheel_step[tid];
-  if (tid < 32) s_rb[tid] = c_res_bit[tid];
+  if (tid < 64) s_step[tid] = c_wheel_step.v[tid];
+  if (tid < 32) s_rb[tid] = c_res_bit.v[tid];
   if (tid < 32) s_pos[tid] = 30u * ((uint32_t)tid >> 3) + w30((uint32_t)tid & 7u);
   if (!EMIT)
     for (uint32_t i = tid; i < (uint32_t)kSmCounters; i += BLOCK) cnt[i] = 0;
@@ -1006,7 +1063,7 @@ sieve_tiles_kernel(SieveArgs a) {
           ClassStep C;
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const uint2 e = c_cls_step[8u * c + j];
+            const uint2 e = c_cls_step.v[8u * c + j];
             C.corr[j] = e.x;
             C.bit[j] = e.y;
           }
@@ -1372,7 +1429,7 @@ __device__ __forceinline__ void tile_seam(const SieveArgs& a, const IntervalDev&
   const bool crossing = iv.seg_k && ((lo_p / 30ull) / iv.seg_k != (hi_p / 30ull) / iv.seg_k);
   unsigned long long* acc = a.acc + (size_t)ivx * kAccStride;
   if (g < 100 && !crossing) {
-    const uint32_t o_prev = (uint32_t)c_res_bit[lo_p % 30ull];
+    const uint32_t o_prev = (uint32_t)c_res_bit.v[lo_p % 30ull];
     atomicAdd(acc + kAccModq + o_prev * kModqBins + (g >> 1), 1ull);
   } else if (g < 2ull * kHistBins) {
     atomicAdd(acc + kAccHist + (g >> 1), 1ull);
@@ -1570,9 +1627,9 @@ __global__ void __launch_bounds__(kScatterBlock) scatter_large_kernel(const uint
   __shared__ int8_t s_rb[32];
   __shared__ uint8_t s_wstart[240];
   __shared__ uint2 s_wstep[64];
-  if (threadIdx.x < 32) s_rb[threadIdx.x] = c_res_bit[threadIdx.x];
-  if (threadIdx.x < 240) s_wstart[threadIdx.x] = c_walk_start[threadIdx.x];
-  if (threadIdx.x < 64) s_wstep[threadIdx.x] = c_walk_step[threadIdx.x];
+  if (threadIdx.x < 32) s_rb[threadIdx.x] = c_res_bit.v[threadIdx.x];
+  if (threadIdx.x < 240) s_wstart[threadIdx.x] = c_walk_start.v[threadIdx.x];
+  if (threadIdx.x < 64) s_wstep[threadIdx.x] = c_walk_step.v[threadIdx.x];
   for (uint32_t i = threadIdx.x; i < n_iv; i += blockDim.x) s_iv[i] = iv[i];
   __syncthreads();
   const uint32_t lane = threadIdx.x & 31u;
@@ -1644,7 +1701,6 @@ __global__ void __launch_bounds__(kScatterBlock) scatter_large_kernel(const uint
 
 int launch_scatter_large(const uint32_t* primes, uint32_t j0, uint32_t j1, const IntervalScatter* iv, uint32_t n_iv,
                          uint32_t* gbm, int sm_count, void* stream, uint32_t* kernels) {
-  if (ensure_tables()) return -1;
   if (j1 <= j0 || n_iv == 0) return 0;
   const uint64_t want = ((uint64_t)(j1 - j0) + kScatterBlock - 1) / kScatterBlock;
   const int grid = (int)(want < (uint64_t)sm_count * 4 ? want : (uint64_t)sm_count * 4);
@@ -1687,51 +1743,6 @@ int read_phase_cycles(unsigned long long* out, int n, bool reset) {
   return 0;
 }
 #endif
-static const int kW30h[8] = {1, 7, 11, 13, 17, 19, 23, 29};
-
-static int ensure_tables() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-  const uint64_t bit = 1ull << dev;
-  if (g_tables_ready.load() & bit) return 0;
-  uint8_t step[64];
-  int8_t rb[32];
-  for (int r = 0; r < 32; ++r) rb[r] = -1;
-  for (int i = 0; i < 8; ++i) rb[kW30h[i]] = (int8_t)i;
-  for (int bi = 0; bi < 8; ++bi)
-    for (int o = 0; o < 8; ++o) {
-      const int bw = kW30h[bi] * kW30h[o];
-      step[bi * 8 + o] = (uint8_t)((bw / 30) | (rb[bw % 30] << 5));
-    }
-  uint8_t wstart[240];
-  uint2 wstep[64], cls[64];
-  for (int bi = 0; bi < 8; ++bi) {
-    int pinv = 1;
-    while ((kW30h[bi] * pinv) % 30 != 1) ++pinv;
-    for (int t = 0; t < 30; ++t) {
-      const int u = (t * pinv) % 30;
-      int adv = 0;
-      while (rb[(u + adv) % 30] < 0) ++adv;
-      wstart[bi * 30 + t] = (uint8_t)(adv | (rb[(u + adv) % 30] << 3));
-    }
-    for (int j = 0; j < 8; ++j) {
-      const int w = kW30h[bi];
-      const int d0 = (w * kW30h[j]) / 30;
-      const int gap = (j < 7 ? kW30h[j + 1] : 31) - kW30h[j];
-      const int corr = j < 7 ? (w * kW30h[j + 1]) / 30 - d0 : w + 0 - d0;  // j = 7: next m is 30(c+1) + 1
-      cls[bi * 8 + j] = make_uint2((uint32_t)(d0 - (j ? (w * kW30h[j - 1]) / 30 : 0)), (uint32_t)rb[(w * kW30h[j]) % 30]);
-      wstep[bi * 8 + j] = make_uint2(~(1u << rb[(w * kW30h[j]) % 30]), (uint32_t)gap | ((uint32_t)corr << 16));
-    }
-  }
-  if (cudaMemcpyToSymbol(c_walk_start, wstart, sizeof(wstart)) != cudaSuccess) return -1;
-  if (cudaMemcpyToSymbol(c_walk_step, wstep, sizeof(wstep)) != cudaSuccess) return -1;
-  if (cudaMemcpyToSymbol(c_cls_step, cls, sizeof(cls)) != cudaSuccess) return -1;
-  if (cudaMemcpyToSymbol(c_wheel_step, step, sizeof(step)) != cudaSuccess) return -1;
-  if (cudaMemcpyToSymbol(c_res_bit, rb, sizeof(rb)) != cudaSuccess) return -1;
-  g_tables_ready.fetch_or(bit);
-  return 0;
-}
-
 void build_presieve_tables(uint32_t* out) {
   static const uint32_t groups[kPreGroups][3] = {{7, 11, 13}, {17, 19, 0}, {23, 29, 0}, {31, 0, 0}};
   for (int g = 0; g < kPreGroups; ++g) {
@@ -1743,7 +1754,7 @@ void build_presieve_tables(uint32_t* out) {
           const uint64_t k = 4ull * j + jb;  // byte index modulo P
           for (int q = 0; q < 3 && groups[g][q]; ++q) {
             const uint32_t p = groups[g][q];
-            if ((30ull * k + kW30h[o]) % p == 0) m &= ~(1u << (8 * jb + o));
+            if ((30ull * k + wheel_residue((int)o)) % p == 0) m &= ~(1u << (8 * jb + o));
           }
         }
       out[kPreOff[g] + j] = m;
@@ -1764,7 +1775,6 @@ static int set_attrs(size_t smem) {
 }
 
 int sieve_kernel_attrs(int block, size_t smem, int* max_ctas_per_sm) {
-  if (ensure_tables()) return -1;
   int rc = 0, n = 0;
   if (block == 512) {
     rc |= set_attrs<512, false>(smem) | set_attrs<512, true>(smem);
@@ -1780,7 +1790,6 @@ int sieve_kernel_attrs(int block, size_t smem, int* max_ctas_per_sm) {
 }
 
 int launch_sieve_stats(const SieveArgs& a, int grid, int block, size_t smem, void* stream) {
-  if (ensure_tables()) return -1;
   cudaStream_t s = (cudaStream_t)stream;
   if (block == 512) sieve_tiles_kernel<512, false><<<grid, 512, smem, s>>>(a);
   else if (block == 1024) sieve_tiles_kernel<1024, false><<<grid, 1024, smem, s>>>(a);
@@ -1789,7 +1798,6 @@ int launch_sieve_stats(const SieveArgs& a, int grid, int block, size_t smem, voi
 }
 
 int launch_sieve_emit(const SieveArgs& a, int grid, int block, size_t smem, void* stream) {
-  if (ensure_tables()) return -1;
   cudaStream_t s = (cudaStream_t)stream;
   if (block == 512) sieve_tiles_kernel<512, true><<<grid, 512, smem, s>>>(a);
   else if (block == 1024) sieve_tiles_kernel<1024, true><<<grid, 1024, smem, s>>>(a);

@@ -152,6 +152,15 @@ int apply_tuning(voss_ctx* c, const voss_tuning& t0) {
 }
 
 
+// A table of the context into device memory, complete on return.  (A plain cudaMemcpy from pageable memory may
+// return with its last part still on the way, and the context's streams do not wait for the legacy
+// stream: the first launch could read the table before it is there.)
+int upload(voss_ctx* c, const DevBuf& dst, const void* src, size_t bytes) {
+  CUDA_TRY(cudaMemcpyAsync(dst.p, src, bytes, cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(cudaStreamSynchronize(c->stream));
+  return VOSS_OK;
+}
+
 // The primes below kClsLimit grouped by residue class mod 30 (SieveArgs::cls_primes).
 int upload_class_primes(voss_ctx* c) {
   int idx[30];
@@ -180,10 +189,10 @@ int upload_class_primes(voss_ctx* c) {
   if ((rc = c->d_cls_primes.ensure(all.size() * sizeof(uint32_t))) || (rc = c->d_cls_inv.ensure(inv.size() * sizeof(double))) ||
       (rc = c->d_cls_index.ensure(index.size() * sizeof(uint32_t))))
     return rc;
-  CUDA_TRY(cudaMemcpy(c->d_cls_primes.p, all.data(), all.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(c->d_cls_inv.p, inv.data(), inv.size() * sizeof(double), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(c->d_cls_index.p, index.data(), index.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  return VOSS_OK;
+  if ((rc = upload(c, c->d_cls_primes, all.data(), all.size() * sizeof(uint32_t))) ||
+      (rc = upload(c, c->d_cls_inv, inv.data(), inv.size() * sizeof(double))))
+    return rc;
+  return upload(c, c->d_cls_index, index.data(), index.size() * sizeof(uint32_t));
 }
 
 TileShape default_shape(const voss_ctx* c) {
@@ -1092,14 +1101,10 @@ VOSS_API int voss_ctx_create(int device, uint64_t max_hi, voss_ctx** out) {
   for (size_t i = 0; i < c->primes.size(); ++i) magic[i] = ~0ull / c->primes[i];
   std::vector<uint32_t> pre(kPreWords);
   build_presieve_tables(pre.data());
-  if (!c->primes.empty()) {
-    if (cudaMemcpy(c->d_primes.p, c->primes.data(), c->primes.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(c->d_magic.p, magic.data(), c->primes.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess)
-      return bail(fail(VOSS_ERR_CUDA, "base prime upload failed"));
-  }
-  if (cudaMemcpy(c->d_pretab.p, pre.data(), kPreWords * 4, cudaMemcpyHostToDevice) != cudaSuccess)
-    return bail(fail(VOSS_ERR_CUDA, "presieve table upload failed"));
-  if ((rc = upload_class_primes(c))) return bail(rc);
+  if ((!c->primes.empty() && ((rc = upload(c, c->d_primes, c->primes.data(), c->primes.size() * 4)) ||
+                              (rc = upload(c, c->d_magic, magic.data(), c->primes.size() * 8)))) ||
+      (rc = upload(c, c->d_pretab, pre.data(), kPreWords * 4)) || (rc = upload_class_primes(c)))
+    return bail(rc);
   voss_tuning t{};
   if ((rc = apply_tuning(c, t))) return bail(rc);
   if (const char* lim = std::getenv("VOSS_STAGE_LIMIT")) {
