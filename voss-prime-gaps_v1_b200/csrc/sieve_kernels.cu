@@ -1766,27 +1766,36 @@ size_t sieve_smem_bytes(uint32_t tile_words) {
   return (size_t)(tile_words + kSpareWords + kPreWords + kSmCounters) * sizeof(uint32_t);
 }
 
+// The largest dynamic shared memory of a kernel is an attribute of the device's function, which all
+// contexts share: it goes to all that a block can have, whatever tile the calling context uses, so that no
+// context lowers it for another.  A tile beyond it is refused without a failing CUDA call, whose error the next
+// launch would report as its own.
 template <int BLOCK, bool EMIT>
-static int set_attrs(size_t smem) {
+static int allow_smem(size_t smem) {
   auto fn = sieve_tiles_kernel<BLOCK, EMIT>;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  int dev = 0, most = 0;
+  cudaFuncAttributes fa;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaFuncGetAttributes(&fa, fn) != cudaSuccess ||
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
     return -1;
-  return 0;
+  most -= (int)fa.sharedSizeBytes;
+  if (smem > (size_t)std::max(most, 0)) return -1;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess ? 0 : -1;
+}
+
+template <int BLOCK>
+static int block_attrs(size_t smem, int* max_ctas_per_sm) {
+  if (allow_smem<BLOCK, false>(smem) || allow_smem<BLOCK, true>(smem)) return -1;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(max_ctas_per_sm, sieve_tiles_kernel<BLOCK, false>, BLOCK,
+                                                       smem) == cudaSuccess
+             ? 0
+             : -1;
 }
 
 int sieve_kernel_attrs(int block, size_t smem, int* max_ctas_per_sm) {
-  int rc = 0, n = 0;
-  if (block == 512) {
-    rc |= set_attrs<512, false>(smem) | set_attrs<512, true>(smem);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sieve_tiles_kernel<512, false>, 512, smem) != cudaSuccess) rc = -1;
-  } else if (block == 1024) {
-    rc |= set_attrs<1024, false>(smem) | set_attrs<1024, true>(smem);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sieve_tiles_kernel<1024, false>, 1024, smem) != cudaSuccess) rc = -1;
-  } else {
-    return -1;
-  }
-  if (max_ctas_per_sm) *max_ctas_per_sm = n;
-  return rc;
+  if (block == 512) return block_attrs<512>(smem, max_ctas_per_sm);
+  if (block == 1024) return block_attrs<1024>(smem, max_ctas_per_sm);
+  return -1;
 }
 
 int launch_sieve_stats(const SieveArgs& a, int grid, int block, size_t smem, void* stream) {
