@@ -112,7 +112,9 @@ typedef struct voss_interval_stats {
 } voss_interval_stats;
 
 /* Sieve tuning; zero fields take the library's defaults.  While block_threads, chunk_words, coop_div
- * and mult_factor are all zero, launches too small for the default tile choose a smaller one. */
+ * and mult_factor are all zero, launches too small for the default tile choose a smaller one.
+ * voss_ctx_get_tuning reports the default tile's values then; all four set to those mean the same as all
+ * four zero, so a tuning that was read can be set again. */
 typedef struct voss_tuning {
   uint32_t block_threads;   /* 512 or 1024 */
   uint32_t chunk_words;     /* odd; a tile is block_threads * chunk_words 32-bit words */

@@ -1,0 +1,30 @@
+"""Saving a context's tuning and setting it again keeps the automatic tile shape.  The shape shows in the number
+of kernels of a short launch near 10^12: the chosen small tile comes with a pre-pass, the fixed one
+without."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+LO, HI = 10**12 - 10**7, 10**12
+
+
+def kernels(ctx):
+    ctx.sieve_range(LO, HI)
+    return ctx.last_phase_ms()[3]
+
+
+def test_the_automatic_shape_survives_a_round_trip():
+    import voss
+    with voss.Context(10**12) as ctx:
+        automatic = kernels(ctx)
+        ctx.set_tuning(chunk_words=49)
+        assert kernels(ctx) != automatic  # what this test tells the two by
+        t0 = ctx.set_tuning()
+        ctx.set_tuning(**t0)
+        assert kernels(ctx) == automatic
+        ctx.set_tuning(**{**t0, "mr_route": 0xFFFFFFFF})  # another field changed alone
+        assert kernels(ctx) == automatic
+        ctx.set_tuning(**{**t0, "coop_div": 64})  # one of the shape's own
+        assert kernels(ctx) != automatic
+        ctx.set_tuning(**t0)
+        assert kernels(ctx) == automatic and ctx.tuning() == t0

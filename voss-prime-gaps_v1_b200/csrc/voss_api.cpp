@@ -116,13 +116,20 @@ int set_error(int code, const char* msg) { return voss_host::fail(code, "%s", ms
 
 namespace voss_host {
 
+// The shape of long runs, which a launch too small for it replaces (choose_shape) while the shape is automatic.
+constexpr uint32_t kAutoBlock = 1024, kAutoChunk = 49, kAutoCoopDiv = 80, kAutoMultFactor = 8;
+
 int apply_tuning(voss_ctx* c, const voss_tuning& t0) {
   voss_tuning t = t0;
-  const bool auto_shape = !t.block_threads && !t.chunk_words && !t.coop_div && !t.mult_factor;
-  if (!t.block_threads) t.block_threads = 1024;
-  if (!t.chunk_words) t.chunk_words = t.block_threads == 1024 ? 49 : 45;
-  if (!t.coop_div) t.coop_div = 80;
-  if (!t.mult_factor) t.mult_factor = 8;
+  // Automatic: none of the four fields set, or all four as get_tuning reports the automatic shape, so that
+  // a caller may save a tuning, change another field of it and set it again.
+  const bool auto_shape = (!t.block_threads && !t.chunk_words && !t.coop_div && !t.mult_factor) ||
+                          (t.block_threads == kAutoBlock && t.chunk_words == kAutoChunk &&
+                           t.coop_div == kAutoCoopDiv && t.mult_factor == kAutoMultFactor);
+  if (!t.block_threads) t.block_threads = kAutoBlock;
+  if (!t.chunk_words) t.chunk_words = t.block_threads == kAutoBlock ? kAutoChunk : 45;
+  if (!t.coop_div) t.coop_div = kAutoCoopDiv;
+  if (!t.mult_factor) t.mult_factor = kAutoMultFactor;
   if (!t.walk_sixteenths) t.walk_sixteenths = 2;
   // the 4096-interval batch (10^4..10^8 long, up to 10^16) takes 20.4 ms from 15 to 60 and 21.4 at 5; a
   // thousand intervals of 10^3..10^5 up to 10^18 take 0.80 ms up to 25 and 0.95 above
