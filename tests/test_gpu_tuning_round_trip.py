@@ -1,6 +1,7 @@
 """Saving a context's tuning and setting it again keeps the automatic tile shape.  The shape shows in the number
 of kernels of a short launch near 10^12: the chosen small tile comes with a pre-pass, the fixed one
 without."""
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -28,3 +29,19 @@ def test_the_automatic_shape_survives_a_round_trip():
         assert kernels(ctx) != automatic
         ctx.set_tuning(**t0)
         assert kernels(ctx) == automatic and ctx.tuning() == t0
+
+
+def test_the_autotuner_times_the_automatic_shape(tmp_path, monkeypatch):
+    import voss
+    from voss import autotune
+    monkeypatch.setenv("VOSS_TUNE_CACHE", str(tmp_path / "tune.json"))
+    with voss.Context(10**12) as ctx:
+        automatic = kernels(ctx)
+        seen = []
+        for cand in autotune.CANDIDATES:
+            ctx.set_tuning(**cand)
+            seen.append(kernels(ctx))
+        assert seen[0] == automatic
+        lo = np.array([LO], dtype=np.uint64)
+        autotune.tune_intervals(ctx, lo, lo + np.uint64(10**7), candidates=autotune.CANDIDATES[:1])
+        assert kernels(ctx) == automatic

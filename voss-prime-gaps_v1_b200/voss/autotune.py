@@ -1,10 +1,10 @@
 """Autotuner for the interval work queue.
 
 For a batch of intervals it picks the sieve tuning (tile shape = block_threads x chunk_words,
-the small/medium prime split coop_div, the multiples-walk threshold mult_factor) by timing a
-fixed candidate set on a sample of the batch's interval-size classes, with the kernel time
-the library measures (voss_last_kernel_ms).  Results are cached per (device, size-class
-signature) in a JSON file so that later batches of the same shape reuse them.
+the small/medium prime split coop_div, the pre-pass threshold mult_factor) by timing a
+candidate set, the library's automatic shape first, on a sample of the batch's interval-size
+classes, with the kernel time the library measures (voss_last_kernel_ms).  Results are cached per
+(device, size-class signature) in a JSON file so that later batches of the same shape reuse them.
 """
 from __future__ import annotations
 
@@ -14,7 +14,8 @@ import time
 
 import numpy as np
 
-# candidate tunings: tile bytes from 200 KB (1 CTA/SM) down to 36 KB (several CTAs/SM), with the
+# candidate tunings: the automatic shape (the values that tuning() reports for it: the library's default tile, or a
+# smaller one for small batches), then fixed tiles of 200 KB (1 CTA/SM) down to 36 KB (several CTAs/SM), with the
 # small/medium split (coop_div) and the pre-pass threshold (mult_factor) near their measured optima
 CANDIDATES = [
     dict(block_threads=1024, chunk_words=49, coop_div=80, mult_factor=8),
