@@ -29,9 +29,11 @@ __global__ void large_gather_kernel(const LargeGapDev* __restrict__ in, const ui
 
 // Lists of up to kSmallSort records, in the stream behind the tiles and before the host knows how
 // many there are: block b of G places the records of the b-th G-th of [lo, hi).  It goes over all positions once,
-// counts those below its part and lists those in it (a 148th of the records: gaps lie evenly over a
-// range), ranks the list against itself and writes each record to its place.  A part with more
-// records than the list holds is taken in halves; the positions are distinct, so that ends.
+// counts those below its part and lists those in it (a 148th of the records of a whole list: gaps lie
+// evenly over a range), ranks the list against itself and writes each record to its place.  A part with more
+// records than the list holds is taken in pieces, halved until one fits; the positions are distinct, so that
+// ends.  A list cut short at `cap` holds what the first tiles found, nearly all of it in a few parts: 10,000
+// of the 2.2e6 gaps >= 200 of 2e11 integers take one block 0.43 ms, beside 34 ms of tiles.
 // Bound by the latency of its reads, n per block from L2, where ranking every record against all n was
 // bound by n^2 compares: with the launch's other closing work 17.4 us for 10,602 records, 47.9 before,
 // 17.2 us for 15,826, 64.4 before, 11.4 us for 308, 15.1 before.  One launch and no second round trip
@@ -48,10 +50,11 @@ large_rank_kernel(const LargeGapDev* __restrict__ in, const uint32_t* __restrict
   const uint32_t n = *count < cap ? *count : cap;
   if (n > kSmallSort) return;
   const unsigned long long span = hi - lo, width = span / gridDim.x + 1ull, b = blockIdx.x;
-  unsigned long long from = b == 0 ? 0ull : lo + min(b * width, span);
-  const unsigned long long end = b + 1 == gridDim.x ? ~0ull : lo + min((b + 1) * width, span);
+  unsigned long long from = lo + min(b * width, span);
+  const unsigned long long end = lo + min((b + 1) * width, span);
+  unsigned long long piece = end - from;
   while (from < end) {
-    unsigned long long to = end;
+    unsigned long long to = from + min(piece, end - from);
     while (true) {
       __syncthreads();
       if (threadIdx.x == 0) s_below = s_listed = 0;
@@ -73,7 +76,8 @@ large_rank_kernel(const LargeGapDev* __restrict__ in, const uint32_t* __restrict
       if (threadIdx.x % 32 == 0 && below) atomicAdd(&s_below, below);
       __syncthreads();
       if (s_listed <= kRankList || to - from < 2ull) break;
-      to = from + (to - from) / 2ull;
+      piece = (to - from) / 2ull;
+      to = from + piece;
     }
     const uint32_t m = min(s_listed, kRankList);
     for (uint32_t i = threadIdx.x; i < m; i += kRankBlock) {
@@ -84,6 +88,7 @@ large_rank_kernel(const LargeGapDev* __restrict__ in, const uint32_t* __restrict
       out[rank] = in[s_idx[i]];
     }
     from = to;
+    if (m < kRankList / 4) piece *= 2ull;
   }
 }
 
