@@ -37,6 +37,8 @@ int fail(int code, const char* fmt, ...) {
   vsnprintf(buf, sizeof(buf), fmt, ap);
   va_end(ap);
   g_err = buf;
+  // reported here: a later launch that asks for the last error must not take this one for its own
+  if (code == VOSS_ERR_CUDA || code == VOSS_ERR_NOMEM) cudaGetLastError();
   return code;
 }
 
