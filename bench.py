@@ -301,8 +301,6 @@ def mr_mulmods(sample) -> tuple[int, int]:
 
 
 _MR_DOUBLE_END = 1 << 49  # below it the kernel's products are in double precision
-_FP64_OPS_PER_PRODUCT = 6
-_FP64_LANES_PER_CYCLE_SM = 62.0  # fp64 fma, measured on a B200
 
 
 def mr_products(sample) -> tuple[int, int, int]:
@@ -577,9 +575,7 @@ def run_mr(a) -> dict:
     m_dbl, m_small, m_full = (k * scale for k in mr_products(msample))
     m_all = m_dbl + m_small + m_full
     peak_full, peak_small = ctx.probe_mulmod()
-    sm_hz = 1e6 * (clk["sm_mhz"] or 1965.0)
-    peak_dbl = (_FP64_LANES_PER_CYCLE_SM / _FP64_OPS_PER_PRODUCT * sm_hz
-                * torch.cuda.get_device_properties(0).multi_processor_count)
+    peak_dbl = ctx.probe_mulmod_double()
     t_ideal = m_dbl / peak_dbl + m_small / peak_small + m_full / peak_full
     t_meas = ms * 1e-3
     got = d_out.cpu().numpy()
@@ -642,10 +638,9 @@ def run_mr(a) -> dict:
                      "products_from_2_63": m_full,
                      "peak_below_2_49_per_s": peak_dbl, "peak_small_per_s": peak_small,
                      "peak_full_per_s": peak_full,
-                     "peak_source": "below 2^49: six fp64 operations per product at the fp64 pipe's measured "
-                                    "rate; above: voss_probe_mulmod, independent Montgomery squaring chains on "
-                                    "this GPU in this run (moduli < 2^63 and >= 2^63); peak = the products' "
-                                    "time-weighted rate",
+                     "peak_source": "voss_probe_mulmod_double and voss_probe_mulmod: independent squaring chains on "
+                                    "this GPU in this run (products in double below 2^49, Montgomery moduli "
+                                    "< 2^63 and >= 2^63); peak = the products' time-weighted rate",
                      "count_sample": int(msample.size),
                      "traffic_note": "8 B read + 1 B written per candidate; DRAM figures in "
                                      "profiles/mr_kernel_2e6.md"},

@@ -322,6 +322,8 @@ VOSS_API int voss_probe_smem_rmw(voss_ctx* ctx, double* gbs);
  * active, no memory traffic), for moduli of 64 bits (full) and below 2^63 (small): the roofline
  * denominator of the Miller-Rabin kernels.  No counterpart in the reference. */
 VOSS_API int voss_probe_mulmod(voss_ctx* ctx, double* full_per_s, double* small_per_s);
+/* The same for the products in double precision that candidates below 2^49 are tested with. */
+VOSS_API int voss_probe_mulmod_double(voss_ctx* ctx, double* per_s);
 /* Device time (ms, CUDA events) of the last sieve launch on the context's events
  * (voss_sieve_range[_device], voss_sieve_intervals, voss_gaps_at_least, voss_primes_range):
  * sieve_ms from the launch's first device operation (descriptor copies, memsets) to the end of

@@ -586,10 +586,10 @@ int launch_prove_gaps(const uint64_t* d_p_after, const int32_t* d_gap, uint64_t 
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-// Peak rate of the Montgomery product on this device: independent squaring chains, every lane
-// active, no branches and no memory traffic.  The roofline denominator of the Miller-Rabin
-// kernels, which spend their time in the same products (one figure per variant: moduli below
-// and above 2^63).
+// Peak rates of the modular products on this device: independent squaring chains, every lane
+// active, no branches and no memory traffic.  The roofline denominators of the primality
+// kernels, which spend their time in the same products (one figure per variant: doubles below 2^49,
+// Montgomery moduli below and above 2^63).
 constexpr int kMulmodChains = 8;
 constexpr int kMulmodIters = 2048;
 constexpr int kMulmodBlock = 256;
@@ -613,25 +613,38 @@ __global__ void __launch_bounds__(kMulmodBlock) mulmod_probe_kernel(uint64_t nba
   if (acc == 1ull) sink[0] = acc;  // keeps the chains live; practically never taken
 }
 
-template <bool kSmallN>
-static int probe_mulmod_one(int sm_count, cudaStream_t s, uint64_t* sink, double* per_s) {
+__global__ void __launch_bounds__(kMulmodBlock) dmod_probe_kernel(uint64_t nbase, uint64_t* sink) {
+  const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const DMod M = dmod_setup(nbase | (tid << 1) | 1ull);
+  double x[kMulmodChains];
+#pragma unroll
+  for (int c = 0; c < kMulmodChains; ++c) x[c] = (double)(nbase >> 2) + (double)c;
+#pragma unroll 1
+  for (int i = 0; i < kMulmodIters; ++i) {
+#pragma unroll
+    for (int c = 0; c < kMulmodChains; ++c) x[c] = dmod_mul(x[c], x[c], M);
+  }
+  double acc = 0;
+#pragma unroll
+  for (int c = 0; c < kMulmodChains; ++c) acc += x[c];
+  if (acc == 1.0) sink[0] = 1;  // as above
+}
+
+static int probe_products(void (*kernel)(uint64_t, uint64_t*), uint64_t nbase, int sm_count, cudaStream_t s,
+                          uint64_t* sink, double* per_s) {
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mulmod_probe_kernel<kSmallN>, kMulmodBlock, 0) !=
-          cudaSuccess ||
-      occ < 1)
-    return -1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kMulmodBlock, 0) != cudaSuccess || occ < 1) return -1;
   const int grid = sm_count * occ;  // one full wave
-  const uint64_t nbase = kSmallN ? (1ull << 62) : (3ull << 62);
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess) return -1;
   if (cudaEventCreate(&e1) != cudaSuccess) {
     cudaEventDestroy(e0);
     return -1;
   }
-  mulmod_probe_kernel<kSmallN><<<grid, kMulmodBlock, 0, s>>>(nbase, sink);  // warm-up
+  kernel<<<grid, kMulmodBlock, 0, s>>>(nbase, sink);  // warm-up
   const int reps = 3;
   cudaEventRecord(e0, s);
-  for (int r = 0; r < reps; ++r) mulmod_probe_kernel<kSmallN><<<grid, kMulmodBlock, 0, s>>>(nbase, sink);
+  for (int r = 0; r < reps; ++r) kernel<<<grid, kMulmodBlock, 0, s>>>(nbase, sink);
   cudaEventRecord(e1, s);
   const cudaError_t st = cudaEventSynchronize(e1);
   float ms = 0;
@@ -643,12 +656,14 @@ static int probe_mulmod_one(int sm_count, cudaStream_t s, uint64_t* sink, double
   return 0;
 }
 
-int probe_mulmod(int sm_count, void* stream, double* full_per_s, double* small_per_s) {
+int probe_mulmod(int sm_count, void* stream, double* full_per_s, double* small_per_s, double* dbl_per_s) {
   cudaStream_t s = (cudaStream_t)stream;
   uint64_t* sink = nullptr;
   if (cudaMalloc(&sink, sizeof(uint64_t)) != cudaSuccess) return -1;
-  int rc = probe_mulmod_one<false>(sm_count, s, sink, full_per_s);
-  if (rc == 0) rc = probe_mulmod_one<true>(sm_count, s, sink, small_per_s);
+  int rc = 0;
+  if (full_per_s) rc |= probe_products(mulmod_probe_kernel<false>, 3ull << 62, sm_count, s, sink, full_per_s);
+  if (small_per_s) rc |= probe_products(mulmod_probe_kernel<true>, 1ull << 62, sm_count, s, sink, small_per_s);
+  if (dbl_per_s) rc |= probe_products(dmod_probe_kernel, kDModEnd >> 1, sm_count, s, sink, dbl_per_s);
   cudaFree(sink);
   return rc;
 }

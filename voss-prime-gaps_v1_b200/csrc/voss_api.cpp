@@ -1490,7 +1490,15 @@ VOSS_API int voss_probe_smem_rmw(voss_ctx* c, double* gbs) {
 VOSS_API int voss_probe_mulmod(voss_ctx* c, double* full_per_s, double* small_per_s) {
   if (!c || !full_per_s || !small_per_s) return fail(VOSS_ERR_ARG, "NULL argument");
   cudaSetDevice(c->device);
-  if (probe_mulmod(c->sm_count, c->stream, full_per_s, small_per_s)) return fail(VOSS_ERR_CUDA, "probe failed");
+  if (probe_mulmod(c->sm_count, c->stream, full_per_s, small_per_s, nullptr))
+    return fail(VOSS_ERR_CUDA, "probe failed");
+  return VOSS_OK;
+}
+
+VOSS_API int voss_probe_mulmod_double(voss_ctx* c, double* per_s) {
+  if (!c || !per_s) return fail(VOSS_ERR_ARG, "NULL argument");
+  cudaSetDevice(c->device);
+  if (probe_mulmod(c->sm_count, c->stream, nullptr, nullptr, per_s)) return fail(VOSS_ERR_CUDA, "probe failed");
   return VOSS_OK;
 }
 

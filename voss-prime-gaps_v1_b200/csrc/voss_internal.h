@@ -234,7 +234,8 @@ int launch_mr(const uint64_t* d_n, uint64_t count, uint8_t* d_out, void* stream,
 // kernel, then the interiors; count < 2^31.
 int launch_prove_gaps(const uint64_t* d_p_after, const int32_t* d_gap, uint64_t count, uint8_t* d_ok,
                       uint64_t* d_ends, uint8_t* d_ends_ok, void* stream, int sm_count);
-// Montgomery products per second of independent squaring chains (moduli above / below 2^63).
-int probe_mulmod(int sm_count, void* stream, double* full_per_s, double* small_per_s);
+// Modular products per second of independent squaring chains (Montgomery moduli above and below 2^63,
+// doubles below 2^49); a null pointer: not measured.
+int probe_mulmod(int sm_count, void* stream, double* full_per_s, double* small_per_s, double* dbl_per_s);
 
 }  // namespace voss

@@ -137,6 +137,7 @@ SIGNATURES = {
     "voss_last_phase_ms": (c_int, [c_void_p, POINTER(c_double), POINTER(c_double), POINTER(c_double),
                                    POINTER(c_uint32)]),
     "voss_probe_mulmod": (c_int, [c_void_p, POINTER(c_double), POINTER(c_double)]),
+    "voss_probe_mulmod_double": (c_int, [c_void_p, POINTER(c_double)]),
 }
 
 _lib = None

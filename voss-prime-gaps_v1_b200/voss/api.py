@@ -264,6 +264,12 @@ class Context:
         N.check(self.lib.voss_probe_mulmod(self._h, byref(f), byref(s)))
         return f.value, s.value
 
+    def probe_mulmod_double(self) -> float:
+        """Products/s in double precision, for moduli below 2^49."""
+        d = c_double()
+        N.check(self.lib.voss_probe_mulmod_double(self._h, byref(d)))
+        return d.value
+
 
 def write_artifacts(res: RangeResult, out_dir: str) -> None:
     """Write the reference's CSV artifacts for a REF_COMPAT range (voss_write_artifacts)."""
