@@ -167,7 +167,7 @@ def profile_traffic_per_unit() -> tuple[float | None, str | None]:
     except OSError:
         return None, None
     m = re.search(r"dram_bytes_per_integer:\s*([0-9.eE+-]+)", txt)
-    return (float(m.group(1)), rel + " (10^11 capture, scaled by integers)") if m else (None, None)
+    return (float(m.group(1)), "committed ncu capture at 10^11, scaled by integers") if m else (None, None)
 
 
 _COPRIME30 = [sum(1 for r in range(1, x + 1) if r % 2 and r % 3 and r % 5) for x in range(30)]
@@ -507,13 +507,13 @@ def run_intervals(a) -> dict:
             "ms": pre_ms, "clears": work["prepass_hits"],
             "issue_frac_ncu": 0.674, "alu_frac_ncu": 0.442,
             "source": "issue and ALU-pipe fractions of peak (active cycles) of scatter_large_kernel from the "
-                      "committed capture profiles/scatter_large_kernel_intervals.md; one 64-bit reduction per "
+                      "committed ncu capture on the interval batch; one 64-bit reduction per "
                       "(prime, interval) pair, ms includes the batch's copies and bitmap memset"},
         "roofline": {"bound": "smem", "achieved": achieved, "peak": smem_peak, "unit": "GB/s",
                      "frac": achieved / smem_peak, "traffic": None, "kernel": "sieve_tiles_kernel",
                      "kernel_ms": tile_ms, "algorithmic_bytes": alg_bytes,
                      "peak_source": "voss_probe_smem_rmw (this GPU, this run)",
-                     "traffic_note": "DRAM traffic of this launch: profiles/launches_intervals_4096.md"},
+                     "traffic_note": "DRAM traffic of this launch: the committed launch list of the interval batch"},
         "clocks": clk,
         "gpu_launches": a.steps * phases[-1][3],
     }
@@ -642,8 +642,8 @@ def run_mr(a) -> dict:
                                     "this GPU in this run (products in double below 2^49, Montgomery moduli "
                                     "< 2^63 and >= 2^63); peak = the products' time-weighted rate",
                      "count_sample": int(msample.size),
-                     "traffic_note": "8 B read + 1 B written per candidate; DRAM figures in "
-                                     "profiles/mr_kernel_2e6.md"},
+                     "traffic_note": "8 B read + 1 B written per candidate; DRAM figures in the committed "
+                                     "ncu capture of mr_kernel"},
         "clocks": clk,
         "gpu_launches": a.steps,
     }
