@@ -975,6 +975,17 @@ int run_range_device(voss_ctx* c, uint64_t lo, uint64_t hi, uint32_t flags, uint
   return VOSS_OK;
 }
 
+// Work queued on `later` from here on runs behind what is queued on `earlier`.
+int stream_after(cudaStream_t later, cudaStream_t earlier) {
+  if (later == earlier) return VOSS_OK;
+  cudaEvent_t e;
+  CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  cudaError_t st = cudaEventRecord(e, earlier);
+  if (st == cudaSuccess) st = cudaStreamWaitEvent(later, e, 0);
+  cudaEventDestroy(e);
+  return st == cudaSuccess ? VOSS_OK : fail(VOSS_ERR_CUDA, "ordering two streams failed: %s", cudaGetErrorString(st));
+}
+
 // The first n device large-gap records, sorted by position on the device (positions < hi), in
 // the context's pinned staging.
 int stage_large_sorted(voss_ctx* c, uint64_t n, uint64_t hi, voss_large_gap** out) {
@@ -1176,16 +1187,13 @@ VOSS_API int voss_sieve_range_device(voss_ctx* c, uint64_t lo, uint64_t hi, uint
   if (!c) return fail(VOSS_ERR_ARG, "ctx is NULL");
   cudaSetDevice(c->device);
   cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
-  int rc = run_range_device(c, lo, hi, flags, seg_num, kDefaultLargeCap, s);
-  if (rc) return rc;
-  if (s != c->stream) {  // later fetches run on the context stream
-    cudaEvent_t e;
-    CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    CUDA_TRY(cudaEventRecord(e, s));
-    CUDA_TRY(cudaStreamWaitEvent(c->stream, e, 0));
-    cudaEventDestroy(e);
-  }
-  return VOSS_OK;
+  // The workspace is the context's, whichever stream a launch runs on: each one waits for the one before,
+  // through the context's stream, on which later calls and fetches run.
+  int rc;
+  if ((rc = stream_after(s, c->stream))) return rc;
+  rc = run_range_device(c, lo, hi, flags, seg_num, kDefaultLargeCap, s);
+  const int rc_after = stream_after(c->stream, s);
+  return rc ? rc : rc_after;
 }
 
 VOSS_API int voss_fetch_range(voss_ctx* c, voss_range_stats* st, voss_large_gap* large,
