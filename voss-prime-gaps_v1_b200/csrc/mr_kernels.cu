@@ -352,8 +352,10 @@ __device__ __noinline__ bool call_lucas(uint64_t n) {
 // Bound by the pipe of the products: 5e6 primes below 10^12 take 0.50 ms (two tests in double
 // precision; 3.6 ms with six Montgomery tests each), 4,000,001 random odd 64-bit numbers 0.34 ms
 // (0.77 ms with up to twelve bases and the survivors in a work list for a second kernel), 1000 of
-// them 24 us (123 us).  Eight blocks per SM, two waves, against 4 and 16: 0.34, 0.37 and
-// 0.35 ms (a second wave evens out what the warps of the first happen to find).
+// them 24 us (123 us).  Eight blocks per SM were chosen with the tests inlined (four resident: two waves, the second
+// evening out what the warps of the first happen to find).  Large batches run them as calls now (below), five
+// resident, and 8 is no longer the best: 4, 5, 8, 10, 15 and 16 per SM take 334, 339, 341, 321, 329 and 333 us
+// for these 64-bit numbers, 525, 516, 492, 499, 488 and 487 us for the primes.
 constexpr int kMrBlock = 256;
 constexpr int kMrBlocksPerSm = 8;
 constexpr int kMrQueue = 64;  // at most 31 waiting + 32 arriving

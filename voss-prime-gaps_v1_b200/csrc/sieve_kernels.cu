@@ -1654,7 +1654,7 @@ __global__ void __launch_bounds__(kScatterBlock) scatter_large_kernel(const uint
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t jb = j0 + blockIdx.x * blockDim.x + (threadIdx.x & ~31u); jb < j1; jb += stride) {
     const uint32_t j = min(jb + lane, j1 - 1u);
-    const uint32_t p = primes[j];  // >= 2^13 (choose_shape)
+    const uint32_t p = primes[j];  // >= 2^13 (choose_shape); with the smallest tile that can be set >= 2^11
     const double inv = __drcp_rn((double)p);
     // intervals are sorted by sqrt_hi, descending: p reaches the first n_reach of them
     uint32_t lo = 0, hi = jb + lane < j1 ? n_iv : 0;
@@ -1665,8 +1665,9 @@ __global__ void __launch_bounds__(kScatterBlock) scatter_large_kernel(const uint
     const uint32_t n_reach = lo, reach_w = __reduce_max_sync(kFull, n_reach);
     if (__all_sync(kFull, p < (1u << 30))) {
       // The first multiple's offset d = q p - vbase with q = vbase / p rounded to an integer (adding
-      // 2^52 in the same rounding leaves it in the low mantissa bits: q < 2^52): d is in
-      // (-0.63 p, 0.63 p), so the low 32 bits hold it, and a negative one needs one p more.
+      // 2^52 in the same rounding leaves it in the low mantissa bits: q < 2^51 for vbase < 2^62): vd and
+      // inv are off by a relative 2^-53 each, so |d| < 0.63 p for p >= 2^13 and below p for p >= 2^11.
+      // The low 32 bits hold it, and a negative one needs one p more.
       auto first = [&](const uint4& h) {  // h: one 16-byte load per pair (vbase_d, vbase_lo, span32)
         const double vd = __hiloint2double((int)h.y, (int)h.x);
         const uint32_t d = (uint32_t)__double2loint(__fma_rn(vd, inv, 4503599627370496.0)) * p - h.z;

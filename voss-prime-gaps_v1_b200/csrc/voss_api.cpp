@@ -219,6 +219,10 @@ TileShape default_shape(const voss_ctx* c) {
 //    2^11..2^19: 8192, 32768, 131072, 524288 for 10^5..10^8 integers);
 //  - in a single wave of short chunks, small primes up to tile/40: a warp each instead of two lanes
 //    each, whose clears in a row are the longest chain of such a launch ([1, 10^7] 67 -> 57 us).
+// A workspace without room for the pre-pass's bitmap gains less: its tiles then walk the primes from the lowered
+// bound on one by one, but still in no more time than the default tile takes them by class (a server slot
+// with 256 bytes of bitmap, one request of 10^6, 10^7, 10^8 integers: 129, 126, 144 us against 141, 225, 225
+// at 10^12; 3.8, 3.9, 4.1 ms against 4.0, 4.4, 4.7 near 10^16; 40 and 200 at a time alike or better).
 // Device time in the default tile and so: 10^6 integers at 10^12 115 -> 62 us, 10^7 203 -> 70,
 // 10^8 201 -> 117, 10^9 354 -> 272; [1, 10^8] 306 -> 85, [1, 10^9] 251 -> 219.
 TileShape choose_shape(const voss_ctx* c, const uint64_t* lo, const uint64_t* hi, uint32_t n, uint64_t max_tiles) {
@@ -777,7 +781,7 @@ int launch_routed(voss_ctx* c, Workspace& W, const LaunchEvents& E, const Interv
       return fail(VOSS_ERR_CUDA, "short-interval launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     k += nc ? 4 : 3;
   }
-  if (E.ev2) CUDA_TRY(cudaEventRecord(E.ev2, s));  // finalize and the Miller-Rabin path count in the launch's time
+  if (E.ev2) CUDA_TRY(cudaEventRecord(E.ev2, s));  // the Miller-Rabin path counts in the launch's time
   if (kernels) *kernels = k;
   return VOSS_OK;
 }

@@ -82,8 +82,9 @@ struct Workspace {
 };
 
 // Events bracketing one launch: ev0 before all of its device work (descriptor copies, memsets),
-// ev1 after the tile kernel, ev2 after the stitch/reduce kernels; evp (optional) after the
-// large-prime pre-pass, just before the tile kernel.
+// ev1 after the tile kernel, ev2 after the kernels that close the launch (seams, results, the sort of a
+// short gap list, the short-interval route); evp (optional) after the large-prime pre-pass, just before
+// the tile kernel.
 struct LaunchEvents {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, evp = nullptr;
 };
@@ -135,9 +136,9 @@ constexpr uint64_t kMaxHi = 1ull << 62;
 constexpr uint32_t kOverCap = 1u << 16;
 constexpr uint64_t kDefaultLargeCap = 1ull << 22;
 // Large-prime pre-pass windows: bitmap bytes per window, inside the 126 MB L2 next to the primes
-// the pre-pass reads (23 MB of 32-bit primes below 10^8).  On the 4096-interval batch 48 MB
-// windows measured 9.46 ms against 9.62 ms for 32 MB, 9.83 ms for 24 MB and 9.61 ms for 64 MB; the
-// 157 MB bitmap of 4.7e9 integers near 10^15 takes 1.30 ms in four pieces against 4.24 ms in one.
+// the pre-pass reads (23 MB of 32-bit primes below 10^8).  The 4096-interval batch's pre-pass takes 7.8 ms
+// with 48 MB, 8.5, 8.1, 8.0 and 8.1 ms with 16, 24, 32 and 64 MB; the 157 MB bitmap of 4.7e9 integers
+// near 10^15 1.30 ms in four pieces against 4.24 ms in one.
 #ifndef VOSS_SCATTER_WINDOW_MB
 #define VOSS_SCATTER_WINDOW_MB 48
 #endif
@@ -177,7 +178,7 @@ struct voss_ctx {
   uint32_t r_tiles = 0;
   uint64_t r_large_cap = 0;
   float sieve_ms = 0, total_ms = 0;
-  uint32_t last_kernels = 0;  // kernels of the last launch_plan_ws (+ finalize for intervals)
+  uint32_t last_kernels = 0;  // kernels of the last launch (with the short-interval route's)
   // host side of the large-gap list: pinned, grow-only staging for the device-to-host copy of
   // the list (sorted on the device), so that repeated calls touch no fresh pages
   voss_large_gap* h_large = nullptr;

@@ -10,7 +10,7 @@
 //   claim tile indices from one atomic counter.
 //   Per-interval accumulators (u64, kAccStride per interval) hold the counters every tile
 //   adds into; per-tile partials carry the first/last prime of each tile so that the gaps
-//   across tile seams can be added afterwards by the stitch kernel.
+//   across tile seams can be added afterwards (stitch_kernel or tail_kernel).
 #pragma once
 
 #include <cstdint>
@@ -125,7 +125,7 @@ struct TilePartial {
   uint32_t count;
   uint32_t max_gap;  // largest in-tile gap (0 if < 2 primes)
   uint32_t max_lo;   // value offset of its lower prime
-  uint32_t bgap;     // gap from the previous non-empty tile's last prime (stitch kernel)
+  uint32_t bgap;     // gap from the previous non-empty tile's last prime (where stitch_kernel runs)
   uint64_t bgap_lo;  // that gap's lower prime
 };
 

@@ -160,7 +160,7 @@ class Context:
         return a.value, b.value
 
     def last_phase_ms(self) -> tuple[float, float, float, int]:
-        """(pre-pass incl. copies and memsets, tile kernel, stitch/reduce/finalize) in ms of the
+        """(pre-pass incl. copies and memsets, tile kernel, the kernels behind it) in ms of the
         last launch, and the number of kernels it launched."""
         a, b, t, k = c_double(), c_double(), c_double(), c_uint32()
         N.check(self.lib.voss_last_phase_ms(self._h, byref(a), byref(b), byref(t), byref(k)))
