@@ -45,3 +45,16 @@ def test_the_autotuner_times_the_automatic_shape(tmp_path, monkeypatch):
         lo = np.array([LO], dtype=np.uint64)
         autotune.tune_intervals(ctx, lo, lo + np.uint64(10**7), candidates=autotune.CANDIDATES[:1])
         assert kernels(ctx) == automatic
+
+
+def test_a_tie_goes_to_the_automatic_shape(tmp_path, monkeypatch):
+    import voss
+    from voss import autotune
+    monkeypatch.setenv("VOSS_TUNE_CACHE", str(tmp_path / "tune.json"))
+    with voss.Context(10**12) as ctx:
+        automatic = kernels(ctx)
+        times = iter([2.490, 2.488, 2.486])  # each a little faster than the one before
+        monkeypatch.setattr(ctx, "last_kernel_ms", lambda: (0.0, next(times)))
+        lo = np.array([LO], dtype=np.uint64)
+        autotune.tune_intervals(ctx, lo, lo + np.uint64(10**6), reps=1, candidates=autotune.CANDIDATES[:3])
+        assert kernels(ctx) == automatic

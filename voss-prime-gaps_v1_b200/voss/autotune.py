@@ -27,6 +27,8 @@ CANDIDATES = [
     dict(block_threads=512, chunk_words=9, coop_div=16, mult_factor=4),
 ]
 
+MARGIN = 0.01  # by which a fixed tile has to be faster than the best before it: the runs of one differ by less
+
 CLASS_EDGES = (10**5, 10**6, 10**7)  # interval lengths: tiny / small / medium / large
 
 
@@ -83,7 +85,7 @@ def tune_intervals(ctx, lo, hi, sample: int = 512, reps: int = 2, seed: int = 1,
         t = float(np.median(ms))
         name = "%dx%d/c%d/m%d" % (cand["block_threads"], cand["chunk_words"], cand["coop_div"], cand["mult_factor"])
         timings[name] = t
-        if t < best_ms:
+        if best is None or t < (1 - MARGIN) * best_ms:
             best, best_ms = cand, t
     ctx.set_tuning(**best)
     res = {"tuning": best, "timings_ms": timings, "signature": sig, "when": time.time()}
