@@ -16,7 +16,7 @@
 //
 // Arithmetic, by the size of n:
 //   n < 2^49: products mod n in double precision from exact fma halves (DMod): six operations of the
-//             fp64 pipe, 9.8 products per cycle and SM measured;
+//             fp64 pipe, 9.96 products per cycle and SM measured;
 //   others:   64-bit Montgomery multiplication with R = 2^64 (mul.lo/mul.hi on the integer pipe, no
 //             128-bit division), 2.36 per cycle and SM.
 // One kernel does all of it: candidates that trial division leaves open wait in per-warp queues by
